@@ -71,6 +71,11 @@ struct Ctx {
     std::map<int, int> warm;
     bool interp_alloc = false;
     unsigned long long gen = 0;  // bumped by every change of the history
+    // Within one call the next step goes on from the previous one: the B2 sums held are its own (b2_cont),
+    // and after an RK54 step whose row nobody edited the last stage's right-hand side is the next RK54
+    // step's first (fsal_ok: Dormand-Prince writes the new row before its last stage evaluates it)
+    bool b2_cont = false, fsal_ok = false;
+    void new_call() { b2_cont = fsal_ok = false; }
     // discrete adjoint (FP64, fixed schedule): the recorded forward and its buffers
     AdjDev ad{};
     size_t ad_cap = 0;
@@ -115,7 +120,7 @@ struct Ctx {
                         d.geS, d.gfS, d.part, d.rowval, d.epart, d.slots, d.stages, d.rhs_out, d.ip,
                         d.rint, scratch_dev, (void*)d.wA1f, (void*)d.wA2f, (void*)d.wB2f, d.KRf, d.dKRf,
                         (void*)d.integ_f, d.inv_len_f, d.inv_dtr_f, d.KRl, (void*)d.wA1l, (void*)d.wA2l,
-                        (void*)d.wB2l, tail};
+                        (void*)d.wB2l, tail, d.inv_len, d.b1, d.b2key, d.b2s, d.b2f, d.b2q};
         for (void* b : bufs) if (b) cudaFree(b);
         std::memset(&d, 0, sizeof d);
         scratch_dev = nullptr;
@@ -141,6 +146,8 @@ struct Ctx {
         if ((s = dalloc(&KR, ncap * L)) || (s = dalloc(&dKR, ncap * L)) || (s = dalloc(&t1g, ncap)) ||
             (s = dalloc(&dt, ncap)) || (s = dalloc(&idt, ncap)) || (s = dalloc(&rv, ncap)) || (s = dalloc(&drv, ncap)))
             return s;
+        double* ilen64 = nullptr;
+        if (!d.mixed && (s = dalloc(&ilen64, ncap))) return s;
         float2 *KRf = nullptr, *dKRf = nullptr;
         float *ilen = nullptr, *idtf = nullptr;
         if (d.mixed && ((s = dalloc(&ilen, ncap)) || (s = dalloc(&idtf, ncap)))) return s;
@@ -168,11 +175,13 @@ struct Ctx {
             CK(cudaMemcpyAsync(idt, d.inv_dtr, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
             CK(cudaMemcpyAsync(rv, d.rvec, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
             CK(cudaMemcpyAsync(drv, d.drvec, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+            if (ilen64) CK(cudaMemcpyAsync(ilen64, d.inv_len, n * sizeof(double), cudaMemcpyDeviceToDevice, st));
             CK(cudaStreamSynchronize(st));
         }
         for (void* b : {(void*)d.KR, (void*)d.dKR, (void*)d.t1grid, (void*)d.dtr, (void*)d.inv_dtr, (void*)d.rvec,
-                        (void*)d.drvec})
+                        (void*)d.drvec, (void*)d.inv_len})
             if (b) cudaFree(b);
+        d.inv_len = ilen64;
         d.KR = KR; d.dKR = dKR; d.t1grid = t1g; d.dtr = dt; d.inv_dtr = idt; d.rvec = rv; d.drvec = drv;
         if (d.mixed) {
             if (d.KRf) cudaFree(d.KRf);
@@ -192,12 +201,30 @@ struct Ctx {
         return DYN_OK;
     }
 
+    // Planes for the B2 sums of one call.  Without the memory for them the stages form
+    // every sum, as the first stage of a call does.
+    void alloc_b2() {
+        if (d.mixed) return;
+        if (cudaMalloc((void**)&d.b2key, L2 * sizeof(int)) == cudaSuccess &&
+            cudaMalloc((void**)&d.b2s, 4 * L2 * sizeof(double2)) == cudaSuccess)
+            return;
+        cudaGetLastError();
+        if (d.b2key) cudaFree(d.b2key);
+        d.b2key = nullptr;
+        d.b2s = nullptr;
+    }
+
     dyn_status upload_times() {
         std::vector<double> inv(n);
         for (size_t k = 0; k < n; ++k) inv[k] = dtr[k] != 0.0 ? 1.0 / dtr[k] : 0.0;
         CK(cudaMemcpyAsync(d.t1grid, t1.data(), n * sizeof(double), cudaMemcpyHostToDevice, st));
         CK(cudaMemcpyAsync(d.dtr, dtr.data(), n * sizeof(double), cudaMemcpyHostToDevice, st));
         CK(cudaMemcpyAsync(d.inv_dtr, inv.data(), n * sizeof(double), cudaMemcpyHostToDevice, st));
+        std::vector<double> il(n, 0.0);
+        if (d.inv_len) {
+            for (size_t k = 0; k + 1 < n; ++k) il[k] = 1.0 / (t1[k + 1] - t1[k]);
+            CK(cudaMemcpyAsync(d.inv_len, il.data(), n * sizeof(double), cudaMemcpyHostToDevice, st));
+        }
         if (d.mixed) CK(launch_time_f32(d.t1grid, d.dtr, (int)n, d.inv_len_f, d.inv_dtr_f, st));
         CK(cudaStreamSynchronize(st));
         return DYN_OK;
@@ -321,6 +348,8 @@ struct Ctx {
             sp.T_next = Tn[s];
             sp.tdiff = Tn[s] - T0;
             sp.dtr_new = n0 >= 2 ? sp.tdiff / prev : 0.0;  // time_steps.cpp:58-67,142-149
+            // a stage at t = 0 gathers nothing, so the one after it starts the sums
+            sp.b2_mode = (s == 0 && !b2_cont) || (s == 1 && !(T0 > 0.0)) ? B2_FILL : B2_KEEP;
         }
         *S_out = S;
         *T_final = Tn[S - 1];
@@ -328,9 +357,9 @@ struct Ctx {
         return DYN_OK;
     }
 
-    dyn_status enqueue_step(int S) {
+    dyn_status enqueue_step(int S, bool fsal) {
         CK(cudaMemcpyAsync(d.stages, stages_h, sizeof(StageDev) * S, cudaMemcpyHostToDevice, st));
-        for (int s = 0; s < S; ++s) CK(launch_stage(d, s, st));
+        for (int s = 0; s < S; ++s) CK(launch_stage(d, s, st, !(s == 0 && fsal)));
         CK(cudaMemcpyAsync(slots_h, d.slots, sizeof(Slots), cudaMemcpyDeviceToHost, st));
         return DYN_OK;
     }
@@ -342,23 +371,26 @@ struct Ctx {
         int S;
         double err_t, Tf, dtrf;
         if ((s = build_step(method, dt, &S, &err_t, &Tf, &dtrf))) return s;
+        const bool fsal = method == DYN_RK54 && fsal_ok;
+        stages_h[0].fsal = fsal;
+        const int key = fsal ? -method : method;
         if (cfg.use_graph && warm[method] > 0) {
-            auto it = graphs.find(method);
+            auto it = graphs.find(key);
             if (it == graphs.end()) {
                 cudaGraph_t g;
                 CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-                dyn_status es = enqueue_step(S);
+                dyn_status es = enqueue_step(S, fsal);
                 cudaError_t ce = cudaStreamEndCapture(st, &g);
                 if (es) return es;
                 CK(ce);
                 cudaGraphExec_t ge;
                 CK(cudaGraphInstantiate(&ge, g, 0));
                 cudaGraphDestroy(g);
-                it = graphs.emplace(method, ge).first;
+                it = graphs.emplace(key, ge).first;
             }
             CK(cudaGraphLaunch(it->second, st));
         } else {
-            if ((s = enqueue_step(S))) return s;
+            if ((s = enqueue_step(S, fsal))) return s;
             warm[method]++;
         }
         CK(cudaStreamSynchronize(st));
@@ -366,6 +398,8 @@ struct Ctx {
         dtr.push_back(dtrf);
         n += 1;
         gen++;
+        b2_cont = true;
+        fsal_ok = method == DYN_RK54 && stages_h[S - 1].T == Tf;
         if (res) {
             res->delta = slots_h->res_err + err_t;
             res->t = Tf;
@@ -712,6 +746,7 @@ static dyn_status tail_fit(Ctx* c, int rollback_loop) {
     if (e == cudaSuccess && d.KRl) e = launch_mirror_lo(d.KR + row, d.KRl + row, c->L, c->st);
     if (e != cudaSuccess) return fail(DYN_ERR_CUDA, cudaGetErrorString(e));
     c->gen++;  // the newest row may have changed
+    c->fsal_ok = false;
     return DYN_OK;
 }
 
@@ -770,11 +805,13 @@ dyn_status dyn_ctx_create(const dyn_config* cfg, const dyn_tables* tb, void** ou
     d.search = cfg->search;
     d.logr = cfg->log_response;
     d.mixed = cfg->precision == DYN_MIXED ? 1 : cfg->precision == DYN_MIXED_DF ? 2 : 0;
-    // tile shape: threads per CTA x targets per thread.  FP64: few wide CTAs
-    // amortize the FP64 reduction; mixed: one target per thread keeps more
-    // warps in flight for the latency-bound gathers.
+    // tile shape: threads per CTA x targets per thread.  FP64: two targets share a warp
+    // reduction from L = 768 on, where enough CTAs are left to balance the SMs; per RK54
+    // step 1 / 2 targets measure 152 / 159 us (L = 64), 228 / 241 (256), 414 / 466 (400),
+    // 555 / 562 (512), 1780 / 1756 (1024).  Mixed: one target per thread keeps more warps
+    // in flight for the latency-bound gathers.
     d.tpb = d.mixed ? 128 : 64;
-    d.kpt = d.mixed ? 1 : (L >= 512 ? 4 : (L >= 256 ? 2 : 1));
+    d.kpt = d.mixed ? 1 : (L >= 768 ? 2 : 1);
     d.nch = (int)((L + (size_t)d.tpb * d.kpt - 1) / ((size_t)d.tpb * d.kpt));
     d.M = make_model(cfg->p, cfg->p2, cfg->lambda, cfg->T0, cfg->Gamma);
 
@@ -784,7 +821,7 @@ dyn_status dyn_ctx_create(const dyn_config* cfg, const dyn_tables* tb, void** ou
     int *a1, *a2, *b2;
     if ((s = dalloc(&th, L)) || (s = dalloc(&p2, L2)) || (s = dalloc(&it, L)) || (s = dalloc(&a1, L2)) ||
         (s = dalloc(&a2, L2)) || (s = dalloc(&b2, L2)) || (s = dalloc(&w1, L2 * m)) || (s = dalloc(&w2, L2 * m)) ||
-        (s = dalloc(&w3, L2 * m)) || (s = dalloc(&d.posB1x, L)) || (s = dalloc(&d.posB1x_next, L)) || (s = dalloc(&d.posB1x_saved, NSAVE * L)) ||
+        (s = dalloc(&w3, L2 * m)) || (s = dalloc(&d.posB1x, L)) || (s = dalloc(&d.posB1x_next, L)) || (s = dalloc(&d.b1, L)) || (s = dalloc(&d.posB1x_saved, NSAVE * L)) ||
         (s = dalloc(&d.posB2x, L2)) || (s = dalloc(&d.posB2x_saved, NSAVE * L2)) ||
         (s = dalloc(&d.h, (size_t)SMAX * L)) || (s = dalloc(&d.gS, L)) || (s = dalloc(&d.geS, L)) ||
         (s = dalloc(&d.gfS, L)) || (s = dalloc(&d.part, L * (size_t)d.nch * 8)) || (s = dalloc(&d.rowval, L)) ||
@@ -847,6 +884,7 @@ dyn_status dyn_ctx_create(const dyn_config* cfg, const dyn_tables* tb, void** ou
             }
         }
     }
+    c->alloc_b2();
     if (cudaMallocHost((void**)&c->stages_h, sizeof(StageDev) * SMAX) != cudaSuccess ||
         cudaMallocHost((void**)&c->slots_h, sizeof(Slots)) != cudaSuccess ||
         cudaMallocHost((void**)&c->rhs_h, sizeof(double2) * L) != cudaSuccess) {
@@ -1272,6 +1310,7 @@ dyn_status dyn_update(void* p, int method, double delta_t, dyn_step_result* res)
     if (method < 1) return fail(DYN_ERR_INVALID, "unknown method");
     if (!(delta_t > 0.0)) return fail(DYN_ERR_INVALID, "delta_t must be positive");
     TraceRange tr("dyn_update");
+    C(p)->new_call();
     return C(p)->step(method, delta_t, res);
 }
 
@@ -1285,6 +1324,7 @@ dyn_status dyn_run(void* p, const dyn_run_params* rp, dyn_step_result* last) {
     if (!rp->dt_schedule && (k.method < 1 || !(k.delta_t > 0.0)))
         return fail(DYN_ERR_STATE, "no step size or method: call dyn_controller_set after dyn_state_upload");
     dyn_step_result r{};
+    c->new_call();  // kept from step to step of one call, not between calls
     for (int it = 0; it < rp->nsteps; ++it) {
         if (rp->tmax > 0 && c->t1[c->n - 1] >= rp->tmax) break;
         if (rp->dt_schedule) {
@@ -1371,6 +1411,7 @@ dyn_status dyn_rollback(void* p, int nrows) {
     const size_t target = c->n - nrows, n_old = c->n;
     c->n = target;
     c->gen++;
+    c->new_call();
     if (dyn_status cs = c->clear_tail(n_old)) return cs;
     c->t1.resize(target);
     c->dtr.resize(target);
@@ -1517,6 +1558,7 @@ dyn_status dyn_adjoint_backward(void* p, const dyn_adjoint_objective* obj, doubl
     const auto t0 = std::chrono::steady_clock::now();
     const size_t n_final = c->n, N = c->adj_dt.size(), L = c->L;
     const std::vector<double> t1_saved = c->t1, dtr_saved = c->dtr;
+    c->new_call();  // every recomputed step starts from a shorter history
     if ((s = c->snapshot(false))) return s;
     CK(cudaMemsetAsync(c->ad.HKR, 0, n_final * L * sizeof(double2), c->st));
     CK(cudaMemsetAsync(c->ad.HdKR, 0, n_final * L * sizeof(double2), c->st));
@@ -1632,6 +1674,7 @@ dyn_status dyn_sparsify(void* p, double threshold, int variant, size_t* n_out) {
     const size_t n_old = c->n;
     c->n = k;
     c->gen++;
+    c->new_call();
     if ((s = c->mirror_all())) return s;
     if ((s = c->clear_tail(n_old))) return s;
     if ((s = c->upload_times())) return s;

@@ -67,6 +67,8 @@ struct Quench {
     long long spars_every;  // periodic sparsify every this many loops (0: never)
 };
 
+constexpr int SIDE_ITEM = 0x8000;  // gather items at or above this row: the rows' own work, a CTA's threads each
+
 struct Work {
     unsigned next, done;
 };
@@ -254,6 +256,9 @@ __device__ void adapt_step(const Quench& q, Plan& pl, const TabDev& tb) {
 // tail; a cap of 64 registers (DYN_BATCH_DF_TPSM = 1024 threads per SM) spills a
 // little but measures best for 64 quenches at L=512: 1.55 ms against 1.62 (56
 // registers), 1.61 (72) and 1.74 (80).
+__device__ __noinline__ void batch_side(const DevCtx& c, const StageDev& sp, const int blk) {
+    mixed::side_rows<true>(c, sp, blk);
+}
 template <int M, int K, int P, int P2, int TPB, bool DF = false>
 __global__ void __launch_bounds__(TPB, DF ? DYN_BATCH_DF_TPSM / TPB : (K == 1 ? DYN_BATCH_TPSM : 512) / TPB)
     k_batch_gather(const Quench* __restrict__ Q, const Plan* __restrict__ PL, const unsigned* __restrict__ items,
@@ -277,14 +282,17 @@ __global__ void __launch_bounds__(TPB, DF ? DYN_BATCH_DF_TPSM / TPB : (K == 1 ? 
             const int i = (int)(e & 0xffffu);
             const StageDev& sp = q.stg[pl.sidx * SMAX + pl.s];
             float2* s_lo = s_lastf + (q.c.L + 2);
-            if constexpr (DF) {
-                mixed::row_setup(q.c, sp, i, true, s_lastf, sh, s_clo);
+            int nch = q.c.nch;
+            if (i >= SIDE_ITEM) {
+                batch_side(q.c, sp, i - SIDE_ITEM);
+                nch = 0;
+            } else if constexpr (DF) {
+                mixed::row_setup<true>(q.c, sp, i, s_lastf, sh, s_clo);
                 mdf::stage_lo(q.c, sp, s_lo);
             } else {
-                mixed::row_setup(q.c, sp, i, true, s_lastf, sh);
+                mixed::row_setup<true>(q.c, sp, i, s_lastf, sh);
             }
             __syncthreads();
-            const int nch = q.c.nch;
             for (int ch0 = 0; ch0 < nch; ch0 += GMAX) {
                 const int ng = min(GMAX, nch - ch0);
                 for (int g = 0; g < ng; ++g) {
@@ -880,7 +888,7 @@ dyn_status dyn_batch_create(const dyn_batch_config* cfg, const dyn_batch_grid* g
             (s = bt->alloc(&d.KRf, cap * L + 16)) || (s = bt->alloc(&d.dKRf, cap * L + 16)) ||
             (s = bt->alloc(&d.t1grid, cap)) || (s = bt->alloc(&d.dtr, cap)) || (s = bt->alloc(&d.inv_dtr, cap)) ||
             (s = bt->alloc(&d.rvec, cap)) || (s = bt->alloc(&d.drvec, cap)) || (s = bt->alloc(&d.inv_len_f, cap)) ||
-            (s = bt->alloc(&d.inv_dtr_f, cap)) || (s = bt->alloc(&d.posB1x, L)) || (s = bt->alloc(&d.posB1x_next, L)) ||
+            (s = bt->alloc(&d.inv_dtr_f, cap)) || (s = bt->alloc(&d.posB1x, L)) || (s = bt->alloc(&d.posB1x_next, L)) || (s = bt->alloc(&d.b1, L)) ||
             (s = bt->alloc(&d.posB1x_saved, NSAVE * L)) || (s = bt->alloc(&d.h, (size_t)SMAX * L)) ||
             (s = bt->alloc(&d.gS, L)) || (s = bt->alloc(&d.geS, L)) || (s = bt->alloc(&d.gfS, L)) ||
             (s = bt->alloc(&d.part, L * nchm * 8)) || (s = bt->alloc(&d.rowval, L)) ||
@@ -924,6 +932,9 @@ dyn_status dyn_batch_create(const dyn_batch_config* cfg, const dyn_batch_grid* g
         for (int b = 0; b < nquench; ++b) order[b] = b;
         std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return bt->qh[a].c.L > bt->qh[b].c.L; });
         std::vector<unsigned> it, ei;
+        // enough for the smaller CTA; with more threads the later items find no row
+        for (int b : order)
+            for (int g = 0; g < (bt->qh[b].c.L + 127) / 128; ++g) it.push_back(((unsigned)b << 16) | (unsigned)(SIDE_ITEM + g));
         for (int b : order)
             for (int i = 0; i < bt->qh[b].c.L; ++i) it.push_back(((unsigned)b << 16) | (unsigned)i);
         for (int b = 0; b < nquench; ++b)

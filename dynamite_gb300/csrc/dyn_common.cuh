@@ -20,6 +20,7 @@ struct DModel {
     int p, p2;
     double cA, cB, cC, cD, cE, cF;
     double T0, Gamma;
+    double iT0;  // 1 / T0
 };
 
 // pow_int (math_ops.cpp:7-21), same multiplication order, no contraction.
@@ -143,6 +144,43 @@ __device__ __forceinline__ double search_pos(int mode, const ListView& L, double
     return mode == 1 ? pos_lower_bound(L, El) : pos_binary(L, El);
 }
 
+// The interval of El in the time list: the largest k in [lo, hi] with list[k] <= El
+// (exact: integer compares on the bit patterns of the non-negative FP64 times).  The
+// caller brackets the answer: list[lo] <= El (or lo = 0) and k(El) <= hi.
+__device__ __forceinline__ int floor_index(const ListView& L, double El, int lo, int hi) {
+    const long long kE = okey(El);
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (okey(L.at(mid)) <= kE) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// The same interval searched outwards from a guess k in [0, L.n - 1] (the one of
+// the previous stage): two probes where it still holds, a doubling bracket otherwise.
+__device__ __forceinline__ int floor_index_near(const ListView& L, double El, int k) {
+    const long long kE = okey(El);
+    const int last = L.n - 1;
+    if (okey(L.at(k)) <= kE) {
+        int lo = k, step = 1;
+        while (lo + step <= last && okey(L.at(lo + step)) <= kE) { lo += step; step <<= 1; }
+        return step == 1 ? lo : floor_index(L, El, lo, min(lo + step - 1, last));
+    }
+    int hi = k, step = 1;
+    while (hi - step > 0 && okey(L.at(hi - step)) > kE) { hi -= step; step <<= 1; }
+    return floor_index(L, El, max(hi - step, 0), hi - 1);
+}
+
+// Which of a target's four B2 sums a stage has to form: bits 0..3 for S0, S1
+// (rows X-1, X), D1, D2 (derivative rows X, X+1; D2 only on the cubic branch).
+// key: the row whose sums are held; dirty: the first row rewritten since.
+__device__ __forceinline__ int b2_need(int X, int key, int dirty, bool cubic) {
+    const int all = cubic ? 15 : 7;
+    if (X != key) return all;
+    return (X - 1 >= dirty ? 1 : 0) | (X >= dirty ? 6 : 0) | (cubic && X + 1 >= dirty ? 8 : 0);
+}
+
 // Reduce-scatter of 8 per-lane values over a warp: afterwards lane l with
 // (l & 3) == 0 holds the warp total of value index ((l>>4)&1)*4+((l>>3)&1)*2+((l>>2)&1).
 // 9 adds per lane instead of 40 for eight independent butterflies.
@@ -172,6 +210,25 @@ __device__ __forceinline__ double warp_reduce8(const double v[8], int lane) {
 }
 __device__ __forceinline__ int warp_reduce8_index(int lane) {
     return ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+}
+
+// The same for 6 values: lane l with (l & 3) == 0 holds the total of value
+// warp_reduce6_index(l) where that is below 6 (8 adds per lane).
+__device__ __forceinline__ double warp_reduce6(const double v[6], int lane) {
+    const bool b16 = lane & 16, b8 = lane & 8, b4 = lane & 4;
+    double w[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        w[k] = (b16 ? v[k + 3] : v[k]) + __shfl_xor_sync(0xffffffffu, b16 ? v[k] : v[k + 3], 16);
+    const double x0 = (b8 ? w[2] : w[0]) + __shfl_xor_sync(0xffffffffu, b8 ? w[0] : w[2], 8);
+    const double x1 = w[1] + __shfl_xor_sync(0xffffffffu, w[1], 8);
+    double y = (b4 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, b4 ? x0 : x1, 4);
+    y += __shfl_xor_sync(0xffffffffu, y, 2);
+    y += __shfl_xor_sync(0xffffffffu, y, 1);
+    return y;
+}
+__device__ __forceinline__ int warp_reduce6_index(int lane) {
+    return (lane & 8) && (lane & 4) ? 6 : ((lane >> 4) & 1) * 3 + ((lane & 8) ? 2 : (lane >> 2) & 1);
 }
 
 // Programmatic dependent launch: a kernel launched with programmatic stream

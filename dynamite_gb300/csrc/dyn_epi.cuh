@@ -85,32 +85,58 @@ __device__ __forceinline__ double2 dot2s(const double* __restrict__ w, const dou
     return acc;
 }
 
-// B1 Hermite coefficients of one target row (index_vec.cu:399-441 form,
-// with the per-row division folded into c3).
-struct B1Row {
-    int F, cubic;
-    double c0, c1, c2, c3;
-};
-
-__device__ __forceinline__ B1Row b1_row(const DevCtx& c, double pos, int maxceil, int nrows) {
+// B1 interpolation of a row at position pos (index_vec.cu:399-441 form, with the
+// per-row division folded into c3); idtr(k) gives 1/delta_t_ratio of row k.  Written
+// out in fused operations so that every kernel that forms it rounds alike.
+template <typename InvDtr>
+__device__ __forceinline__ B1Row b1_at(double pos, int maxceil, int nrows, InvDtr idtr) {
     B1Row r;
     long long F = (long long)floor(pos);
     if (F < 1) F = 1; else if (F > maxceil) F = maxceil;
     r.F = (int)F;
-    const double u = (double)F - pos, u2 = u * u, u3 = u2 * u;
+    const double u = __dsub_rn((double)F, pos), u2 = __dmul_rn(u, u), u3 = __dmul_rn(u2, u);
     r.cubic = F < nrows - 1;
     if (r.cubic) {
-        r.c0 = 1.0 - 3.0 * u2 - 2.0 * u3;
-        r.c1 = 3.0 * u2 + 2.0 * u3;
-        r.c2 = u + 2.0 * u2 + u3;
-        r.c3 = (u2 + u3) * c.inv_dtr[F + 1];
+        r.c1 = fma(2.0, u3, __dmul_rn(3.0, u2));
+        r.c0 = __dsub_rn(1.0, r.c1);
+        r.c2 = __dadd_rn(fma(2.0, u2, u), u3);
+        r.c3 = __dmul_rn(__dadd_rn(u2, u3), idtr(r.F + 1));
     } else {
-        r.c0 = 1.0 - u2;
+        r.c0 = __dsub_rn(1.0, u2);
         r.c1 = u2;
-        r.c2 = u + u2;
+        r.c2 = __dadd_rn(u, u2);
         r.c3 = 0.0;
     }
     return r;
+}
+__device__ __forceinline__ B1Row b1_row(const DevCtx& c, double pos, int maxceil, int nrows) {
+    return b1_at(pos, maxceil, nrows, [&](int k) { return c.inv_dtr[k]; });
+}
+
+// What a stage needs once per target row and no target does: QK^{B1}[i,0] and rInt_i for
+// the epilogue, and the next stage's B1 position (theta_i T_next in the list that the row
+// this stage writes will end).  Its chains of dependent loads run beside the gathers, in
+// CTAs of their own.
+__device__ __forceinline__ void side_row(const DevCtx& c, const StageDev& sp, const B1Row& r, int i) {
+    const int L = c.L;
+    if (sp.T > 0.0) {
+        const double2 x0 = c.KR[(size_t)(r.F - 1) * L], x1 = c.KR[(size_t)r.F * L];
+        const double2 d1 = c.dKR[(size_t)r.F * L];
+        double qb = fma(-r.c2, d1.x, fma(r.c1, x1.x, __dmul_rn(r.c0, x0.x)));
+        double ri = fma(-r.c2, c.drvec[r.F], fma(r.c1, c.rvec[r.F], __dmul_rn(r.c0, c.rvec[r.F - 1])));
+        if (r.cubic) {
+            qb = fma(-r.c3, c.dKR[(size_t)(r.F + 1) * L].x, qb);
+            ri = fma(-r.c3, c.drvec[r.F + 1], ri);
+        }
+        c.rowval[i] = make_double2(qb, ri);
+    } else {
+        c.rowval[i] = make_double2(c.KR[0].x, c.rvec[0]);
+    }
+    if (i == 0) c.slots->q0 = c.KR[(size_t)(sp.nrows - 1) * L].x;
+    if (sp.kind != KIND_RHS && sp.pos_reuse < 0) {
+        const ListView lv{c.t1grid, sp.nrows_next, sp.T_next};
+        c.posB1x_next[i] = search_pos(c.search, lv, __dmul_rn(c.theta[i], sp.T_next));
+    }
 }
 
 namespace epi {
@@ -127,24 +153,33 @@ __device__ __forceinline__ void rows(const DevCtx& c, const StageDev& sp, const 
     for (int k = 0; k < EP_N; ++k) ep[k] = 0.0;
 
     if (tid < EPI_ROWS && i < L) {
-        double a[8];
+        double2 hs;
+        if (s == 0 && sp.fsal) {
+            hs = c.h[(size_t)(RK54_STAGES - 1) * L + i];
+        } else {
+            constexpr int NP = MIXED ? 8 : 6;
+            double a[NP];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) a[k] = 0.0;
-        for (int ch = 0; ch < c.nch; ++ch) {
+            for (int k = 0; k < NP; ++k) a[k] = 0.0;
+            for (int ch = 0; ch < c.nch; ++ch) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) a[k] += c.part[((size_t)i * c.nch + ch) * 8 + k];
+                for (int k = 0; k < NP; ++k) a[k] += c.part[((size_t)ch * NP + k) * L + i];
+            }
+            const double t = sp.T, th = c.theta[i];
+            const double tA = t * th, tR = t * (1.0 - th);
+            const double2 q = c.KR[(size_t)(sp.nrows - 1) * L + i];
+            const double2 rv = c.rowval[i];
+            const double rE = c.rowval[L - 1].y;
+            const double q0 = c.slots->q0;
+            const double fac1 = Sig<P, P2>::d1(Mo, q0) * Mo.iT0, fac2 = q0 * Mo.iT0;
+            double d1 = rv.x * fac1 + q.x * (-rE) + a[0] * tR + a[1] * tA;
+            if constexpr (MIXED) d1 += a[2] * tA;
+            constexpr int B = MIXED ? 3 : 2;  // a[B]: ConvR(QRA2, SigmaKB2) and on
+            double d2 = Sig<P, P2>::d1(Mo, rv.x) * fac2 + q.y * (2.0 * Mo.Gamma) + a[B] * tR + a[B + 1] * tA;
+            if constexpr (MIXED) d2 += a[5] * tA;
+            d2 -= q.x * rv.y;
+            hs = make_double2(d1 + d2 * th, (q.y * (-rE) + a[NP - 2] * tR) + (q.y * rv.y - a[NP - 1] * tR) * th);
         }
-        const double t = sp.T, th = c.theta[i];
-        const double tA = t * th, tR = t * (1.0 - th);
-        const double2 q = c.KR[(size_t)(sp.nrows - 1) * L + i];
-        const double2 rv = c.rowval[i];
-        const double rE = c.rowval[L - 1].y;
-        const double q0 = c.slots->q0;
-        const double fac1 = Sig<P, P2>::d1(Mo, q0) / Mo.T0, fac2 = q0 / Mo.T0;
-        const double d1 = rv.x * fac1 + q.x * (-rE) + a[0] * tR + a[1] * tA + a[2] * tA;
-        const double d2 = Sig<P, P2>::d1(Mo, rv.x) * fac2 + q.y * (2.0 * Mo.Gamma) + a[3] * tR + a[4] * tA +
-                          a[5] * tA - q.x * rv.y;
-        const double2 hs = make_double2(d1 + d2 * th, (q.y * (-rE) + a[6] * tR) + (q.y * rv.y - a[7] * tR) * th);
         c.h[(size_t)s * L + i] = hs;
         if (sp.kind == KIND_RHS) {
             c.rhs_out[i] = hs;
@@ -207,7 +242,7 @@ __device__ __forceinline__ void rows(const DevCtx& c, const StageDev& sp, const 
                 ep[6] = (tw * dsk) * g0.y;
                 ep[7] = (tw * sr) * h0.x;
                 ep[8] = (tw * sk) * h0.y;
-                if (i == 0) ep[9] = (dsk * g0.x + sk * h0.x) / Mo.T0;
+                if (i == 0) ep[9] = (dsk * g0.x + sk * h0.x) * Mo.iT0;
             }
             const double td = sp.tdiff;
             c.KR[(size_t)sp.n0 * L + i] = g;
@@ -226,13 +261,23 @@ __device__ __forceinline__ void rows(const DevCtx& c, const StageDev& sp, const 
             ep[0] = (tw * (dd * g.y)) * g.x;
             ep[1] = (tw * sk) * g.y;
             if (i == 0) {
-                ep[2] = (sk * g.x) / Mo.T0;
+                ep[2] = (sk * g.x) * Mo.iT0;
                 ep[12] = g.x;
                 ep[13] = sk;
             }
             // positions of the next stage (searched by the gather kernel)
-            const double pos = sp.pos_reuse >= 0 ? c.posB1x_saved[(size_t)sp.pos_reuse * L + i] : c.posB1x_next[i];
+            double pos;
+            if (s == 0 && sp.fsal) {  // no gather ran: searched here, in the list the row about to be written ends
+                const ListView lv{c.t1grid, sp.nrows_next, sp.T_next};
+                pos = search_pos(c.search, lv, __dmul_rn(c.theta[i], sp.T_next));
+            } else {
+                pos = sp.pos_reuse >= 0 ? c.posB1x_saved[(size_t)sp.pos_reuse * L + i] : c.posB1x_next[i];
+            }
             c.posB1x[i] = pos;
+            // the next stage's B1 row; delta_t_ratio of the row being written is not in memory yet
+            c.b1[i] = b1_at(pos, sp.nrows_next - 1 < 1 ? 1 : sp.nrows_next - 1, sp.nrows_next, [&](int k) {
+                return k != sp.n0 ? c.inv_dtr[k] : sp.dtr_new != 0.0 ? 1.0 / sp.dtr_new : 0.0;
+            });
             if (sp.pos_save >= 0) c.posB1x_saved[(size_t)sp.pos_save * L + i] = pos;
         }
     }
@@ -307,13 +352,14 @@ __device__ __forceinline__ void fold(const DevCtx& c, const StageDev& sp, const 
         c.t1grid[n0] = sp.T_next;
         c.dtr[n0] = sp.dtr_new;
         c.inv_dtr[n0] = sp.dtr_new != 0.0 ? 1.0 / sp.dtr_new : 0.0;
+        if (c.inv_len) c.inv_len[n0 - 1] = 1.0 / sp.tdiff;
         if constexpr (MIXED) {
             c.inv_dtr_f[n0] = sp.dtr_new != 0.0 ? (float)(1.0 / sp.dtr_new) : 0.0f;
             c.inv_len_f[n0 - 1] = (float)(1.0 / sp.tdiff);
         }
         if (sp.last) {
             sl->res_err = s_tot[10];
-            sl->res_energy = -(s_tot[1] + s_tot[13] / Mo.T0);
+            sl->res_energy = -(s_tot[1] + s_tot[13] * Mo.iT0);
             sl->res_r = r_new;
             sl->res_qk0 = s_tot[12];
             sl->res_dr = sl->dr;

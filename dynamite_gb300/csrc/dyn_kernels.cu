@@ -24,15 +24,6 @@
 
 namespace dyn {
 
-// Position of theta_i * T_next for the next stage (the row written by this
-// stage's epilogue becomes the last list entry), computed while the gather
-// kernel runs so the epilogue only copies it.
-__device__ __forceinline__ void next_position(const DevCtx& c, const StageDev& sp, int i) {
-    if (sp.kind == KIND_RHS || sp.pos_reuse >= 0) return;
-    const ListView lv{c.t1grid, sp.nrows_next, sp.T_next};
-    c.posB1x_next[i] = search_pos(c.search, lv, __dmul_rn(c.theta[i], sp.T_next));
-}
-
 // ------------------------------------------------------------------------
 // Log-space response (the reference's -R option).  QK is interpolated as in
 // the linear form; QR is interpolated as f = log QR with the derivatives
@@ -73,18 +64,65 @@ __device__ __forceinline__ double b1_log(double c0, double c1, double c2, double
 // k_main: fused gathers + Sigma + convolution products for one stage.
 // LOGR: QR gathers in log space (the last row's logs staged after it in
 // shared memory).
-template <int M, int K, int P, int P2, bool LOGR = false>
-__global__ void __launch_bounds__(128) k_main(const DevCtx c, const int s) {
+
+// f' and f'' of a target: neighbouring exponents share their power, q^(P-1) (cA + cB q)
+// and q^(P-2) (cC + cD q), one FP64 operation fewer each than Sig's two powers
+template <int P, int P2>
+struct SigT {
+    __device__ __forceinline__ static double d1(const DModel& M, double q) {
+        if constexpr (P >= 2 && P2 == P + 1) return ipow_c<P - 1>(q) * fma(M.cB, q, M.cA);
+        else return Sig<P, P2>::d1(M, q);
+    }
+    __device__ __forceinline__ static double d2(const DModel& M, double q) {
+        if constexpr (P >= 2 && P2 == P + 1) return ipow_c<P - 2>(q) * fma(M.cD, q, M.cC);
+        else return Sig<P, P2>::d2(M, q);
+    }
+    __device__ __forceinline__ static void d12(const DModel& M, double q, double& a, double& b) {
+        a = d1(M, q);
+        b = d2(M, q);
+    }
+};
+
+// One of the four B2 stencil sums of target ij (0: S0, 1: S1, 2: D1, 3: D2)
+template <int M>
+__device__ __forceinline__ double2 b2_sum(const DevCtx& c, const size_t ij, const int X, const int which, const int m) {
+    const size_t at = (size_t)(X - 1) * c.L + __ldg(c.iB2 + ij) + (size_t)(which == 0 ? 0 : which == 3 ? 2 : 1) * c.L;
+    return dot2g<M>(c.wB2 + ij * m, (which < 2 ? c.KR : c.dKR) + at, m);
+}
+
+// Bound by the FP64 pipe (2 lanes per SM and clock: a warp instruction holds it 16
+// cycles whatever its lanes do), so what counts is FP64 instructions per target: ~200
+// when every stage formed its four B2 sums (80), divided for its position (10) and kept
+// eight row sums; ~130 with the sums kept, stored inverse interval lengths, shared powers
+// and six row sums.  L = 512, 1500 rows: 111 us a stage before, 76 us after (pipe 86 %
+// busy); the first stage of a call, which forms all sums through the list, 105 us.
+//
+// KEEP: the B2 sums live in planes over the stages of a call (B2Mode).  The targets
+// that need a sum push it on a list in shared memory, the CTA's threads work the
+// list off with full warps whatever targets it came from, and every target then
+// reads its four sums back.  Without planes (KEEP false: the allocation-free
+// right-hand side, or no memory for them) every target forms its own.
+template <int M, int K, int P, int P2, bool LOGR, bool KEEP>
+__global__ void __launch_bounds__(64) k_main(const DevCtx c, const int s) {
     wait_prior_grid();
     const StageDev& sp = c.stages[s];
-    const int L = c.L, tpb = blockDim.x, i = blockIdx.y;
+    const int L = c.L, tpb = blockDim.x, nside = (L + tpb - 1) / tpb;
+    if (blockIdx.y < nside) {  // the rows' own work, tpb rows a CTA
+        const int r = blockIdx.y * tpb + threadIdx.x;
+        if (blockIdx.x == 0 && r < L) side_row(c, sp, c.b1[r], r);
+        return;
+    }
+    // rows near theta = 1 first: most of their targets read the row being written, the longest work
+    const int i = L - 1 - (blockIdx.y - nside);
+    const size_t L2 = (size_t)L * L;
     const int nrows = sp.nrows;
     const double t = sp.T;
     const bool live = t > 0.0;
     extern __shared__ double2 s_last[];
-    __shared__ double s_c[4];
-    __shared__ int s_bi[2];
-    __shared__ double s_red[4][8];
+    __shared__ double s_red[2][6];
+    __shared__ int s_X[KEEP ? 64 * K : 1];
+    __shared__ unsigned short s_job[KEEP ? 4 * 64 * K : 1];  // (local target << 2) | sum
+    __shared__ int s_njob;
 
     double* s_logR = reinterpret_cast<double*>(s_last + L);  // LOGR only: [L]
 
@@ -94,48 +132,100 @@ __global__ void __launch_bounds__(128) k_main(const DevCtx c, const int s) {
         s_last[k] = v;
         if constexpr (LOGR) s_logR[k] = v.y > 0.0 ? log(v.y) : v.y;
     }
-    if (threadIdx.x == 0) {
-        if (live) {
-            const B1Row r = b1_row(c, c.posB1x[i], sp.maxceil, nrows);
-            s_c[0] = r.c0; s_c[1] = r.c1; s_c[2] = r.c2; s_c[3] = r.c3;
-            s_bi[0] = r.F; s_bi[1] = r.cubic;
-            if (blockIdx.x == 0) {
-                // QK^{B1}[i,0] and rInt_i for the epilogue
-                const double2 x0 = c.KR[(size_t)(r.F - 1) * L], x1 = c.KR[(size_t)r.F * L];
-                const double2 d1 = c.dKR[(size_t)r.F * L];
-                double qb = r.c0 * x0.x + r.c1 * x1.x - r.c2 * d1.x;
-                double ri = r.c0 * c.rvec[r.F - 1] + r.c1 * c.rvec[r.F] - r.c2 * c.drvec[r.F];
-                if (r.cubic) {
-                    qb -= r.c3 * c.dKR[(size_t)(r.F + 1) * L].x;
-                    ri -= r.c3 * c.drvec[r.F + 1];
-                }
-                c.rowval[i] = make_double2(qb, ri);
-            }
-        } else {
-            s_bi[0] = 1; s_bi[1] = 0;
-            s_c[0] = s_c[1] = s_c[2] = s_c[3] = 0.0;
-            if (blockIdx.x == 0) c.rowval[i] = make_double2(c.KR[0].x, c.rvec[0]);
-        }
-        if (i == 0 && blockIdx.x == 0) c.slots->q0 = KRl[0].x;
-    }
-    if (threadIdx.x == 32 && blockIdx.x == 0) next_position(c, sp, i);
-    __syncthreads();
+    if (threadIdx.x == 0) s_njob = 0;
+    B1Row r1 = {};
+    if (live) r1 = c.b1[i];
 
     const DModel Mo = c.M;
     const int m = M > 0 ? M : c.m;
-    const double bc0 = s_c[0], bc1 = s_c[1], bc2 = s_c[2], bc3 = s_c[3];
-    const int F = s_bi[0], cubic1 = s_bi[1];
     const int maxX = sp.maxX;
     const double2 fill = c.KR[0];
     const ListView lv{c.t1grid, nrows, t};
     const double* pos2_src = sp.b2_reuse >= 0
-        ? (sp.b2_reuse == NSAVE ? c.posB2x : c.posB2x_saved + (size_t)sp.b2_reuse * L * L) : nullptr;
+        ? (sp.b2_reuse == NSAVE ? c.posB2x : c.posB2x_saved + (size_t)sp.b2_reuse * L2) : nullptr;
     double* pos2_dst = sp.b2_save >= 0
-        ? (sp.b2_save == NSAVE ? c.posB2x : c.posB2x_saved + (size_t)sp.b2_save * L * L) : nullptr;
+        ? (sp.b2_save == NSAVE ? c.posB2x : c.posB2x_saved + (size_t)sp.b2_save * L2) : nullptr;
+    const bool keep = KEEP && sp.b2_mode == B2_KEEP;
+    const int dirty = b2_dirty(sp);
+    __syncthreads();
 
-    double acc[8];
+    // ---- positions of the targets in the history: row X, offset x in its interval
+    int X[K];
+    double x[K];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) acc[k] = 0.0;
+    for (int kk = 0; kk < K; ++kk) {
+        const int j = blockIdx.x * tpb * K + kk * tpb + threadIdx.x;
+        const size_t ij = (size_t)i * L + j;
+        X[kk] = 1;
+        x[kk] = 0.0;
+        int need = 0;
+        if (live && j < L) {
+            const int key = keep ? c.b2key[ij] : 0;
+            if (pos2_src || sp.kind == KIND_RHS) {
+                const double pos2 = pos2_src ? pos2_src[ij] : search_pos(c.search, lv, __dmul_rn(__ldg(c.phi2 + ij), t));
+                long long Xl = (long long)pos2;
+                if (Xl > maxX) Xl = maxX;
+                if (Xl < 1) Xl = 1;
+                X[kk] = (int)Xl;
+                x[kk] = __dsub_rn(pos2, (double)Xl);
+                if (pos2_dst) pos2_dst[ij] = pos2;
+            } else {
+                const double El = __dmul_rn(__ldg(c.phi2 + ij), t);
+                const int k = key > 0 ? floor_index_near(lv, El, min(key, nrows) - 1) : floor_index(lv, El, 0, nrows - 1);
+                if (k >= nrows - 1) {
+                    X[kk] = nrows;
+                } else {
+                    x[kk] = __dmul_rn(__dsub_rn(El, lv.at(k)), __ldg(c.inv_len + k));
+                    X[kk] = k + 1;
+                }
+                if (pos2_dst) pos2_dst[ij] = (double)X[kk] + x[kk];
+                if (X[kk] > maxX) { x[kk] += (double)(X[kk] - maxX); X[kk] = maxX; }
+                if (X[kk] < 1) { x[kk] -= (double)(1 - X[kk]); X[kk] = 1; }
+            }
+            if constexpr (KEEP) {
+                need = b2_need(X[kk], key, dirty, X[kk] < nrows - 1);
+                s_X[kk * tpb + threadIdx.x] = X[kk];
+                if (X[kk] != key) c.b2key[ij] = X[kk];
+            }
+        }
+        if constexpr (KEEP) {
+            // push this target's sums: one reservation per warp, sum by sum in lane order
+            const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
+            unsigned b[4];
+            int tot = 0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                b[q] = __ballot_sync(0xffffffffu, need >> q & 1);
+                tot += __popc(b[q]);
+            }
+            if (tot) {
+                int base = 0;
+                if ((threadIdx.x & 31) == 0) base = atomicAdd(&s_njob, tot);
+                base = __shfl_sync(0xffffffffu, base, 0);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (need >> q & 1) s_job[base + __popc(b[q] & lt)] = (unsigned short)((kk * tpb + threadIdx.x) << 2 | q);
+                    base += __popc(b[q]);
+                }
+            }
+        }
+    }
+    if constexpr (KEEP) {
+        __syncthreads();
+        const int nj = s_njob;
+        for (int q = threadIdx.x; q < nj; q += tpb) {
+            const int job = s_job[q], tl = job >> 2, which = job & 3;
+            const size_t ij = (size_t)i * L + blockIdx.x * tpb * K + tl;
+            c.b2s[which * L2 + ij] = b2_sum<M>(c, ij, s_X[tl], which, m);
+        }
+        __syncthreads();
+    }
+
+    const double bc0 = r1.c0, bc1 = r1.c1, bc2 = r1.c2, bc3 = r1.c3;
+    const int F = r1.F, cubic1 = r1.cubic;
+    double acc[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) acc[k] = 0.0;
 
 #pragma unroll
     for (int kk = 0; kk < K; ++kk) {
@@ -167,71 +257,66 @@ __global__ void __launch_bounds__(128) k_main(const DevCtx c, const int s) {
                     if constexpr (LOGR) b1.y = b1_log(bc0, bc1, bc2, cubic1 ? bc3 : 0.0, x0.y, x1.y, d1.y, d2.y, b1.y);
                 }
                 {
-                    double pos2;
-                    if (pos2_src) pos2 = pos2_src[ij];
-                    else {
-                        pos2 = search_pos(c.search, lv, __dmul_rn(__ldg(c.phi2 + ij), t));
-                        if (pos2_dst) pos2_dst[ij] = pos2;
+                    const bool cubic2 = X[kk] < nrows - 1;
+                    const double x1 = x[kk], x2 = x1 * x1;
+                    double2 S0, S1, D1, D2 = make_double2(0.0, 0.0);
+                    if constexpr (KEEP) {
+                        S0 = c.b2s[ij];
+                        S1 = c.b2s[L2 + ij];
+                        D1 = c.b2s[2 * L2 + ij];
+                        if (cubic2) D2 = c.b2s[3 * L2 + ij];
+                    } else {
+                        S0 = b2_sum<M>(c, ij, X[kk], 0, m);
+                        S1 = b2_sum<M>(c, ij, X[kk], 1, m);
+                        D1 = b2_sum<M>(c, ij, X[kk], 2, m);
+                        if (cubic2) D2 = b2_sum<M>(c, ij, X[kk], 3, m);
                     }
-                    long long X = (long long)pos2;
-                    if (X > maxX) X = maxX;
-                    if (X < 1) X = 1;
-                    const double x = pos2 - (double)X, x2 = x * x, x3 = x2 * x;
-                    const size_t base = (size_t)(X - 1) * L + __ldg(c.iB2 + ij);
-                    const double* w = c.wB2 + ij * m;
-                    const double2 S0 = dot2g<M>(w, c.KR + base, m);
-                    const double2 S1 = dot2g<M>(w, c.KR + base + L, m);
-                    const double2 D1 = dot2g<M>(w, c.dKR + base + L, m);
-                    if (X < nrows - 1) {
-                        const double2 D2 = dot2g<M>(w, c.dKR + base + 2 * L, m);
-                        const double e0 = 1.0 - 3.0 * x2 + 2.0 * x3, e1 = x - 2.0 * x2 + x3;
-                        const double e2 = 3.0 * x2 - 2.0 * x3;
-                        const double e3 = (x3 - x2) * c.inv_dtr[X + 1];
-                        b2.x = e0 * S0.x + e1 * D1.x + e2 * S1.x + e3 * D2.x;
-                        b2.y = e0 * S0.y + e1 * D1.y + e2 * S1.y + e3 * D2.y;
+                    if (cubic2) {
+                        // Hermite weights through y = x^3 - x^2: e1 = x - x^2 + y, e2 = x^2 - 2 y, e0 = 1 - e2
+                        const double y = fma(x2, x1, -x2), e1 = (x1 - x2) + y, e2 = fma(-2.0, y, x2), e0 = 1.0 - e2;
+                        const double e3 = y * c.inv_dtr[X[kk] + 1];
+                        b2.x = fma(e3, D2.x, fma(e2, S1.x, fma(e1, D1.x, e0 * S0.x)));
+                        b2.y = fma(e3, D2.y, fma(e2, S1.y, fma(e1, D1.y, e0 * S0.y)));
                         // index_mat.cu:203-212: Hermite of log of the row sums
                         if (LOGR && S0.y > 0.0 && S1.y > 0.0)
                             b2.y = exp(e0 * log(S0.y) + e1 * (D1.y / S0.y) + e2 * log(S1.y) + e3 * (D2.y / S1.y));
                     } else {
-                        const double e0 = 1.0 - x2, e2 = x - x2;
-                        b2.x = e0 * S0.x + x2 * S1.x + e2 * D1.x;
-                        b2.y = e0 * S0.y + x2 * S1.y + e2 * D1.y;
+                        const double e0 = 1.0 - x2, e2 = x1 - x2;
+                        b2.x = fma(e2, D1.x, fma(x2, S1.x, e0 * S0.x));
+                        b2.y = fma(e2, D1.y, fma(x2, S1.y, e0 * S0.y));
                         if (LOGR && S0.y > 0.0 && S1.y > 0.0)  // index_mat.cu:216-222
                             b2.y = exp(e0 * log(S0.y) + x2 * log(S1.y) + e2 * (D1.y / S0.y));
                     }
-                    if (c.rec) c.rec[ij] = GatherRec{a1, a2, b1, b2, x, (int)X, 0};
+                    if (c.rec) c.rec[ij] = GatherRec{a1, a2, b1, b2, x1, X[kk], 0};
                 }
             } else {
                 a1 = a2 = b1 = b2 = fill;
             }
             double sKA1, dA1, sKB1, dB1, sKB2, dB2;
-            Sig<P, P2>::d12(Mo, a1.x, sKA1, dA1);
-            const double sRA1 = dA1 * a1.y;
-            const double sRA2 = Sig<P, P2>::d2(Mo, a2.x) * a2.y;
-            Sig<P, P2>::d12(Mo, b1.x, sKB1, dB1);
-            const double sRB1 = dB1 * b1.y;
-            Sig<P, P2>::d12(Mo, b2.x, sKB2, dB2);
-            const double sRB2 = dB2 * b2.y;
+            SigT<P, P2>::d12(Mo, a1.x, sKA1, dA1);
+            SigT<P, P2>::d12(Mo, b1.x, sKB1, dB1);
+            SigT<P, P2>::d12(Mo, b2.x, sKB2, dB2);
             const double wj = __ldg(c.integ + j);
-            const double wRA2 = wj * sRA2, wQRA2 = wj * a2.y;
+            const double wQRA2 = wj * a2.y, wRA2 = wQRA2 * SigT<P, P2>::d2(Mo, a2.x);
             acc[0] = fma(wRA2, b2.x, acc[0]);            // ConvR(SigmaRA2, QKB2)
-            acc[1] = fma(wj * sRA1, b1.x, acc[1]);       // ConvA(SigmaRA1, QKB1)
-            acc[2] = fma(wj * sKA1, b1.y, acc[2]);       // ConvA(SigmaKA1, QRB1)
-            acc[3] = fma(wQRA2, sKB2, acc[3]);           // ConvR(QRA2, SigmaKB2)
-            acc[4] = fma(wj * a1.y, sKB1, acc[4]);       // ConvA(QRA1, SigmaKB1)
-            acc[5] = fma(wj * a1.x, sRB1, acc[5]);       // ConvA(QKA1, SigmaRB1)
-            acc[6] = fma(wRA2, b2.y, acc[6]);            // ConvR(SigmaRA2, QRB2)
-            acc[7] = fma(wQRA2, sRB2, acc[7]);           // ConvR(QRA2, SigmaRB2)
+            // ConvA(SigmaRA1, QKB1) + ConvA(SigmaKA1, QRB1)
+            acc[1] = fma(wj, fma(sKA1, b1.y, (dA1 * a1.y) * b1.x), acc[1]);
+            acc[2] = fma(wQRA2, sKB2, acc[2]);           // ConvR(QRA2, SigmaKB2)
+            // ConvA(QRA1, SigmaKB1) + ConvA(QKA1, SigmaRB1)
+            acc[3] = fma(wj, fma(a1.x, dB1 * b1.y, a1.y * sKB1), acc[3]);
+            acc[4] = fma(wRA2, b2.y, acc[4]);            // ConvR(SigmaRA2, QRB2)
+            acc[5] = fma(wQRA2, dB2 * b2.y, acc[5]);     // ConvR(QRA2, SigmaRB2)
         }
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const double r = warp_reduce8(acc, lane);
-    if ((lane & 3) == 0) s_red[warp][warp_reduce8_index(lane)] = r;
+    const double r = warp_reduce6(acc, lane);
+    const int ri = warp_reduce6_index(lane);
+    if ((lane & 3) == 0 && ri < 6) s_red[warp][ri] = r;
     __syncthreads();
-    if (threadIdx.x < 8) {
+    if (threadIdx.x < 6) {
         double v = 0.0;
         for (int w = 0; w < (tpb >> 5); ++w) v += s_red[w][threadIdx.x];
-        c.part[((size_t)i * gridDim.x + blockIdx.x) * 8 + threadIdx.x] = v;
+        c.part[((size_t)blockIdx.x * 6 + threadIdx.x) * L + i] = v;
     }
 }
 
@@ -259,6 +344,7 @@ __global__ void k_pos_init(const DevCtx c, const int nrows) {
     for (int i = threadIdx.x; i < L; i += blockDim.x) {
         const double p = search_pos(c.search, lv, __dmul_rn(c.theta[i], T));
         c.posB1x[i] = p;
+        c.b1[i] = b1_row(c, p, nrows - 1 < 1 ? 1 : nrows - 1, nrows);
         mx = fmax(mx, p);
     }
     for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -315,6 +401,7 @@ __global__ void k_pos_b1_exact(const DevCtx c, const int nrows, const double* po
     for (int i = threadIdx.x; i < L; i += blockDim.x) {
         const double p = pos1_given ? pos1_given[i] : search_pos(c.search, lv, mul(c.theta[i], T));
         c.posB1x[i] = p;
+        c.b1[i] = b1_row(c, p, nrows - 1 < 1 ? 1 : nrows - 1, nrows);
         mx = i == 0 ? p : fmax(mx, p);
     }
     for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -683,22 +770,24 @@ __global__ void k_fp64_probe(double* out, int iters) {
 
 // ------------------------------------------------------------------------
 // launch wrappers
-template <int M, int K, int P, int P2, bool LOGR>
+template <int M, int K, int P, int P2, bool LOGR, bool KEEP>
 static cudaError_t launch_main_t(const DevCtx& c, int s, cudaStream_t st) {
-    dim3 grid(c.nch, c.L), block(c.tpb);
+    dim3 grid(c.nch, c.L + (c.L + c.tpb - 1) / c.tpb), block(c.tpb);
     const size_t smem = (size_t)c.L * (LOGR ? sizeof(double2) + sizeof(double) : sizeof(double2));
     static std::atomic<unsigned long long> devs{0};
-    const cudaError_t e = raise_smem_limit(k_main<M, K, P, P2, LOGR>, smem, 4096 * (int)(smem / c.L), devs);
+    const cudaError_t e = raise_smem_limit(k_main<M, K, P, P2, LOGR, KEEP>, smem, 4096 * (int)(smem / c.L), devs);
     if (e != cudaSuccess) return e;
-    return launch_pdl(k_main<M, K, P, P2, LOGR>, grid, block, smem, st, c, s);
+    return launch_pdl(k_main<M, K, P, P2, LOGR, KEEP>, grid, block, smem, st, c, s);
 }
 
 template <int M, int P, int P2, bool LOGR>
 static cudaError_t launch_main_kl(const DevCtx& c, int s, cudaStream_t st) {
+    if (c.b2key) return c.kpt == 1 ? launch_main_t<M, 1, P, P2, LOGR, true>(c, s, st)
+                                   : launch_main_t<M, 2, P, P2, LOGR, true>(c, s, st);
     switch (c.kpt) {
-        case 1: return launch_main_t<M, 1, P, P2, LOGR>(c, s, st);
-        case 2: return launch_main_t<M, 2, P, P2, LOGR>(c, s, st);
-        default: return launch_main_t<M, 4, P, P2, LOGR>(c, s, st);
+        case 1: return launch_main_t<M, 1, P, P2, LOGR, false>(c, s, st);
+        case 2: return launch_main_t<M, 2, P, P2, LOGR, false>(c, s, st);
+        default: return launch_main_t<M, 4, P, P2, LOGR, false>(c, s, st);
     }
 }
 
@@ -709,20 +798,20 @@ static cudaError_t launch_main_k(const DevCtx& c, int s, cudaStream_t st) {
 }
 
 template <int P, int P2>
-static cudaError_t launch_stage_pp(const DevCtx& c, int s, cudaStream_t st) {
-    cudaError_t e;
-    if (c.mixed) e = launch_main_mixed(c, s, st);
-    else e = c.m == 10 ? launch_main_k<10, P, P2>(c, s, st) : launch_main_k<0, P, P2>(c, s, st);
+static cudaError_t launch_stage_pp(const DevCtx& c, int s, cudaStream_t st, bool gather) {
+    cudaError_t e = cudaSuccess;
+    if (gather && c.mixed) e = launch_main_mixed(c, s, st);
+    else if (gather) e = c.m == 10 ? launch_main_k<10, P, P2>(c, s, st) : launch_main_k<0, P, P2>(c, s, st);
     if (e != cudaSuccess) return e;
     const int G = (c.L + EPI_ROWS - 1) / EPI_ROWS;
     if (c.mixed) return launch_pdl(k_epi<P, P2, true>, dim3(G), dim3(EPI_T), 0, st, c, s);
     return launch_pdl(k_epi<P, P2, false>, dim3(G), dim3(EPI_T), 0, st, c, s);
 }
 
-cudaError_t launch_stage(const DevCtx& c, int s, cudaStream_t st) {
-    if (c.M.p == 3 && c.M.p2 == 4) return launch_stage_pp<3, 4>(c, s, st);
-    if (c.M.p == 3 && c.M.p2 == 0) return launch_stage_pp<3, 0>(c, s, st);
-    return launch_stage_pp<-1, -1>(c, s, st);
+cudaError_t launch_stage(const DevCtx& c, int s, cudaStream_t st, bool gather) {
+    if (c.M.p == 3 && c.M.p2 == 4) return launch_stage_pp<3, 4>(c, s, st, gather);
+    if (c.M.p == 3 && c.M.p2 == 0) return launch_stage_pp<3, 0>(c, s, st, gather);
+    return launch_stage_pp<-1, -1>(c, s, st, gather);
 }
 
 template <int P, int P2>

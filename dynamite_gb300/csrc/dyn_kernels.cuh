@@ -8,6 +8,7 @@
 namespace dyn {
 
 constexpr int SMAX = 32;      // most stages of one step (SERK2 with q <= 16)
+constexpr int RK54_STAGES = 7;
 constexpr int NSAVE = 3;      // SSPRK(10,4) keeps positions of stages 2..4
 constexpr int EPI_T = 32;     // threads per epilogue CTA (one warp)
 constexpr int EPI_ROWS = 32;  // rows per epilogue CTA (one row per lane; spreading rows over
@@ -15,6 +16,15 @@ constexpr int EPI_ROWS = 32;  // rows per epilogue CTA (one row per lane; spread
 constexpr int EP_N = 16;      // per-CTA epilogue partials
 
 enum StageKind { KIND_TABLEAU = 0, KIND_SERK = 1, KIND_RHS = 2 };
+
+// What a stage does with the B2 row sums held in DevCtx::b2key and its planes.
+// A target's four stencil sums (S0, S1 over (QK, QR) of rows X-1, X; D1, D2 over
+// (dQK, dQR) of rows X, X+1) depend on the stage only through its row X and
+// through rows that were rewritten since: between two stages of a step phi2 t
+// moves by a fraction of one interval, so few targets change X, and the only
+// rewritten row is the one the step writes.  The sums are kept within one call
+// (dyn_update, dyn_run, dyn_batch_run); its first stage computes all of them.
+enum B2Mode { B2_FILL = 0, B2_KEEP = 1 };
 
 // One RK stage as the device sees it; the host fills an array of these per
 // step (pinned buffer -> one H2D copy), so a captured graph replays any step.
@@ -26,7 +36,8 @@ struct StageDev {
     int ncoef, serk_mode;    // serk_mode: 0 first stage, 1 even, 2 odd
     int maxceil, maxX;       // B1 Floor clamp and B2 row clamp of this stage (from nrows)
     int fresh;               // 1: the gather searches the B1 positions itself (after a rollback)
-    int pad_;
+    int fsal;                // 1: the right-hand side is the previous step's last one (RK54 follows RK54): no gather
+    int b2_mode;             // B2Mode of this stage (single contexts; the batch's is in its plan)
     double T;        // t1grid.back() while this stage's RHS is evaluated
     double T_next;   // time of the row this stage writes
     double tdiff;    // T_next - t1grid[n0-1]
@@ -46,6 +57,13 @@ struct Slots {
     int pad;
     // step result, written by the last epilogue block of the last stage
     double res_err, res_energy, res_r, res_qk0, res_dr;
+};
+
+// B1 interpolation of one target row: the interval F and the Hermite weights on C/R rows
+// F-1, F (c0, c1) and derivative rows F, F+1 (-c2, -c3; c3 has the 1/delta_t_ratio)
+struct B1Row {
+    double c0, c1, c2, c3;
+    int F, cubic;
 };
 
 // Per-target gathered values of one stage, recorded by k_main when
@@ -81,14 +99,20 @@ struct DevCtx {
     double* drvec;
     double* posB1x;        // [L]
     double* posB1x_next;   // [L] next stage's positions, written by the gather kernel
+    B1Row* b1;             // [L] B1 rows of the stage about to run (from posB1x)
     double* posB1x_saved;  // [NSAVE][L]
     double* posB2x;        // [L*L]
     double* posB2x_saved;  // [NSAVE][L*L]
+    double* inv_len;       // [cap] 1/(t1grid[k+1]-t1grid[k]) (FP64 contexts)
+    int* b2key;            // [L*L] row X whose B2 sums the planes hold (null: none kept)
+    double2* b2s;          // [4][L*L] S0, S1, D1, D2 (FP64 form)
+    float2* b2f;           // [4][L*L] S0, S1, D1, D2 (mixed 1); [2][L*L] D1, D2 (mixed 2)
+    float4* b2q;           // [2][L*L] S0, S1 as (QK hi, lo, QR hi, lo) (mixed 2)
     double2* h;            // [SMAX][L]
     double2* gS;           // SERK running stage value [L]
     double2* geS;          // SERK previous odd value [L]
     double2* gfS;          // SERK combination [L]
-    double* part;          // [L][nch][8]
+    double* part;          // [nch][6 or 8][L] row sums: FP64 form 6 (the two ConvA pairs added), mixed forms 8
     double2* rowval;       // [L] (QK^{B1}[i,0], rInt_i)
     double* epart;         // [G][EP_N]
     Slots* slots;
@@ -114,6 +138,10 @@ struct DevCtx {
     double* rint;          // [L]
     GatherRec* rec;        // [L*L] gathered values of this stage, or null
 };
+
+// The first history row that may have changed since the previous stage's gather:
+// the row the step writes, or at stage 0 the one the previous step finished
+__host__ __device__ inline int b2_dirty(const StageDev& sp) { return sp.s == 0 ? sp.n0 - 1 : sp.n0; }
 
 // Adjoint state of the FP64 path (dyn_adjoint.cu): cotangents of the
 // history and per-step stage snapshots from the recompute.
@@ -171,6 +199,7 @@ inline DModel make_model(int p, int p2, double lambda, double T0, double Gamma) 
     M.cF = (1 - lambda) * p2 * (p2 - 1) * (p2 - 2);
     M.T0 = T0;
     M.Gamma = Gamma;
+    M.iT0 = 1.0 / T0;
     return M;
 }
 
@@ -224,7 +253,8 @@ cudaError_t launch_tail_fit(const DevCtx& c, int nrows, int rollback_loop, doubl
                             cudaStream_t st);
 
 // launch wrappers (dyn_kernels.cu)
-cudaError_t launch_stage(const DevCtx& c, int s, cudaStream_t st);
+// gather false: the epilogue alone (StageDev::fsal)
+cudaError_t launch_stage(const DevCtx& c, int s, cudaStream_t st, bool gather = true);
 cudaError_t launch_main_only(const DevCtx& c, int s, cudaStream_t st);
 cudaError_t launch_epi_only(const DevCtx& c, int s, cudaStream_t st);
 cudaError_t launch_pos_init(const DevCtx& c, int nrows, cudaStream_t st);

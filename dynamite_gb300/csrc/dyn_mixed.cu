@@ -25,8 +25,13 @@ __global__ void __launch_bounds__(128, K == 1 ? 10 : 4) k_main_mixed(const DevCt
     const StageDev& sp = c.stages[s];
     extern __shared__ float2 s_lastf[];
     __shared__ mixed::RowShared sh;
-    const int i = blockIdx.y;
-    mixed::row_setup(c, sp, i, blockIdx.x == 0, s_lastf, sh);
+    const int nside = (c.L + blockDim.x - 1) / blockDim.x;
+    if (blockIdx.y < nside) {
+        if (blockIdx.x == 0) mixed::side_rows<false>(c, sp, blockIdx.y);
+        return;
+    }
+    const int i = blockIdx.y - nside;
+    mixed::row_setup<false>(c, sp, i, s_lastf, sh);
     __syncthreads();
     mixed::chunk_sums<M, K, P, P2>(c, sp, blockIdx.x, 0, s_lastf, sh, i);
     __syncthreads();
@@ -42,9 +47,14 @@ __global__ void __launch_bounds__(128, K == 1 ? 8 : 4) k_main_df(const DevCtx c,
     extern __shared__ float2 s_row[];  // [L+2] hi, [L+2] lo of the last history row
     __shared__ mixed::RowShared sh;
     __shared__ float s_clo[4];
-    const int i = blockIdx.y;
+    const int nside = (c.L + blockDim.x - 1) / blockDim.x;
+    if (blockIdx.y < nside) {
+        if (blockIdx.x == 0) mixed::side_rows<false>(c, sp, blockIdx.y);
+        return;
+    }
+    const int i = blockIdx.y - nside;
     float2* s_lo = s_row + (c.L + 2);
-    mixed::row_setup(c, sp, i, blockIdx.x == 0, s_row, sh, s_clo);
+    mixed::row_setup<false>(c, sp, i, s_row, sh, s_clo);
     mdf::stage_lo(c, sp, s_lo);
     __syncthreads();
     mdf::chunk_dd<M, K, P, P2>(c, sp, blockIdx.x, 0, s_row, s_lo, s_clo, sh, i);
@@ -56,7 +66,7 @@ namespace {
 
 template <int M, int K, int P, int P2>
 cudaError_t launch_df(const DevCtx& c, int s, cudaStream_t st) {
-    dim3 grid(c.nch, c.L), block(c.tpb);
+    dim3 grid(c.nch, c.L + (c.L + c.tpb - 1) / c.tpb), block(c.tpb);
     const size_t smem = 2 * (size_t)(c.L + 2) * sizeof(float2);  // > 48 KB from L = 3071 on
     static std::atomic<unsigned long long> devs{0};
     const cudaError_t e = raise_smem_limit(k_main_df<M, K, P, P2>, smem, 2 * (4096 + 2) * (int)sizeof(float2), devs);
@@ -67,7 +77,7 @@ cudaError_t launch_df(const DevCtx& c, int s, cudaStream_t st) {
 template <int M, int K, int P, int P2>
 cudaError_t launch_t(const DevCtx& c, int s, cudaStream_t st) {
     if (c.mixed == 2) return launch_df<M, K, P, P2>(c, s, st);
-    dim3 grid(c.nch, c.L), block(c.tpb);
+    dim3 grid(c.nch, c.L + (c.L + c.tpb - 1) / c.tpb), block(c.tpb);
     return launch_pdl(k_main_mixed<M, K, P, P2>, grid, block, (size_t)(c.L + 2) * sizeof(float2), st, c, s);
 }
 

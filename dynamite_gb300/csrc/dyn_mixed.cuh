@@ -3,7 +3,7 @@
 // shared by the single-quench kernel (dyn_mixed.cu) and the batched
 // persistent kernel (dyn_batch.cu) so that both run the same arithmetic.
 #pragma once
-#include "dyn_kernels.cuh"
+#include "dyn_epi.cuh"
 
 namespace dyn {
 namespace mixed {
@@ -241,19 +241,6 @@ __device__ __forceinline__ void warp_reduce8_pair(const float hv[8], const float
     Lo = yl;
 }
 
-// The interval of El in the time list: the largest k in [lo, hi] with list[k] <= El
-// (exact: integer compares on the bit patterns of the non-negative FP64 times).  The
-// caller brackets the answer: list[lo] <= El (or lo = 0) and k(El) <= hi.
-__device__ __forceinline__ int floor_index(const ListView& L, double El, int lo, int hi) {
-    const long long kE = okey(El);
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (okey(L.at(mid)) <= kE) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
 // The 1-based position of El in the list split into floor X and FP32 offset x from
 // its interval k: X = k + 1, x = (El - list[k]) / (list[k+1] - list[k]) with one
 // FP64 difference scaled by the stored FP32 inverse length (El at or past the last
@@ -277,13 +264,24 @@ struct RowShared {
 };
 
 // Row set-up for target row i: stages the last history row (FP32 mirror) in
-// shared memory and forms the row's B1 Hermite constants in FP64 from the
-// master history.  With `first` set (one block per row) it also writes the
-// row's QK^{B1}[i,0] and rInt_i, C(t,0) (row 0) and the next stage's B1
-// position.  A stage flagged `fresh` searches the row's B1 position itself
-// (after a rollback) instead of reading the one the previous stage left.
-__device__ __forceinline__ void row_setup(const DevCtx& c, const StageDev& sp, const int i, const bool first,
-                                          float2* s_lastf, RowShared& sh, float* clo = nullptr) {
+// shared memory, rounds the row's B1 weights to FP32 (clo: their low parts) and
+// brackets the B2 intervals of its targets.  A stage flagged `fresh` (after a
+// rollback or an upload) searches the row's B1 position itself instead of
+// taking the row the previous stage's epilogue left.
+// Only the batch plans such stages (FRESH); the search stays out of line, off the
+// gather's registers.
+static __device__ __noinline__ void fresh_b1(const DevCtx& c, const StageDev& sp, const int i, B1Row* out) {
+    *out = b1_row(c, search_pos(c.search, ListView{c.t1grid, sp.nrows, sp.T}, __dmul_rn(c.theta[i], sp.T)), sp.maxceil,
+                  sp.nrows);
+}
+template <bool FRESH>
+__device__ __forceinline__ void stage_b1(const DevCtx& c, const StageDev& sp, const int i, B1Row* out) {
+    if (FRESH && sp.fresh) fresh_b1(c, sp, i, out);
+    else *out = c.b1[i];
+}
+template <bool FRESH>
+__device__ __forceinline__ void row_setup(const DevCtx& c, const StageDev& sp, const int i, float2* s_lastf,
+                                          RowShared& sh, float* clo = nullptr) {
     const int L = c.L, tpb = blockDim.x;
     const int nrows = sp.nrows;
     const double t = sp.T;
@@ -292,44 +290,15 @@ __device__ __forceinline__ void row_setup(const DevCtx& c, const StageDev& sp, c
     for (int k = threadIdx.x; k < L; k += tpb) s_lastf[k] = KRl[k];
     if (threadIdx.x == 0) s_lastf[L] = make_float2(0.f, 0.f), s_lastf[L + 1] = make_float2(0.f, 0.f);
     if (threadIdx.x == 0) {
-        if (live) {
-            const double pos = sp.fresh ? search_pos(c.search, ListView{c.t1grid, nrows, t}, __dmul_rn(c.theta[i], t))
-                                        : c.posB1x[i];
-            long long F = (long long)floor(pos);
-            if (F < 1) F = 1; else if (F > sp.maxceil) F = sp.maxceil;
-            const double u = (double)F - pos, u2 = u * u, u3 = u2 * u;
-            const int cubic = F < nrows - 1;
-            double c0, c1, c2, c3;
-            if (cubic) {
-                c0 = 1.0 - 3.0 * u2 - 2.0 * u3; c1 = 3.0 * u2 + 2.0 * u3; c2 = u + 2.0 * u2 + u3;
-                c3 = (u2 + u3) * c.inv_dtr[F + 1];
-            } else {
-                c0 = 1.0 - u2; c1 = u2; c2 = u + u2; c3 = 0.0;
-            }
-            sh.c[0] = (float)c0; sh.c[1] = (float)c1; sh.c[2] = (float)c2; sh.c[3] = (float)c3;
-            if (clo) {
-                clo[0] = (float)(c0 - (double)sh.c[0]); clo[1] = (float)(c1 - (double)sh.c[1]);
-                clo[2] = (float)(c2 - (double)sh.c[2]); clo[3] = (float)(c3 - (double)sh.c[3]);
-            }
-            sh.bi[0] = (int)F; sh.bi[1] = cubic;
-            if (first) {
-                const double2 x0 = c.KR[(size_t)(F - 1) * L], x1 = c.KR[(size_t)F * L];
-                const double2 d1 = c.dKR[(size_t)F * L];
-                double qb = c0 * x0.x + c1 * x1.x - c2 * d1.x;
-                double ri = c0 * c.rvec[F - 1] + c1 * c.rvec[F] - c2 * c.drvec[F];
-                if (cubic) {
-                    qb -= c3 * c.dKR[(size_t)(F + 1) * L].x;
-                    ri -= c3 * c.drvec[F + 1];
-                }
-                c.rowval[i] = make_double2(qb, ri);
-            }
-        } else {
-            sh.bi[0] = 1; sh.bi[1] = 0;
-            sh.c[0] = sh.c[1] = sh.c[2] = sh.c[3] = 0.f;
-            if (clo) clo[0] = clo[1] = clo[2] = clo[3] = 0.f;
-            if (first) c.rowval[i] = make_double2(c.KR[0].x, c.rvec[0]);
+        B1Row r = {};
+        r.F = 1;
+        if (live) stage_b1<FRESH>(c, sp, i, &r);
+        sh.bi[0] = r.F; sh.bi[1] = r.cubic;
+        sh.c[0] = (float)r.c0; sh.c[1] = (float)r.c1; sh.c[2] = (float)r.c2; sh.c[3] = (float)r.c3;
+        if (clo) {
+            clo[0] = (float)(r.c0 - (double)sh.c[0]); clo[1] = (float)(r.c1 - (double)sh.c[1]);
+            clo[2] = (float)(r.c2 - (double)sh.c[2]); clo[3] = (float)(r.c3 - (double)sh.c[3]);
         }
-        if (i == 0 && first) c.slots->q0 = c.KR[(size_t)(nrows - 1) * L].x;
     }
     // B2 brackets: phi2 is non-decreasing along a row (checked when the tables are
     // loaded), so every target of 32-target segment w has its interval in
@@ -342,12 +311,16 @@ __device__ __forceinline__ void row_setup(const DevCtx& c, const StageDev& sp, c
             sh.seg[w] = floor_index(lv, __dmul_rn(c.phi2[(size_t)i * L + j], t), 0, nrows - 1);
         }
     }
-    if (threadIdx.x == 32 && first && sp.kind != KIND_RHS && sp.pos_reuse < 0) {
-        // next stage's B1 position of this row (the row this stage writes
-        // becomes the last list entry)
-        const ListView lvn{c.t1grid, sp.nrows_next, sp.T_next};
-        c.posB1x_next[i] = search_pos(c.search, lvn, __dmul_rn(c.theta[i], sp.T_next));
-    }
+}
+
+// The rows' own work (side_row) for rows blk*blockDim.x on, one thread a row
+template <bool FRESH>
+__device__ __forceinline__ void side_rows(const DevCtx& c, const StageDev& sp, const int blk) {
+    const int i = blk * blockDim.x + threadIdx.x;
+    if (i >= c.L) return;
+    B1Row r = {};
+    if (sp.T > 0.0) stage_b1<FRESH>(c, sp, i, &r);
+    side_row(c, sp, r, i);
 }
 
 // One chunk of tpb*K targets of row i: A1/A2 from the staged row, B1 and B2
@@ -496,7 +469,7 @@ __device__ __forceinline__ void fold_chunks(const DevCtx& c, const int i, const 
             const float2 hl = sh.red[(g * nw + w) * 8 + k];
             pair_add(h, l, hl.x, hl.y);
         }
-        c.part[((size_t)i * nch + ch0 + g) * 8 + k] = (double)h + (double)l;
+        c.part[((size_t)(ch0 + g) * 8 + k) * c.L + i] = (double)h + (double)l;
     }
 }
 

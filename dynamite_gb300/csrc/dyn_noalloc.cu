@@ -49,14 +49,15 @@ constexpr int MAX_G = (MAX_LEN + EPI_ROWS - 1) / EPI_ROWS;
 
 // scratch layout, in doubles
 constexpr size_t OFF_PART = 0;
-constexpr size_t N_PART = (size_t)MAX_LEN * MAX_NCH * 8;
+constexpr size_t N_PART = (size_t)MAX_LEN * MAX_NCH * 6;
 constexpr size_t OFF_EPART = OFF_PART + N_PART;
 constexpr size_t N_EPART = (size_t)MAX_G * EP_N;
 constexpr size_t OFF_ROWVAL = OFF_EPART + N_EPART;        // double2[MAX_LEN]
 constexpr size_t OFF_H = OFF_ROWVAL + 2 * (size_t)MAX_LEN; // double2[MAX_LEN]
 constexpr size_t OFF_POS = OFF_H + 2 * (size_t)MAX_LEN;    // double[MAX_LEN]
 constexpr size_t OFF_INV = OFF_POS + MAX_LEN;              // double[MAX_ROWS]
-constexpr size_t OFF_SLOTS = OFF_INV + MAX_ROWS;           // Slots, rounded up
+constexpr size_t OFF_B1 = OFF_INV + MAX_ROWS;              // B1Row[MAX_LEN]
+constexpr size_t OFF_SLOTS = OFF_B1 + MAX_LEN * (sizeof(B1Row) / 8);  // Slots, rounded up
 constexpr size_t N_SLOTS = (sizeof(Slots) + 7) / 8 + 8;
 constexpr size_t OFF_STAGE = OFF_SLOTS + N_SLOTS;          // StageDev
 constexpr size_t N_STAGE = (sizeof(StageDev) + 7) / 8 + 8;
@@ -139,17 +140,7 @@ extern "C" dyn_status dyn_rhs_noalloc(const dyn_noalloc_rhs* a, void* stream) {
     c.tpb = TPB;
     c.kpt = L >= 512 ? 4 : (L >= 256 ? 2 : 1);
     c.nch = (L + c.tpb * c.kpt - 1) / (c.tpb * c.kpt);
-    DModel& M = c.M;
-    M.p = a->p;
-    M.p2 = a->p2;
-    M.cA = a->lambda * a->p;
-    M.cB = (1 - a->lambda) * a->p2;
-    M.cC = a->lambda * a->p * (a->p - 1);
-    M.cD = (1 - a->lambda) * a->p2 * (a->p2 - 1);
-    M.cE = a->lambda * a->p * (a->p - 1) * (a->p - 2);
-    M.cF = (1 - a->lambda) * a->p2 * (a->p2 - 1) * (a->p2 - 2);
-    M.T0 = a->T0;
-    M.Gamma = a->Gamma;
+    c.M = make_model(a->p, a->p2, a->lambda, a->T0, a->Gamma);
     c.theta = a->theta;
     c.phi2 = a->phi2;
     c.integ = a->integ;
@@ -171,6 +162,7 @@ extern "C" dyn_status dyn_rhs_noalloc(const dyn_noalloc_rhs* a, void* stream) {
     c.h = reinterpret_cast<double2*>(base + OFF_H);
     c.posB1x = base + OFF_POS;
     c.inv_dtr = base + OFF_INV;
+    c.b1 = reinterpret_cast<B1Row*>(base + OFF_B1);
     c.slots = reinterpret_cast<Slots*>(base + OFF_SLOTS);
     c.stages = reinterpret_cast<StageDev*>(base + OFF_STAGE);
     c.rhs_out = reinterpret_cast<double2*>(a->out);
