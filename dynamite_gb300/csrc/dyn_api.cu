@@ -119,8 +119,8 @@ struct Ctx {
                         d.rvec, d.drvec, d.posB1x, d.posB1x_next, d.posB1x_saved, d.posB2x, d.posB2x_saved, d.h, d.gS,
                         d.geS, d.gfS, d.part, d.rowval, d.epart, d.slots, d.stages, d.rhs_out, d.ip,
                         d.rint, scratch_dev, (void*)d.wA1f, (void*)d.wA2f, (void*)d.wB2f, d.KRf, d.dKRf,
-                        (void*)d.integ_f, d.inv_len_f, d.inv_dtr_f, d.KRl, (void*)d.wA1l, (void*)d.wA2l,
-                        (void*)d.wB2l, tail, d.inv_len, d.b1, d.b2key, d.b2s, d.b2f, d.b2q};
+                        (void*)d.integ_f, d.inv_len_f, d.inv_dtr_f, d.KRq, (void*)d.wA1q, (void*)d.wA2q,
+                        (void*)d.wB2q, tail, d.inv_len, d.b1, d.b2key, d.b2s, d.b2f, d.b2q};
         for (void* b : bufs) if (b) cudaFree(b);
         std::memset(&d, 0, sizeof d);
         scratch_dev = nullptr;
@@ -148,25 +148,11 @@ struct Ctx {
             return s;
         double* ilen64 = nullptr;
         if (!d.mixed && (s = dalloc(&ilen64, ncap))) return s;
-        float2 *KRf = nullptr, *dKRf = nullptr;
-        float *ilen = nullptr, *idtf = nullptr;
-        if (d.mixed && ((s = dalloc(&ilen, ncap)) || (s = dalloc(&idtf, ncap)))) return s;
-        // +16 elements: the 16-byte segment loads of the mixed kernel may touch
-        // one element past the end of the last row
-        if (d.mixed && ((s = dalloc(&KRf, ncap * L + 16)) || (s = dalloc(&dKRf, ncap * L + 16)))) return s;
-        float2* KRl = nullptr;
-        if (d.mixed == 2 && (s = dalloc(&KRl, ncap * L + 16))) return s;
-        // rows not written yet meet the zero taps of the gather segments: keep them finite
-        if (d.mixed) {
-            CK(cudaMemsetAsync(KRf, 0, (ncap * L + 16) * sizeof(float2), st));
-            CK(cudaMemsetAsync(dKRf, 0, (ncap * L + 16) * sizeof(float2), st));
-        }
-        if (KRl) CK(cudaMemsetAsync(KRl, 0, (ncap * L + 16) * sizeof(float2), st));
-        if (n && d.mixed) {
-            CK(cudaMemcpyAsync(KRf, d.KRf, n * L * sizeof(float2), cudaMemcpyDeviceToDevice, st));
-            CK(cudaMemcpyAsync(dKRf, d.dKRf, n * L * sizeof(float2), cudaMemcpyDeviceToDevice, st));
-        }
-        if (n && KRl) CK(cudaMemcpyAsync(KRl, d.KRl, n * L * sizeof(float2), cudaMemcpyDeviceToDevice, st));
+        float2 *KRf = nullptr, *dKRf = nullptr, *ilen = nullptr, *idtf = nullptr;
+        float4* KRq = nullptr;  // +2: seg10 (dyn_mixed.cuh) may touch two elements past the last row
+        if (d.mixed && ((s = dalloc(&ilen, ncap)) || (s = dalloc(&idtf, ncap)) || (s = dalloc(&dKRf, ncap * L + 2)) ||
+                        (d.mixed == 2 ? (s = dalloc(&KRq, ncap * L)) : (s = dalloc(&KRf, ncap * L + 2)))))
+            return s;
         if (n) {
             CK(cudaMemcpyAsync(KR, d.KR, n * L * sizeof(double2), cudaMemcpyDeviceToDevice, st));
             CK(cudaMemcpyAsync(dKR, d.dKR, n * L * sizeof(double2), cudaMemcpyDeviceToDevice, st));
@@ -184,17 +170,17 @@ struct Ctx {
         d.inv_len = ilen64;
         d.KR = KR; d.dKR = dKR; d.t1grid = t1g; d.dtr = dt; d.inv_dtr = idt; d.rvec = rv; d.drvec = drv;
         if (d.mixed) {
-            if (d.KRf) cudaFree(d.KRf);
-            if (d.dKRf) cudaFree(d.dKRf);
-            if (d.inv_len_f) cudaFree(d.inv_len_f);
-            if (d.inv_dtr_f) cudaFree(d.inv_dtr_f);
-            if (d.KRl) cudaFree(d.KRl);
+            for (void* b : {(void*)d.KRf, (void*)d.KRq, (void*)d.dKRf, (void*)d.inv_len_f, (void*)d.inv_dtr_f})
+                if (b) cudaFree(b);
             d.KRf = KRf;
+            d.KRq = KRq;
             d.dKRf = dKRf;
-            d.KRl = KRl;
             d.inv_len_f = ilen;
             d.inv_dtr_f = idtf;
-            if (n) CK(launch_time_f32(d.t1grid, d.dtr, (int)n, d.inv_len_f, d.inv_dtr_f, st));
+            if (n) {
+                CK(launch_mirror(d, 0, n * L, st));
+                CK(launch_time_f32(d.t1grid, d.dtr, (int)n, d.inv_len_f, d.inv_dtr_f, st));
+            }
         }
         cap = ncap;
         drop_graphs();
@@ -204,14 +190,18 @@ struct Ctx {
     // Planes for the B2 sums of one call.  Without the memory for them the stages form
     // every sum, as the first stage of a call does.
     void alloc_b2() {
-        if (d.mixed) return;
+        const bool df = d.mixed == 2;
         if (cudaMalloc((void**)&d.b2key, L2 * sizeof(int)) == cudaSuccess &&
-            cudaMalloc((void**)&d.b2s, 4 * L2 * sizeof(double2)) == cudaSuccess)
+            (d.mixed ? cudaMalloc((void**)&d.b2f, (df ? 2 : 4) * L2 * sizeof(float2))
+                     : cudaMalloc((void**)&d.b2s, 4 * L2 * sizeof(double2))) == cudaSuccess &&
+            (!df || cudaMalloc((void**)&d.b2q, 2 * L2 * sizeof(float4)) == cudaSuccess))
             return;
         cudaGetLastError();
-        if (d.b2key) cudaFree(d.b2key);
+        for (void* b : {(void*)d.b2key, (void*)d.b2s, (void*)d.b2f, (void*)d.b2q}) if (b) cudaFree(b);
         d.b2key = nullptr;
         d.b2s = nullptr;
+        d.b2f = nullptr;
+        d.b2q = nullptr;
     }
 
     dyn_status upload_times() {
@@ -233,22 +223,12 @@ struct Ctx {
     // FP32 mirror of rows [0, n) from the FP64 master (mixed form)
     dyn_status mirror_all() {
         if (!d.mixed || n == 0) return DYN_OK;
-        CK(launch_mirror_rows(d.KR, d.KRf, n * L, st));
-        CK(launch_mirror_rows(d.dKR, d.dKRf, n * L, st));
-        if (d.KRl) CK(launch_mirror_lo(d.KR, d.KRl, n * L, st));
+        CK(launch_mirror(d, 0, n * L, st));
         return DYN_OK;
     }
 
     dyn_status pos_init() {
         CK(launch_pos_init(d, (int)n, st));
-        return DYN_OK;
-    }
-
-    // After the history shrank or was replaced (old length n_old): the FP32 mirror
-    // rows [n, n_old + 1) leave the history and are zeroed (clear_mirror_rows)
-    dyn_status clear_tail(size_t n_old) {
-        if (!d.mixed) return DYN_OK;
-        CK(clear_mirror_rows(d, n, std::min(std::max(n_old, n) + 1, cap), st));
         return DYN_OK;
     }
 
@@ -742,8 +722,7 @@ static dyn_status tail_fit(Ctx* c, int rollback_loop) {
     DevCtx& d = c->d;
     const size_t row = (c->n - 1) * (size_t)c->L;
     cudaError_t e = launch_tail_fit(d, (int)c->n, rollback_loop, c->cfg.delta_max, c->tail, c->st);
-    if (e == cudaSuccess && d.mixed) e = launch_mirror_rows(d.KR + row, d.KRf + row, c->L, c->st);
-    if (e == cudaSuccess && d.KRl) e = launch_mirror_lo(d.KR + row, d.KRl + row, c->L, c->st);
+    if (e == cudaSuccess && d.mixed) e = launch_mirror(d, row, c->L, c->st);
     if (e != cudaSuccess) return fail(DYN_ERR_CUDA, cudaGetErrorString(e));
     c->gen++;  // the newest row may have changed
     c->fsal_ok = false;
@@ -847,42 +826,36 @@ dyn_status dyn_ctx_create(const dyn_config* cfg, const dyn_tables* tb, void** ou
     cudaMemset(d.slots, 0, sizeof(Slots));
     if (d.mixed) {
         const size_t planes = (m + 1) / 2;
-        float2 *f1, *f2, *f3;
-        if ((s = dalloc(&f1, planes * L2)) || (s = dalloc(&f2, planes * L2)) || (s = dalloc(&f3, planes * L2))) { delete c; return s; }
-        d.wA1f = f1; d.wA2f = f2; d.wB2f = f3;
-        float* itf;  // [2L]: int.dat as FP32 (hi, lo) planes
-        if ((s = dalloc(&itf, 2 * L))) { delete c; return s; }
+        const double* w64[3] = {w1, w2, w3};
+        for (int k = 0; k < 3; ++k) {
+            void* out;
+            if (d.mixed == 2) {
+                float4* q;
+                if ((s = dalloc(&q, planes * L2))) { delete c; return s; }
+                (k == 0 ? d.wA1q : k == 1 ? d.wA2q : d.wB2q) = q;
+                out = q;
+            } else {
+                float2* f;
+                if ((s = dalloc(&f, planes * L2))) { delete c; return s; }
+                (k == 0 ? d.wA1f : k == 1 ? d.wA2f : d.wB2f) = f;
+                out = f;
+            }
+            if (launch_weights_tapmajor(w64[k], out, d.mixed, L2, (int)m, c->st) != cudaSuccess) {
+                delete c;
+                return fail(DYN_ERR_CUDA, "FP32 weight copies failed");
+            }
+        }
+        float2* itf;
+        if ((s = dalloc(&itf, L))) { delete c; return s; }
         d.integ_f = itf;
-        d.integ_l = itf + L;
-        {
-            std::vector<float> hl(2 * L);
-            for (size_t k = 0; k < L; ++k) {
-                hl[k] = (float)tb->integ[k];
-                hl[L + k] = (float)(tb->integ[k] - (double)hl[k]);
-            }
-            if (cudaMemcpy(itf, hl.data(), 2 * L * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) {
-                delete c;
-                return fail(DYN_ERR_CUDA, "FP32 int.dat copy failed");
-            }
-        }
-        if (launch_weights_tapmajor(w1, f1, L2, (int)m, c->st) != cudaSuccess ||
-            launch_weights_tapmajor(w2, f2, L2, (int)m, c->st) != cudaSuccess ||
-            launch_weights_tapmajor(w3, f3, L2, (int)m, c->st) != cudaSuccess || cudaStreamSynchronize(c->st) != cudaSuccess) {
+        std::vector<float2> hl(L);
+        for (size_t k = 0; k < L; ++k) hl[k] = hi_lo(tb->integ[k]);
+        if (cudaMemcpy(itf, hl.data(), L * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess ||
+            cudaStreamSynchronize(c->st) != cudaSuccess) {
             delete c;
-            return fail(DYN_ERR_CUDA, "FP32 weight copies failed");
+            return fail(DYN_ERR_CUDA, "FP32 int.dat copy failed");
         }
-        if (d.mixed == 2) {
-            float2 *l1, *l2, *l3;
-            if ((s = dalloc(&l1, planes * L2)) || (s = dalloc(&l2, planes * L2)) || (s = dalloc(&l3, planes * L2))) { delete c; return s; }
-            d.wA1l = l1; d.wA2l = l2; d.wB2l = l3;
-            if (launch_weights_tapmajor_lo(w1, l1, L2, (int)m, c->st) != cudaSuccess ||
-                launch_weights_tapmajor_lo(w2, l2, L2, (int)m, c->st) != cudaSuccess ||
-                launch_weights_tapmajor_lo(w3, l3, L2, (int)m, c->st) != cudaSuccess ||
-                cudaStreamSynchronize(c->st) != cudaSuccess) {
-                delete c;
-                return fail(DYN_ERR_CUDA, "FP32 weight low parts failed");
-            }
-        }
+        model_quads(d.M, d.cq);
     }
     c->alloc_b2();
     if (cudaMallocHost((void**)&c->stages_h, sizeof(StageDev) * SMAX) != cudaSuccess ||
@@ -917,7 +890,6 @@ dyn_status dyn_state_init(void* p, double delta_t) {
     if (!p) return fail(DYN_ERR_INVALID, "null ctx");
     Ctx* c = C(p);
     const int L = c->L;
-    const size_t n_old = c->n;
     c->n = 1;
     c->gen++;
     c->t1.assign(1, 0.0);
@@ -931,7 +903,6 @@ dyn_status dyn_state_init(void* p, double delta_t) {
     if (s) return s;
     CK(launch_rstep_exact(c->d, 1, c->d.drvec, c->st));
     if ((s = c->mirror_all())) return s;
-    if ((s = c->clear_tail(n_old))) return s;
     c->ctl.delta_t = delta_t > 0 ? delta_t : c->cfg.delta_t_min;
     c->ctl.loop = 0;
     c->last_rollback_loop = -1000;
@@ -963,7 +934,6 @@ dyn_status dyn_state_upload(void* p, const dyn_state* stt) {
             return fail(DYN_ERR_INVALID, "QK, QR, dQK and dQR must be finite");
     c->drop_graphs();
     c->gen++;
-    const size_t n_old = c->n;
     c->n = 0;
     dyn_status s = c->ensure_rows(n + 1);
     if (s) return s;
@@ -980,7 +950,6 @@ dyn_status dyn_state_upload(void* p, const dyn_state* stt) {
     c->t1.assign(stt->t1grid, stt->t1grid + n);
     c->dtr.assign(stt->delta_t_ratio, stt->delta_t_ratio + n);
     if ((s = c->mirror_all())) return s;
-    if ((s = c->clear_tail(n_old))) return s;
     if ((s = c->upload_times())) return s;
     if ((s = c->pos_init())) return s;
     CK(cudaStreamSynchronize(c->st));
@@ -1127,7 +1096,6 @@ dyn_status dyn_state_upload_dev(void* p, const dyn_state_dev* stt) {
     }
     c->drop_graphs();
     c->gen++;
-    const size_t n_old = c->n;
     c->n = 0;
     dyn_status s = c->ensure_rows(n + 1);
     if (s) return s;
@@ -1139,7 +1107,6 @@ dyn_status dyn_state_upload_dev(void* p, const dyn_state_dev* stt) {
     c->t1 = std::move(t1);
     c->dtr = std::move(dtr);
     if ((s = c->mirror_all())) return s;
-    if ((s = c->clear_tail(n_old))) return s;
     if ((s = c->upload_times())) return s;
     if ((s = c->pos_init())) return s;
     CK(cudaStreamSynchronize(c->st));
@@ -1157,11 +1124,7 @@ dyn_status dyn_state_rows_load_dev(void* p, size_t row0, size_t nrows, const dyn
     CK(cudaMemcpyAsync(c->d.rvec + row0, src->rvec + row0, nrows * sizeof(double), cudaMemcpyDeviceToDevice, c->st));
     CK(cudaMemcpyAsync(c->d.drvec + row0, src->drvec + row0, nrows * sizeof(double), cudaMemcpyDeviceToDevice,
                        c->st));
-    if (c->d.mixed) {
-        CK(launch_mirror_rows(c->d.KR + o, c->d.KRf + o, cnt, c->st));
-        CK(launch_mirror_rows(c->d.dKR + o, c->d.dKRf + o, cnt, c->st));
-        if (c->d.KRl) CK(launch_mirror_lo(c->d.KR + o, c->d.KRl + o, cnt, c->st));
-    }
+    if (c->d.mixed) CK(launch_mirror(c->d, o, cnt, c->st));
     c->gen++;
     CK(cudaStreamSynchronize(c->st));
     return DYN_OK;
@@ -1408,11 +1371,10 @@ dyn_status dyn_rollback(void* p, int nrows) {
     if (!p) return fail(DYN_ERR_INVALID, "null ctx");
     Ctx* c = C(p);
     if (nrows < 0 || (size_t)nrows >= c->n - 1) return fail(DYN_ERR_INVALID, "cannot roll back that many rows");
-    const size_t target = c->n - nrows, n_old = c->n;
+    const size_t target = c->n - nrows;
     c->n = target;
     c->gen++;
     c->new_call();
-    if (dyn_status cs = c->clear_tail(n_old)) return cs;
     c->t1.resize(target);
     c->dtr.resize(target);
     c->ctl.delta_t = c->t1[target - 1] - c->t1[target - 2];
@@ -1671,12 +1633,10 @@ dyn_status dyn_sparsify(void* p, double threshold, int variant, size_t* n_out) {
     c->drop_graphs();
     c->t1 = t1n;
     c->dtr = dtrn;
-    const size_t n_old = c->n;
     c->n = k;
     c->gen++;
     c->new_call();
     if ((s = c->mirror_all())) return s;
-    if ((s = c->clear_tail(n_old))) return s;
     if ((s = c->upload_times())) return s;
     if ((s = c->pos_init())) return s;
     CK(cudaStreamSynchronize(c->st));

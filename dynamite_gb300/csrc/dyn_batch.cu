@@ -56,6 +56,9 @@ struct Plan {
     double dtr_last;        // delta_t_ratio of the newest row (the controller's ratio == 1 test)
     int spars_loop;         // loop of the last periodic sparsify (-1: none)
     int last_rb;            // loop of the last rollback (simulation_runner.cpp:53: -1000)
+    unsigned call;          // Work::call of the last live stage, 0 after the history was cut back:
+                            // the B2 sums held are of that call
+    int fsal_ok;            // the last step was RK54: its last right-hand side is a next RK54 step's first
 };
 
 struct Quench {
@@ -67,11 +70,17 @@ struct Quench {
     long long spars_every;  // periodic sparsify every this many loops (0: never)
 };
 
-constexpr int SIDE_ITEM = 0x8000;  // gather items at or above this row: the rows' own work, a CTA's threads each
-
 struct Work {
     unsigned next, done;
+    unsigned pad[30];
+    unsigned call;  // number of the running dyn_batch_run / dyn_batch_enqueue call (off the counters' cache line)
 };
+// Whether quench stage sp goes on from a stage of the same call (B2Mode), and whether it needs
+// no gather at all: then its right-hand side is the previous step's last one
+__device__ __forceinline__ bool in_call(const Plan& pl, unsigned call) { return pl.call == call; }
+__device__ __forceinline__ bool is_fsal(const Plan& pl, const StageDev& sp, unsigned call) {
+    return sp.s == 0 && sp.fsal && in_call(pl, call);
+}
 
 // ------------------------------------------------------------------ planner
 // Stage descriptors of the next step (Ctx::build_step in dyn_api.cu, itself
@@ -168,6 +177,7 @@ __device__ void begin_step(const Quench& q, Plan& pl, const TabDev& tb) {
         sp.maxceil = sp.nrows - 1 < 1 ? 1 : sp.nrows - 1;
         sp.maxX = sp.nrows - 1;
         sp.fresh = s == 0 ? pl.fresh : 0;
+        sp.fsal = s == 0 && method == DYN_RK54 ? pl.fsal_ok : 0;
         sp.nrows_next = n0 + 1;
         sp.T = s == 0 ? T0 : Tn[s - 1];
         sp.T_next = Tn[s];
@@ -175,6 +185,7 @@ __device__ void begin_step(const Quench& q, Plan& pl, const TabDev& tb) {
         sp.dtr_new = n0 >= 2 ? __ddiv_rn(sp.tdiff, prev) : 0.0;
     }
     pl.fresh = 0;
+    pl.fsal_ok = 0;
     pl.S = S;
     pl.s = 0;
     pl.sidx = nb;
@@ -194,6 +205,7 @@ __device__ void finish_step(const Quench& q, Plan& pl, const StageDev& last) {
     pl.T_prev = pl.T_last;
     pl.T_last = last.T_next;
     pl.dtr_last = last.dtr_new;
+    pl.fsal_ok = pl.method == DYN_RK54 && last.T == last.T_next;
     pl.energy = sl->res_energy;
     pl.r = sl->res_r;
     pl.qk0 = sl->res_qk0;
@@ -232,6 +244,8 @@ __device__ void adapt_step(const Quench& q, Plan& pl, const TabDev& tb) {
             pl.loop -= nr;
             pl.last_rb = pl.loop;
             pl.fresh = 1;
+            pl.call = 0;
+            pl.fsal_ok = 0;
         }
         dt = __dmul_rn(0.5, fmin(fmax(dt, dmin), __ddiv_rn(tb.rmax[method - 1], sr)));
         method = method > 3 ? 2 + (2 * (method - 3)) / 2 : DYN_SSPRK104;
@@ -244,68 +258,89 @@ __device__ void adapt_step(const Quench& q, Plan& pl, const TabDev& tb) {
 // TPB threads per CTA; the register cap keeps DYN_BATCH_TPSM (K = 1) or 512
 // (K = 2) threads resident per SM: the gathers are latency-bound.
 #ifndef DYN_BATCH_TPSM
-#define DYN_BATCH_TPSM 1280
+#define DYN_BATCH_TPSM 1152
 #endif
 #ifndef DYN_BATCH_SHIFT
 #define DYN_BATCH_SHIFT 0
 #endif
 #ifndef DYN_BATCH_DF_TPSM
-#define DYN_BATCH_DF_TPSM 1024
+#define DYN_BATCH_DF_TPSM 1152
 #endif
-// DF: the (hi, lo) form (mdf::chunk_dd): twice the staged row and a double-float
-// tail; a cap of 64 registers (DYN_BATCH_DF_TPSM = 1024 threads per SM) spills a
-// little but measures best for 64 quenches at L=512: 1.55 ms against 1.62 (56
-// registers), 1.61 (72) and 1.74 (80).
-__device__ __noinline__ void batch_side(const DevCtx& c, const StageDev& sp, const int blk) {
-    mixed::side_rows<true>(c, sp, blk);
+// 56 registers (1152 threads) measure best in both forms.  64 quenches, L = 512, 800 rows:
+// plain 0.71 ms (48 registers 0.81, spilling; 64: 0.70, but slower on short rows, L = 256
+// 63 us against 61), (hi, lo) with its sums kept 1.06 ms (64: 1.09, 72: 1.11).
+//
+// DF: the (hi, lo) form (mdf::chunk_dd).  Bound by issue slots and the latency of its loads:
+// ~1,300 instructions per 32 targets, of which the compensated A1/A2 sums are ~40 %.
+// One (quench, row) of a gather launch
+struct GatherItem {
+    const StageDev* sp;
+    int quench, row;  // row < 0: no item left
+    bool run, keep;
+};
+template <bool KEEP>
+__device__ __forceinline__ void fetch_item(const Quench* Q, const Plan* PL, const unsigned* items, unsigned nitems, Work* work,
+                                           int force, GatherItem& out) {
+    const unsigned k = atomicAdd(&work->next, 1u);
+    out.row = -1;
+    if (k >= nitems) return;
+    const unsigned e = __ldg(items + k);
+    const Plan& pl = PL[e >> 16];
+    const StageDev* sp = Q[e >> 16].stg + pl.sidx * SMAX + pl.s;
+    const unsigned call = work->call;
+    out.sp = sp;
+    out.quench = (int)(e >> 16);
+    out.row = (int)(e & 0xffffu);
+    out.run = pl.status == DYN_QUENCH_RUNNING && (force || !is_fsal(pl, *sp, call));
+    out.keep = KEEP && (force ? force == 2 : in_call(pl, call));
 }
-template <int M, int K, int P, int P2, int TPB, bool DF = false>
+// KEEP: the B2 sums are kept in planes over the stages of a call.  force 0: each quench's
+// plan says whether its planes go on from the previous stage; 1, 2: measurement, all fill /
+// all keep.
+template <int M, int K, int P, int P2, int TPB, bool DF, bool KEEP>
 __global__ void __launch_bounds__(TPB, DF ? DYN_BATCH_DF_TPSM / TPB : (K == 1 ? DYN_BATCH_TPSM : 512) / TPB)
     k_batch_gather(const Quench* __restrict__ Q, const Plan* __restrict__ PL, const unsigned* __restrict__ items,
-                   const unsigned nitems, Work* work) {
+                   const unsigned nitems, Work* work, const int force) {
     wait_prior_grid();
-    extern __shared__ float2 s_lastf[];
+    extern __shared__ float4 s_row[];  // the quench's newest row: float4 [L] (DF), float2 [L + 2]
+    float2* s_lastf = reinterpret_cast<float2*>(s_row);
     __shared__ mixed::RowShared sh;
-    __shared__ float s_clo[4];
-    __shared__ unsigned s_item[2];  // the item being worked on and the next one
+    __shared__ mdf::RowConst rc;
+    __shared__ mixed::B2Jobs<KEEP ? TPB * K : 0> jb;
+    __shared__ GatherItem s_item[2];  // the item being worked on and the next one
     constexpr int GMAX = mixed::RED_CAP / (8 * (TPB / 32));  // chunks per fold
-    int p = 0;
-    if (threadIdx.x == 0) s_item[0] = atomicAdd(&work->next, 1u);
+    int p = 0, par = 0;
+    if (threadIdx.x == 0) {
+        fetch_item<KEEP>(Q, PL, items, nitems, work, force, s_item[0]);
+        jb.n[0][0] = jb.n[0][1] = 0;
+    }
     __syncthreads();
-    for (;;) {
-        const unsigned it = s_item[p];
-        if (it >= nitems) break;
-        const unsigned e = __ldg(items + it);
-        const Quench& q = Q[e >> 16];
-        const Plan& pl = PL[e >> 16];
-        if (pl.status == DYN_QUENCH_RUNNING) {
-            const int i = (int)(e & 0xffffu);
-            const StageDev& sp = q.stg[pl.sidx * SMAX + pl.s];
-            float2* s_lo = s_lastf + (q.c.L + 2);
-            int nch = q.c.nch;
-            if (i >= SIDE_ITEM) {
-                batch_side(q.c, sp, i - SIDE_ITEM);
-                nch = 0;
-            } else if constexpr (DF) {
-                mixed::row_setup<true>(q.c, sp, i, s_lastf, sh, s_clo);
-                mdf::stage_lo(q.c, sp, s_lo);
-            } else {
-                mixed::row_setup<true>(q.c, sp, i, s_lastf, sh);
-            }
-            __syncthreads();
+    while (s_item[p].row >= 0) {
+        const GatherItem& it = s_item[p];
+        const DevCtx& c = Q[it.quench].c;
+        const StageDev& sp = *it.sp;
+        const int i = it.row;
+        const bool keep = KEEP && it.keep;
+        if (it.run) {
+            if constexpr (DF) mdf::row_setup<true>(c, sp, i, s_row, sh, rc, !keep);
+            else mixed::row_setup<true>(c, sp, i, s_lastf, sh, !keep);
+        }
+        __syncthreads();
+        // the next item, by a thread of the last warp while the others work on this one
+        if (threadIdx.x == TPB - 32) fetch_item<KEEP>(Q, PL, items, nitems, work, force, s_item[p ^ 1]);
+        if (it.run) {
+            const int nch = c.nch;
             for (int ch0 = 0; ch0 < nch; ch0 += GMAX) {
                 const int ng = min(GMAX, nch - ch0);
-                for (int g = 0; g < ng; ++g) {
-                    if constexpr (DF) mdf::chunk_dd<M, K, P, P2>(q.c, sp, ch0 + g, g, s_lastf, s_lo, s_clo, sh, i);
-                    else mixed::chunk_sums<M, K, P, P2, DYN_BATCH_SHIFT>(q.c, sp, ch0 + g, g, s_lastf, sh, i);
+                for (int g = 0; g < ng; ++g, par ^= 1) {
+                    if constexpr (DF) mdf::chunk_dd<M, K, P, P2>(c, sp, ch0 + g, g, s_row, rc, sh, i, jb, par, keep);
+                    else mixed::chunk_sums<M, K, P, P2, DYN_BATCH_SHIFT != 0>(c, sp, ch0 + g, g, s_lastf, sh, i, jb, par, keep);
                 }
                 __syncthreads();
-                mixed::fold_chunks(q.c, i, nch, ch0, ng, sh);
+                mixed::fold_chunks<DF>(c, i, ch0, ng, sh);
                 if (ch0 + GMAX < nch) __syncthreads();
             }
         }
-        // the next item goes to the other slot: threads still reading s_item[p] are unaffected
-        if (threadIdx.x == 0) s_item[p ^ 1] = atomicAdd(&work->next, 1u);
         __syncthreads();
         p ^= 1;
     }
@@ -318,9 +353,10 @@ __global__ void __launch_bounds__(TPB, DF ? DYN_BATCH_DF_TPSM / TPB : (K == 1 ? 
 
 template <int P, int P2>
 __global__ void __launch_bounds__(EPI_T) k_batch_epi(const Quench* __restrict__ Q, Plan* __restrict__ PL,
-                                                     const unsigned* __restrict__ eitems, const TabDev* __restrict__ tb) {
+                                                     const unsigned* __restrict__ eitems, const TabDev* __restrict__ tb,
+                                                     const Work* __restrict__ work) {
     wait_prior_grid();
-    const unsigned e = eitems[blockIdx.x];
+    const unsigned e = eitems[blockIdx.x], call = work->call;
     const Quench& q = Q[e >> 16];
     Plan& pl = PL[e >> 16];
     if (pl.status != DYN_QUENCH_RUNNING) return;
@@ -330,11 +366,13 @@ __global__ void __launch_bounds__(EPI_T) k_batch_epi(const Quench* __restrict__ 
     const DevCtx& c = q.c;
     const unsigned G = (unsigned)((c.L + EPI_ROWS - 1) / EPI_ROWS);
     double ep[EP_N];
-    epi::rows<P, P2, true>(c, sp, s, (int)blk, ep);
+    epi::rows<P, P2, true>(c, sp, s, (int)blk, is_fsal(pl, sp, call), ep);
     if (!epi::elect_last(c, ep, blk, G)) return;
     epi::fold<P, P2, true>(c, sp, s, G);
     if (threadIdx.x != 0) return;
     c.slots->counter = 0;
+    // a stage at t = 0 gathers nothing, so the one after it starts the sums
+    pl.call = sp.T > 0.0 ? call : 0;
     if (!sp.last) {
         pl.s = s + 1;
         return;
@@ -352,6 +390,11 @@ __global__ void __launch_bounds__(EPI_T) k_batch_epi(const Quench* __restrict__ 
     }
     adapt_step(q, pl, *tb);
     begin_step(q, pl, *tb);
+}
+
+// A new call begins: what the previous one kept is not taken over
+__global__ void k_batch_call(Work* work) {
+    if (threadIdx.x == 0 && ++work->call == 0) work->call = 1;
 }
 
 // (Re)start quench b's planning from its plan (after creation, upload or new limits)
@@ -385,10 +428,10 @@ struct GridDev {
     double* theta = nullptr;
     double* phi2 = nullptr;
     double* integ = nullptr;
-    float* integ_f = nullptr;
+    float2* integ_f = nullptr;
     int* iA[3] = {nullptr, nullptr, nullptr};
-    float2* wf[3] = {nullptr, nullptr, nullptr};  // tap-major FP32 pair planes
-    float2* wl[3] = {nullptr, nullptr, nullptr};  // their low parts (DYN_MIXED_DF)
+    float2* wf[3] = {nullptr, nullptr, nullptr};  // tap-major FP32 pair planes (DYN_MIXED)
+    float4* wq[3] = {nullptr, nullptr, nullptr};  // the same with low parts (DYN_MIXED_DF)
 };
 
 struct Batch {
@@ -414,6 +457,7 @@ struct Batch {
     int tpb = 128, kpt = 1, ctas = 0;
     int M = 10, pp = 0;  // template selectors: stencil depth, (p, p2) kind
     bool df = false;     // DYN_MIXED_DF: (hi, lo) inputs (mdf::chunk)
+    bool keep = false;   // every quench has planes for its B2 sums
     size_t smem = 0, Lmax = 0;
     cudaGraphExec_t graph = nullptr;
     int graph_ticks = 0;
@@ -437,50 +481,50 @@ struct Batch {
         return DYN_OK;
     }
 
-    template <int M_, int K_, int P_, int P2_, int TPB_>
-    cudaError_t gather_t() {
-        if (df)  // the (hi, lo) form runs one target per thread
-            return launch_pdl(k_batch_gather<M_, 1, P_, P2_, TPB_, true>, dim3(nsm * ctas), dim3(TPB_), smem, st,
-                              (const Quench*)qd, (const Plan*)pd, (const unsigned*)items, nitems, work);
-        return launch_pdl(k_batch_gather<M_, K_, P_, P2_, TPB_>, dim3(nsm * ctas), dim3(TPB_), smem, st,
-                          (const Quench*)qd, (const Plan*)pd, (const unsigned*)items, nitems, work);
+    // Calls f with the gather kernel of a tile shape.  The (hi, lo) form runs one target per
+    // thread.  It keeps its B2 sums, whose compensated products are most of its work; in the
+    // plain form they cost less than the planes' traffic (64 quenches at L = 512: 0.75 ms a
+    // gather with planes, 0.69 without).
+    template <int M_, int P_, int P2_, typename F>
+    auto with_kernel_m(int threads, int targets, F f) {
+        const bool wide = threads == 256;
+        if (df && keep) return wide ? f(k_batch_gather<M_, 1, P_, P2_, 256, true, true>) : f(k_batch_gather<M_, 1, P_, P2_, 128, true, true>);
+        if (df) return wide ? f(k_batch_gather<M_, 1, P_, P2_, 256, true, false>) : f(k_batch_gather<M_, 1, P_, P2_, 128, true, false>);
+        if (targets == 2) return wide ? f(k_batch_gather<M_, 2, P_, P2_, 256, false, false>) : f(k_batch_gather<M_, 2, P_, P2_, 128, false, false>);
+        return wide ? f(k_batch_gather<M_, 1, P_, P2_, 256, false, false>) : f(k_batch_gather<M_, 1, P_, P2_, 128, false, false>);
     }
-    template <int M_, int K_, int P_, int P2_>
-    cudaError_t gather_b() { return tpb == 256 ? gather_t<M_, K_, P_, P2_, 256>() : gather_t<M_, K_, P_, P2_, 128>(); }
-    template <int M_, int P_, int P2_>
-    cudaError_t gather_k() { return kpt == 2 ? gather_b<M_, 2, P_, P2_>() : gather_b<M_, 1, P_, P2_>(); }
-    template <int P_, int P2_>
-    cudaError_t gather_m() { return M == 10 ? gather_k<10, P_, P2_>() : gather_k<0, P_, P2_>(); }
-    cudaError_t launch_gather() {
-        if (pp == 1) return gather_m<3, 4>();
-        if (pp == 2) return gather_m<3, 0>();
-        return gather_m<-1, -1>();
+    template <int P_, int P2_, typename F>
+    auto with_kernel_p(int threads, int targets, F f) {
+        return M == 10 ? with_kernel_m<10, P_, P2_>(threads, targets, f) : with_kernel_m<0, P_, P2_>(threads, targets, f);
+    }
+    template <typename F>
+    auto with_kernel(int threads, int targets, F f) {
+        if (pp == 1) return with_kernel_p<3, 4>(threads, targets, f);
+        if (pp == 2) return with_kernel_p<3, 0>(threads, targets, f);
+        return with_kernel_p<-1, -1>(threads, targets, f);
+    }
+    cudaError_t launch_gather(int force = 0) {
+        return with_kernel(tpb, kpt, [&](auto* kern) {
+            return launch_pdl(kern, dim3(nsm * ctas), dim3(tpb), smem, st, (const Quench*)qd, (const Plan*)pd,
+                              (const unsigned*)items, nitems, work, force);
+        });
     }
     cudaError_t launch_epi() {
         const Quench* q = qd;
         const unsigned* ei = eitems;
         const TabDev* tb = tabd;
-        if (pp == 1) return launch_pdl(k_batch_epi<3, 4>, dim3(neitems), dim3(EPI_T), 0, st, q, pd, ei, tb);
-        if (pp == 2) return launch_pdl(k_batch_epi<3, 0>, dim3(neitems), dim3(EPI_T), 0, st, q, pd, ei, tb);
-        return launch_pdl(k_batch_epi<-1, -1>, dim3(neitems), dim3(EPI_T), 0, st, q, pd, ei, tb);
+        const Work* w = work;
+        if (pp == 1) return launch_pdl(k_batch_epi<3, 4>, dim3(neitems), dim3(EPI_T), 0, st, q, pd, ei, tb, w);
+        if (pp == 2) return launch_pdl(k_batch_epi<3, 0>, dim3(neitems), dim3(EPI_T), 0, st, q, pd, ei, tb, w);
+        return launch_pdl(k_batch_epi<-1, -1>, dim3(neitems), dim3(EPI_T), 0, st, q, pd, ei, tb, w);
     }
 
     int occupancy(int threads, int targets) {
         int nb = 0;
-        const void* f;
-#define OCC_T(M_, K_, P_, P2_)                                                                        \
-    (df ? (threads == 256 ? (const void*)k_batch_gather<M_, 1, P_, P2_, 256, true>                        \
-                          : (const void*)k_batch_gather<M_, 1, P_, P2_, 128, true>)                       \
-        : (threads == 256 ? (const void*)k_batch_gather<M_, K_, P_, P2_, 256> : (const void*)k_batch_gather<M_, K_, P_, P2_, 128>))
-#define OCC_SEL(P_, P2_) \
-    f = M == 10 ? (targets == 2 ? OCC_T(10, 2, P_, P2_) : OCC_T(10, 1, P_, P2_)) \
-                : (targets == 2 ? OCC_T(0, 2, P_, P2_) : OCC_T(0, 1, P_, P2_))
-        if (pp == 1) { OCC_SEL(3, 4); } else if (pp == 2) { OCC_SEL(3, 0); } else { OCC_SEL(-1, -1); }
-#undef OCC_SEL
-#undef OCC_T
-        // the (hi, lo) form stages 2 (Lmax + 2) float2: above 48 KB from Lmax = 3071 on; the
-        // attribute is set here, before the tile's first launch and any graph capture
-        if (smem > 48 * 1024 &&
+        const void* f = with_kernel(threads, targets, [](auto* kern) { return (const void*)kern; });
+        // the (hi, lo) form stages Lmax float4: with its static part above 48 KB from Lmax = 2700
+        // on; the attribute is set here, before the tile's first launch and any graph capture
+        if (smem > 40 * 1024 &&
             cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
             return 1;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f, threads, smem) != cudaSuccess) return 1;
@@ -604,11 +648,8 @@ struct Batch {
             cudaMemcpyAsync(q.c.t1grid, t1n.data(), k * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess &&
             cudaMemcpyAsync(q.c.dtr, dtrn.data(), k * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess &&
             cudaMemcpyAsync(q.c.inv_dtr, inv.data(), k * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess &&
-            launch_mirror_rows(q.c.KR, q.c.KRf, k * L, st) == cudaSuccess &&
-            launch_mirror_rows(q.c.dKR, q.c.dKRf, k * L, st) == cudaSuccess &&
-            (!q.c.KRl || launch_mirror_lo(q.c.KR, q.c.KRl, k * L, st) == cudaSuccess) &&
-            launch_time_f32(q.c.t1grid, q.c.dtr, (int)k, q.c.inv_len_f, q.c.inv_dtr_f, st) == cudaSuccess &&
-            clear_mirror_rows(q.c, k, std::min((size_t)pl.n + 1, (size_t)q.cap), st) == cudaSuccess;
+            launch_mirror(q.c, 0, k * L, st) == cudaSuccess &&
+            launch_time_f32(q.c.t1grid, q.c.dtr, (int)k, q.c.inv_len_f, q.c.inv_dtr_f, st) == cudaSuccess;
         e = cudaStreamSynchronize(st);  // the host vectors above are sources of the copies
         release();
         if (!ok || e != cudaSuccess) return bfail(DYN_ERR_CUDA, "batch sparsify: " + std::string(cudaGetErrorString(cudaGetLastError())));
@@ -648,12 +689,39 @@ struct Batch {
             }
             pl.spars_loop = pl.loop;
             pl.status = DYN_QUENCH_RUNNING;
+            pl.call = 0;
+            pl.fsal_ok = 0;
             BCK(cudaMemcpyAsync(pd + b, &pl, sizeof(Plan), cudaMemcpyHostToDevice, st));
             k_batch_resume<<<1, 32, 0, st>>>(qd, pd, tabd, (int)b);
             BCK(cudaGetLastError());
             BCK(cudaStreamSynchronize(st));  // &pl is host memory the copy reads
         }
         return any ? read_plans() : DYN_OK;
+    }
+
+    dyn_status new_call() {
+        k_batch_call<<<1, 32, 0, st>>>(work);
+        BCK(cudaGetLastError());
+        return DYN_OK;
+    }
+
+    // Planes for the B2 sums of every quench, from at most a quarter of the memory left
+    // over by the histories; without them each stage forms every sum
+    bool alloc_b2() {
+        size_t need = 0, free_b = 0, total_b = 0;
+        for (const Quench& q : qh) need += (size_t)q.c.L * q.c.L * (sizeof(int) + 2 * sizeof(float4) + 2 * sizeof(float2));
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || need > free_b / 4) return false;
+        const size_t first = allocs.size();
+        for (Quench& q : qh) {
+            const size_t L2 = (size_t)q.c.L * q.c.L;
+            if (alloc(&q.c.b2key, L2) || alloc(&q.c.b2f, 2 * L2) || alloc(&q.c.b2q, 2 * L2)) {
+                cudaGetLastError();
+                for (; allocs.size() > first; allocs.pop_back()) cudaFree(allocs.back());
+                for (Quench& r : qh) r.c.b2key = nullptr, r.c.b2f = nullptr, r.c.b2q = nullptr;
+                return false;
+            }
+        }
+        return true;
     }
 
     dyn_status enqueue_ticks(int n) {
@@ -696,9 +764,7 @@ struct Batch {
         BCK(cudaMemcpyAsync(q.c.inv_dtr, &z, sizeof(double), cudaMemcpyHostToDevice, st));
         BCK(launch_time_f32(q.c.t1grid, q.c.dtr, 1, q.c.inv_len_f, q.c.inv_dtr_f, st));
         BCK(launch_rstep_exact(q.c, 1, q.c.drvec, st));
-        BCK(launch_mirror_rows(q.c.KR, q.c.KRf, L, st));
-        BCK(launch_mirror_rows(q.c.dKR, q.c.dKRf, L, st));
-        if (q.c.KRl) BCK(launch_mirror_lo(q.c.KR, q.c.KRl, L, st));
+        BCK(launch_mirror(q.c, 0, L, st));
         Plan p{};
         p.status = DYN_QUENCH_RUNNING;
         p.n = 1;
@@ -786,12 +852,9 @@ dyn_status dyn_batch_create(const dyn_batch_config* cfg, const dyn_batch_grid* g
         if (!check_tables(L, m, &grids[g].tables, i32, why)) { delete bt; return bfail(DYN_ERR_INVALID, why); }
         const dyn_tables& tb = grids[g].tables;
         if ((s = bt->alloc(&gd.theta, L)) || (s = bt->alloc(&gd.phi2, L2)) || (s = bt->alloc(&gd.integ, L)) ||
-            (s = bt->alloc(&gd.integ_f, 2 * L))) { delete bt; return s; }
-        std::vector<float> f(2 * L);  // int.dat as FP32 (hi, lo) planes
-        for (size_t k = 0; k < L; ++k) {
-            f[k] = (float)tb.integ[k];
-            f[L + k] = (float)(tb.integ[k] - (double)f[k]);
-        }
+            (s = bt->alloc(&gd.integ_f, L))) { delete bt; return s; }
+        std::vector<float2> f(L);
+        for (size_t k = 0; k < L; ++k) f[k] = hi_lo(tb.integ[k]);
 #define BUP(dst, src, bytes)                                                                       \
     if ((e = cudaMemcpy((void*)(dst), (src), (bytes), cudaMemcpyHostToDevice)) != cudaSuccess) {  \
         delete bt;                                                                                 \
@@ -800,28 +863,30 @@ dyn_status dyn_batch_create(const dyn_batch_config* cfg, const dyn_batch_grid* g
         BUP(gd.theta, tb.theta, L * sizeof(double));
         BUP(gd.phi2, tb.phi2, L2 * sizeof(double));
         BUP(gd.integ, tb.integ, L * sizeof(double));
-        BUP(gd.integ_f, f.data(), 2 * L * sizeof(float));
+        BUP(gd.integ_f, f.data(), L * sizeof(float2));
         const double* w[3] = {tb.weightsA1y, tb.weightsA2y, tb.weightsB2y};
         const size_t planes = (m + 1) / 2;
-        std::vector<float2> wt(planes * L2);
+        // the FP64 rows go through a device buffer and are laid out there (launch_weights_tapmajor)
+        double* w64 = nullptr;
+        if (cudaMalloc((void**)&w64, L2 * m * sizeof(double)) != cudaSuccess) {
+            delete bt;
+            return bfail(DYN_ERR_NOMEM, "cudaMalloc: weight staging");
+        }
         for (int k = 0; k < 3; ++k) {
-            if ((s = bt->alloc(&gd.iA[k], L2)) || (s = bt->alloc(&gd.wf[k], planes * L2))) { delete bt; return s; }
-            BUP(gd.iA[k], i32[k].data(), L2 * sizeof(int));
-            // the layout of k_weights_tapmajor (dyn_mixed.cu)
-            for (size_t tg = 0; tg < L2; ++tg)
-                for (size_t d = 0; d < m; d += 2)
-                    wt[(d >> 1) * L2 + tg] =
-                        make_float2((float)w[k][tg * m + d], d + 1 < m ? (float)w[k][tg * m + d + 1] : 0.0f);
-            BUP(gd.wf[k], wt.data(), planes * L2 * sizeof(float2));
-            if (bt->df) {
-                if ((s = bt->alloc(&gd.wl[k], planes * L2))) { delete bt; return s; }
-                auto lo = [](double v) { return (float)(v - (double)(float)v); };
-                for (size_t tg = 0; tg < L2; ++tg)
-                    for (size_t d = 0; d < m; d += 2)
-                        wt[(d >> 1) * L2 + tg] = make_float2(lo(w[k][tg * m + d]), d + 1 < m ? lo(w[k][tg * m + d + 1]) : 0.0f);
-                BUP(gd.wl[k], wt.data(), planes * L2 * sizeof(float2));
+            s = bt->alloc(&gd.iA[k], L2);
+            if (!s) s = bt->df ? bt->alloc(&gd.wq[k], planes * L2) : bt->alloc(&gd.wf[k], planes * L2);
+            if (!s && ((e = cudaMemcpy(gd.iA[k], i32[k].data(), L2 * sizeof(int), cudaMemcpyHostToDevice)) != cudaSuccess ||
+                       (e = cudaMemcpy(w64, w[k], L2 * m * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess ||
+                       (e = launch_weights_tapmajor(w64, bt->df ? (void*)gd.wq[k] : (void*)gd.wf[k], bt->df ? 2 : 1, L2, (int)m, bt->st)) != cudaSuccess ||
+                       (e = cudaStreamSynchronize(bt->st)) != cudaSuccess))
+                s = bfail(DYN_ERR_CUDA, cudaGetErrorString(e));
+            if (s) {
+                cudaFree(w64);
+                delete bt;
+                return s;
             }
         }
+        cudaFree(w64);
     }
     bt->M = all10 ? 10 : 0;
     // (p, p2) kind shared by all quenches selects the compiled exponents
@@ -831,7 +896,7 @@ dyn_status dyn_batch_create(const dyn_batch_config* cfg, const dyn_batch_grid* g
         pp = pp < 0 ? k : (pp == k ? pp : 0);
     }
     bt->pp = pp;
-    bt->smem = (bt->df ? 2 : 1) * (bt->Lmax + 2) * sizeof(float2);
+    bt->smem = bt->df ? bt->Lmax * sizeof(float4) : (bt->Lmax + 2) * sizeof(float2);
 
     // ---- tableaux
     {
@@ -873,37 +938,31 @@ dyn_status dyn_batch_create(const dyn_batch_config* cfg, const dyn_batch_grid* g
         d.phi2 = gd.phi2;
         d.integ = gd.integ;
         d.integ_f = gd.integ_f;
-        d.integ_l = gd.integ_f + gd.L;
+        model_quads(d.M, d.cq);
         d.iA1 = gd.iA[0];
         d.iA2 = gd.iA[1];
         d.iB2 = gd.iA[2];
         d.wA1f = gd.wf[0];
         d.wA2f = gd.wf[1];
         d.wB2f = gd.wf[2];
-        d.wA1l = gd.wl[0];
-        d.wA2l = gd.wl[1];
-        d.wB2l = gd.wl[2];
+        d.wA1q = gd.wq[0];
+        d.wA2q = gd.wq[1];
+        d.wB2q = gd.wq[2];
         const size_t G = (L + EPI_ROWS - 1) / EPI_ROWS, nchm = (L + nch_max_of - 1) / nch_max_of;
         if ((s = bt->alloc(&d.KR, cap * L)) || (s = bt->alloc(&d.dKR, cap * L)) ||
-            (s = bt->alloc(&d.KRf, cap * L + 16)) || (s = bt->alloc(&d.dKRf, cap * L + 16)) ||
+            (s = bt->df ? bt->alloc(&d.KRq, cap * L) : bt->alloc(&d.KRf, cap * L + 2)) ||  // +2: seg10 (dyn_mixed.cuh)
+            (s = bt->alloc(&d.dKRf, cap * L + 2)) ||
             (s = bt->alloc(&d.t1grid, cap)) || (s = bt->alloc(&d.dtr, cap)) || (s = bt->alloc(&d.inv_dtr, cap)) ||
             (s = bt->alloc(&d.rvec, cap)) || (s = bt->alloc(&d.drvec, cap)) || (s = bt->alloc(&d.inv_len_f, cap)) ||
-            (s = bt->alloc(&d.inv_dtr_f, cap)) || (s = bt->alloc(&d.posB1x, L)) || (s = bt->alloc(&d.posB1x_next, L)) || (s = bt->alloc(&d.b1, L)) ||
+            (s = bt->alloc(&d.inv_dtr_f, cap)) || (s = bt->alloc(&d.posB1x, L)) || (s = bt->alloc(&d.posB1x_next, L)) || (s = bt->alloc(&d.rowval, L)) || (s = bt->alloc(&d.b1, L)) ||
             (s = bt->alloc(&d.posB1x_saved, NSAVE * L)) || (s = bt->alloc(&d.h, (size_t)SMAX * L)) ||
             (s = bt->alloc(&d.gS, L)) || (s = bt->alloc(&d.geS, L)) || (s = bt->alloc(&d.gfS, L)) ||
-            (s = bt->alloc(&d.part, L * nchm * 8)) || (s = bt->alloc(&d.rowval, L)) ||
+            (s = bt->alloc(&d.part, L * nchm * 8)) ||
             (s = bt->alloc(&d.epart, G * EP_N)) || (s = bt->alloc(&d.slots, 1)) || (s = bt->alloc(&d.rhs_out, L)) ||
             (s = bt->alloc(&q.stg, 2 * SMAX))) {
             delete bt;
             return s;
         }
-        if (bt->df) {
-            if ((s = bt->alloc(&d.KRl, cap * L + 16))) { delete bt; return s; }
-            cudaMemset(d.KRl, 0, (cap * L + 16) * sizeof(float2));
-        }
-        // the 16-byte segment loads may touch one element past the last row
-        cudaMemset(d.KRf, 0, (cap * L + 16) * sizeof(float2));
-        cudaMemset(d.dKRf, 0, (cap * L + 16) * sizeof(float2));
         cudaMemset(d.slots, 0, sizeof(Slots));
         cudaMemset(q.stg, 0, 2 * SMAX * sizeof(StageDev));
         q.cap = (int)cap;
@@ -915,6 +974,7 @@ dyn_status dyn_batch_create(const dyn_batch_config* cfg, const dyn_batch_grid* g
         q.dmax = sq.delta_max;
         q.specRad = 4 * std::sqrt(DDf_host(sq.lambda, sq.p, sq.p2, 1));
     }
+    bt->keep = bt->df && bt->alloc_b2();
     if ((s = bt->alloc(&bt->qd, nquench)) || (s = bt->alloc(&bt->pd, nquench)) || (s = bt->alloc(&bt->work, 1))) {
         delete bt;
         return s;
@@ -930,13 +990,20 @@ dyn_status dyn_batch_create(const dyn_batch_config* cfg, const dyn_batch_grid* g
     {
         std::vector<int> order(nquench);
         for (int b = 0; b < nquench; ++b) order[b] = b;
-        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return bt->qh[a].c.L > bt->qh[b].c.L; });
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+            const int la = bt->qh[a].c.L, lb = bt->qh[b].c.L;
+            return la != lb ? la > lb : bt->spec[a].grid < bt->spec[b].grid;
+        });
         std::vector<unsigned> it, ei;
-        // enough for the smaller CTA; with more threads the later items find no row
-        for (int b : order)
-            for (int g = 0; g < (bt->qh[b].c.L + 127) / 128; ++g) it.push_back(((unsigned)b << 16) | (unsigned)(SIDE_ITEM + g));
-        for (int b : order)
-            for (int i = 0; i < bt->qh[b].c.L; ++i) it.push_back(((unsigned)b << 16) | (unsigned)i);
+        // Kept sums leave the stencil weights as most of what a gather reads: the same row of every
+        // quench on a grid in turn, so that they come from memory once and then from L2 (64
+        // quenches at L = 512: 1.70 -> 1.56 ms).  Otherwise the histories are: quench by quench.
+        for (size_t k0 = 0, k1; k0 < order.size(); k0 = k1) {
+            const int g = bt->spec[order[k0]].grid, L = bt->qh[order[k0]].c.L;
+            for (k1 = k0 + 1; bt->keep && k1 < order.size() && bt->spec[order[k1]].grid == g;) ++k1;
+            for (int i = L - 1; i >= 0; --i)
+                for (size_t k = k0; k < k1; ++k) it.push_back(((unsigned)order[k] << 16) | (unsigned)i);
+        }
         for (int b = 0; b < nquench; ++b)
             for (int g = 0; g < (bt->qh[b].c.L + EPI_ROWS - 1) / EPI_ROWS; ++g) ei.push_back(((unsigned)b << 16) | (unsigned)g);
         bt->nitems = (unsigned)it.size();
@@ -1003,10 +1070,7 @@ dyn_status dyn_batch_upload(void* p, int qi, const dyn_state* stt, const dyn_con
     BCK(cudaMemcpyAsync(q.c.t1grid, stt->t1grid, n * sizeof(double), cudaMemcpyHostToDevice, st));
     BCK(cudaMemcpyAsync(q.c.dtr, stt->delta_t_ratio, n * sizeof(double), cudaMemcpyHostToDevice, st));
     BCK(cudaMemcpyAsync(q.c.inv_dtr, inv.data(), n * sizeof(double), cudaMemcpyHostToDevice, st));
-    BCK(launch_mirror_rows(q.c.KR, q.c.KRf, n * L, st));
-    BCK(launch_mirror_rows(q.c.dKR, q.c.dKRf, n * L, st));
-    if (q.c.KRl) BCK(launch_mirror_lo(q.c.KR, q.c.KRl, n * L, st));
-    BCK(clear_mirror_rows(q.c, n, (size_t)q.cap, st));  // whatever the previous history left
+    BCK(launch_mirror(q.c, 0, n * L, st));
     BCK(launch_time_f32(q.c.t1grid, q.c.dtr, (int)n, q.c.inv_len_f, q.c.inv_dtr_f, st));
     Plan pl{};
     pl.status = DYN_QUENCH_RUNNING;
@@ -1102,8 +1166,8 @@ dyn_status dyn_batch_run(void* p, long long max_ticks, long long* ticks_out) {
     TraceRange tr("dyn_batch_run");
     Batch* bt = BT(p);
     long long done = 0;
-    dyn_status s = bt->read_plans();
-    if (s) return s;
+    dyn_status s = bt->new_call();
+    if (s || (s = bt->read_plans())) return s;
     while (done < max_ticks && bt->running() > 0) {
         if ((s = bt->ensure_graph())) return s;
         if (max_ticks - done >= bt->graph_ticks) {
@@ -1125,7 +1189,7 @@ dyn_status dyn_batch_enqueue(void* p, long long ticks) {
     TraceRange tr("dyn_batch_enqueue");
     Batch* bt = BT(p);
     dyn_status s = bt->ensure_graph();
-    if (s) return s;
+    if (s || (s = bt->new_call())) return s;
     long long done = 0;
     for (; done + bt->graph_ticks <= ticks; done += bt->graph_ticks) BCK(cudaGraphLaunch(bt->graph, bt->st));
     return bt->enqueue_ticks((int)(ticks - done));
@@ -1167,9 +1231,13 @@ dyn_status dyn_batch_profile(void* p, int reps, float* ms) {
     cudaEvent_t a, b;
     BCK(cudaEventCreate(&a));
     BCK(cudaEventCreate(&b));
-    BCK(bt->launch_gather());  // warm
+    // the pending stage of every quench: all sums once, then as a stage that goes on from
+    // there, the form all but a call's first stages have
+    dyn_status s = bt->new_call();
+    if (s) return s;
+    BCK(bt->launch_gather(1));
     BCK(cudaEventRecord(a, bt->st));
-    for (int k = 0; k < reps; ++k) BCK(bt->launch_gather());
+    for (int k = 0; k < reps; ++k) BCK(bt->launch_gather(2));
     BCK(cudaEventRecord(b, bt->st));
     BCK(cudaEventSynchronize(b));
     float t = 0;

@@ -113,30 +113,41 @@ __device__ __forceinline__ B1Row b1_row(const DevCtx& c, double pos, int maxceil
     return b1_at(pos, maxceil, nrows, [&](int k) { return c.inv_dtr[k]; });
 }
 
-// What a stage needs once per target row and no target does: QK^{B1}[i,0] and rInt_i for
-// the epilogue, and the next stage's B1 position (theta_i T_next in the list that the row
-// this stage writes will end).  Its chains of dependent loads run beside the gathers, in
-// CTAs of their own.
-__device__ __forceinline__ void side_row(const DevCtx& c, const StageDev& sp, const B1Row& r, int i) {
+// What a stage needs once per target row and no target does: QK^{B1}[i,0] and rInt_i, and
+// the next stage's B1 position (theta_i T_next in the list that the row this stage writes
+// will end), and C(t,0) from row 0.  Not in the epilogue, whose other CTAs already overwrite
+// the newest row: single contexts run these chains of dependent loads beside the gathers in
+// CTAs of their own (side_row), the batch in two threads of the row's CTA (its other CTAs
+// fill the gap; CTAs of their own made its gather 3 % slower).
+__device__ __forceinline__ double2 row_value(const DevCtx& c, const StageDev& sp, const B1Row& r) {
     const int L = c.L;
-    if (sp.T > 0.0) {
-        const double2 x0 = c.KR[(size_t)(r.F - 1) * L], x1 = c.KR[(size_t)r.F * L];
-        const double2 d1 = c.dKR[(size_t)r.F * L];
-        double qb = fma(-r.c2, d1.x, fma(r.c1, x1.x, __dmul_rn(r.c0, x0.x)));
-        double ri = fma(-r.c2, c.drvec[r.F], fma(r.c1, c.rvec[r.F], __dmul_rn(r.c0, c.rvec[r.F - 1])));
-        if (r.cubic) {
-            qb = fma(-r.c3, c.dKR[(size_t)(r.F + 1) * L].x, qb);
-            ri = fma(-r.c3, c.drvec[r.F + 1], ri);
-        }
-        c.rowval[i] = make_double2(qb, ri);
-    } else {
-        c.rowval[i] = make_double2(c.KR[0].x, c.rvec[0]);
+    if (!(sp.T > 0.0)) return make_double2(c.KR[0].x, c.rvec[0]);
+    const double2 x0 = c.KR[(size_t)(r.F - 1) * L], x1 = c.KR[(size_t)r.F * L];
+    const double2 d1 = c.dKR[(size_t)r.F * L];
+    double qb = fma(-r.c2, d1.x, fma(r.c1, x1.x, __dmul_rn(r.c0, x0.x)));
+    double ri = fma(-r.c2, c.drvec[r.F], fma(r.c1, c.rvec[r.F], __dmul_rn(r.c0, c.rvec[r.F - 1])));
+    if (r.cubic) {
+        qb = fma(-r.c3, c.dKR[(size_t)(r.F + 1) * L].x, qb);
+        ri = fma(-r.c3, c.drvec[r.F + 1], ri);
     }
-    if (i == 0) c.slots->q0 = c.KR[(size_t)(sp.nrows - 1) * L].x;
-    if (sp.kind != KIND_RHS && sp.pos_reuse < 0) {
-        const ListView lv{c.t1grid, sp.nrows_next, sp.T_next};
-        c.posB1x_next[i] = search_pos(c.search, lv, __dmul_rn(c.theta[i], sp.T_next));
-    }
+    return make_double2(qb, ri);
+}
+__device__ __forceinline__ double next_position(const DevCtx& c, const StageDev& sp, int i) {
+    const ListView lv{c.t1grid, sp.nrows_next, sp.T_next};
+    return search_pos(c.search, lv, __dmul_rn(c.theta[i], sp.T_next));
+}
+__device__ __forceinline__ void side_value(const DevCtx& c, const StageDev& sp, const B1Row& r, int i) {
+    c.rowval[i] = row_value(c, sp, r);
+    if (i == 0) c.slots->q0 = c.KR[(size_t)(sp.nrows - 1) * c.L].x;
+}
+__device__ __forceinline__ void side_position(const DevCtx& c, const StageDev& sp, int i) {
+    if (sp.kind != KIND_RHS && sp.pos_reuse < 0) c.posB1x_next[i] = next_position(c, sp, i);
+}
+__device__ __forceinline__ void side_row(const DevCtx& c, const StageDev& sp, int i) {
+    B1Row r = {};
+    if (sp.T > 0.0) r = c.b1[i];
+    side_value(c, sp, r, i);
+    side_position(c, sp, i);
 }
 
 namespace epi {
@@ -144,9 +155,11 @@ namespace epi {
 // Rows blk*EPI_ROWS .. +EPI_ROWS of stage s (one row per lane of a one-warp
 // CTA).  Leaves in ep[] the warp sums of the scalars this stage needs:
 // [0..2] r(t) terms, [3..9] dr/dt terms (stage 0), [10] error norm,
-// [12] C(t,0), [13] f'(C(t,0)) (last stage).
+// [12] C(t,0), [13] f'(C(t,0)) (last stage).  fsal: stage 0 of an RK54 step whose right-hand
+// side is the previous step's last one (StageDev::fsal); no gather ran for it.
 template <int P, int P2, bool MIXED>
-__device__ __forceinline__ void rows(const DevCtx& c, const StageDev& sp, const int s, const int blk, double ep[EP_N]) {
+__device__ __forceinline__ void rows(const DevCtx& c, const StageDev& sp, const int s, const int blk,
+                                     const bool fsal, double ep[EP_N]) {
     const int L = c.L, tid = threadIdx.x, i = blk * EPI_ROWS + tid;
     const DModel Mo = c.M;
 #pragma unroll
@@ -154,16 +167,15 @@ __device__ __forceinline__ void rows(const DevCtx& c, const StageDev& sp, const 
 
     if (tid < EPI_ROWS && i < L) {
         double2 hs;
-        if (s == 0 && sp.fsal) {
+        if (fsal) {
             hs = c.h[(size_t)(RK54_STAGES - 1) * L + i];
         } else {
-            constexpr int NP = MIXED ? 8 : 6;
-            double a[NP];
+            double a[6];
 #pragma unroll
-            for (int k = 0; k < NP; ++k) a[k] = 0.0;
+            for (int k = 0; k < 6; ++k) a[k] = 0.0;
             for (int ch = 0; ch < c.nch; ++ch) {
 #pragma unroll
-                for (int k = 0; k < NP; ++k) a[k] += c.part[((size_t)ch * NP + k) * L + i];
+                for (int k = 0; k < 6; ++k) a[k] += c.part[((size_t)ch * 6 + k) * L + i];
             }
             const double t = sp.T, th = c.theta[i];
             const double tA = t * th, tR = t * (1.0 - th);
@@ -172,13 +184,12 @@ __device__ __forceinline__ void rows(const DevCtx& c, const StageDev& sp, const 
             const double rE = c.rowval[L - 1].y;
             const double q0 = c.slots->q0;
             const double fac1 = Sig<P, P2>::d1(Mo, q0) * Mo.iT0, fac2 = q0 * Mo.iT0;
-            double d1 = rv.x * fac1 + q.x * (-rE) + a[0] * tR + a[1] * tA;
-            if constexpr (MIXED) d1 += a[2] * tA;
-            constexpr int B = MIXED ? 3 : 2;  // a[B]: ConvR(QRA2, SigmaKB2) and on
-            double d2 = Sig<P, P2>::d1(Mo, rv.x) * fac2 + q.y * (2.0 * Mo.Gamma) + a[B] * tR + a[B + 1] * tA;
-            if constexpr (MIXED) d2 += a[5] * tA;
-            d2 -= q.x * rv.y;
-            hs = make_double2(d1 + d2 * th, (q.y * (-rE) + a[NP - 2] * tR) + (q.y * rv.y - a[NP - 1] * tR) * th);
+            // fused as written: every kernel that instantiates this rounds alike
+            const double d1 = fma(a[1], tA, fma(a[0], tR, fma(q.x, -rE, __dmul_rn(rv.x, fac1))));
+            const double d2 = fma(-q.x, rv.y, fma(a[3], tA, fma(a[2], tR,
+                              fma(q.y, 2.0 * Mo.Gamma, __dmul_rn(Sig<P, P2>::d1(Mo, rv.x), fac2)))));
+            hs = make_double2(fma(d2, th, d1), fma(fma(-a[5], tR, __dmul_rn(q.y, rv.y)), th,
+                                                   fma(a[4], tR, __dmul_rn(q.y, -rE))));
         }
         c.h[(size_t)s * L + i] = hs;
         if (sp.kind == KIND_RHS) {
@@ -234,45 +245,40 @@ __device__ __forceinline__ void rows(const DevCtx& c, const StageDev& sp, const 
                 Sig<P, P2>::d12(Mo, g0.x, sk, dd);
                 const double sr = dd * g0.y;
                 const double dsk = dd * h0.x;
-                const double dsr = (Sig<P, P2>::d3(Mo, g0.x) * g0.y) * h0.x + dd * h0.y;
+                const double dsr = fma(dd, h0.y, __dmul_rn(Sig<P, P2>::d3(Mo, g0.x) * g0.y, h0.x));
                 const double tw = sp.T * w;
-                ep[3] = (w * sr) * g0.x;
-                ep[4] = (w * sk) * g0.y;
-                ep[5] = (tw * dsr) * g0.x;
-                ep[6] = (tw * dsk) * g0.y;
-                ep[7] = (tw * sr) * h0.x;
-                ep[8] = (tw * sk) * h0.y;
-                if (i == 0) ep[9] = (dsk * g0.x + sk * h0.x) * Mo.iT0;
+                ep[3] = __dmul_rn(w * sr, g0.x);
+                ep[4] = __dmul_rn(w * sk, g0.y);
+                ep[5] = __dmul_rn(tw * dsr, g0.x);
+                ep[6] = __dmul_rn(tw * dsk, g0.y);
+                ep[7] = __dmul_rn(tw * sr, h0.x);
+                ep[8] = __dmul_rn(tw * sk, h0.y);
+                if (i == 0) ep[9] = __dmul_rn(fma(sk, h0.x, __dmul_rn(dsk, g0.x)), Mo.iT0);
             }
             const double td = sp.tdiff;
             c.KR[(size_t)sp.n0 * L + i] = g;
             c.dKR[(size_t)sp.n0 * L + i] = make_double2(td * h0.x, td * h0.y);
             if constexpr (MIXED) {
-                c.KRf[(size_t)sp.n0 * L + i] = make_float2((float)g.x, (float)g.y);
-                if (c.KRl)
-                    c.KRl[(size_t)sp.n0 * L + i] =
-                        make_float2((float)(g.x - (double)(float)g.x), (float)(g.y - (double)(float)g.y));
+                const float2 gx = hi_lo(g.x), gy = hi_lo(g.y);
+                if (c.KRq) c.KRq[(size_t)sp.n0 * L + i] = make_float4(gx.x, gy.x, gx.y, gy.y);
+                else c.KRf[(size_t)sp.n0 * L + i] = make_float2(gx.x, gy.x);
                 c.dKRf[(size_t)sp.n0 * L + i] = make_float2((float)(td * h0.x), (float)(td * h0.y));
             }
             // rstep (time_steps.cpp:83-92) of the new row at its time
             const double tn = sp.T_next, tw = tn * w;
             double sk, dd;
             Sig<P, P2>::d12(Mo, g.x, sk, dd);
-            ep[0] = (tw * (dd * g.y)) * g.x;
-            ep[1] = (tw * sk) * g.y;
+            ep[0] = __dmul_rn(tw * (dd * g.y), g.x);
+            ep[1] = __dmul_rn(tw * sk, g.y);
             if (i == 0) {
-                ep[2] = (sk * g.x) * Mo.iT0;
+                ep[2] = __dmul_rn(sk * g.x, Mo.iT0);
                 ep[12] = g.x;
                 ep[13] = sk;
             }
             // positions of the next stage (searched by the gather kernel)
-            double pos;
-            if (s == 0 && sp.fsal) {  // no gather ran: searched here, in the list the row about to be written ends
-                const ListView lv{c.t1grid, sp.nrows_next, sp.T_next};
-                pos = search_pos(c.search, lv, __dmul_rn(c.theta[i], sp.T_next));
-            } else {
-                pos = sp.pos_reuse >= 0 ? c.posB1x_saved[(size_t)sp.pos_reuse * L + i] : c.posB1x_next[i];
-            }
+            const double pos = sp.pos_reuse >= 0 ? c.posB1x_saved[(size_t)sp.pos_reuse * L + i]
+                               : fsal            ? next_position(c, sp, i)  // no gather ran
+                                                 : c.posB1x_next[i];
             c.posB1x[i] = pos;
             // the next stage's B1 row; delta_t_ratio of the row being written is not in memory yet
             c.b1[i] = b1_at(pos, sp.nrows_next - 1 < 1 ? 1 : sp.nrows_next - 1, sp.nrows_next, [&](int k) {
@@ -354,12 +360,12 @@ __device__ __forceinline__ void fold(const DevCtx& c, const StageDev& sp, const 
         c.inv_dtr[n0] = sp.dtr_new != 0.0 ? 1.0 / sp.dtr_new : 0.0;
         if (c.inv_len) c.inv_len[n0 - 1] = 1.0 / sp.tdiff;
         if constexpr (MIXED) {
-            c.inv_dtr_f[n0] = sp.dtr_new != 0.0 ? (float)(1.0 / sp.dtr_new) : 0.0f;
-            c.inv_len_f[n0 - 1] = (float)(1.0 / sp.tdiff);
+            c.inv_dtr_f[n0] = hi_lo(sp.dtr_new != 0.0 ? 1.0 / sp.dtr_new : 0.0);
+            c.inv_len_f[n0 - 1] = hi_lo(1.0 / sp.tdiff);
         }
         if (sp.last) {
             sl->res_err = s_tot[10];
-            sl->res_energy = -(s_tot[1] + s_tot[13] * Mo.iT0);
+            sl->res_energy = -(s_tot[1] + __dmul_rn(s_tot[13], Mo.iT0));
             sl->res_r = r_new;
             sl->res_qk0 = s_tot[12];
             sl->res_dr = sl->dr;

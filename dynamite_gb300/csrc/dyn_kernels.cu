@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(64) k_main(const DevCtx c, const int s) {
     const int L = c.L, tpb = blockDim.x, nside = (L + tpb - 1) / tpb;
     if (blockIdx.y < nside) {  // the rows' own work, tpb rows a CTA
         const int r = blockIdx.y * tpb + threadIdx.x;
-        if (blockIdx.x == 0 && r < L) side_row(c, sp, c.b1[r], r);
+        if (blockIdx.x == 0 && r < L) side_row(c, sp, r);
         return;
     }
     // rows near theta = 1 first: most of their targets read the row being written, the longest work
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(EPI_T) k_epi(const DevCtx c, const int s) {
     wait_prior_grid();
     const StageDev& sp = c.stages[s];
     double ep[EP_N];
-    epi::rows<P, P2, MIXED>(c, sp, s, blockIdx.x, ep);
+    epi::rows<P, P2, MIXED>(c, sp, s, blockIdx.x, s == 0 && sp.fsal, ep);
     if (!epi::elect_last(c, ep, blockIdx.x, gridDim.x)) return;
     epi::fold<P, P2, MIXED>(c, sp, s, gridDim.x);
     if (threadIdx.x == 0) c.slots->counter = 0;

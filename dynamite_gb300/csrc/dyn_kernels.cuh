@@ -112,27 +112,28 @@ struct DevCtx {
     double2* gS;           // SERK running stage value [L]
     double2* geS;          // SERK previous odd value [L]
     double2* gfS;          // SERK combination [L]
-    double* part;          // [nch][6 or 8][L] row sums: FP64 form 6 (the two ConvA pairs added), mixed forms 8
+    double* part;          // [nch][6][L] row sums (each of the two ConvA pairs added)
     double2* rowval;       // [L] (QK^{B1}[i,0], rInt_i)
     double* epart;         // [G][EP_N]
     Slots* slots;
     StageDev* stages;      // [SMAX]
     double2* rhs_out;      // [L]
-    // mixed form: FP32 copies of the weights, tap-major ([ceil(m/2)][L*L] tap
-    // pairs), and FP32 mirror of the history
+    // mixed forms: FP32 mirror of the history and copies of the weights, tap-major
+    // ([ceil(m/2)][L*L] tap pairs).  Plain (mixed 1): float2 (QK, QR) and tap pairs; (hi, lo)
+    // (mixed 2): float4 with the low parts v - (double)(float)v behind the high ones, one load each
     const float2* wA1f;
     const float2* wA2f;
     const float2* wB2f;
     float2* KRf;
-    float2* dKRf;
-    float2* KRl;           // mixed 2: low parts of (QK, QR), KR - (double)KRf
-    const float2* wA1l;    // mixed 2: low parts of the FP32 weights (same layout as wA1f)
-    const float2* wA2l;
-    const float2* wB2l;
-    const float* integ_f;  // [L]   int.dat in FP32
-    const float* integ_l;  // [L]   its low parts, int.dat - (double)integ_f (mixed forms)
-    float* inv_dtr_f;      // [cap] 1/delta_t_ratio in FP32
-    float* inv_len_f;      // [cap] 1/(t1grid[k+1]-t1grid[k]) in FP32
+    const float4* wA1q;
+    const float4* wA2q;
+    const float4* wB2q;
+    float4* KRq;
+    float2* dKRf;          // (dQK, dQR) in FP32 (both)
+    const float2* integ_f; // [L]   int.dat (hi, lo)
+    float2* inv_dtr_f;     // [cap] 1/delta_t_ratio (hi, lo)
+    float2* inv_len_f;     // [cap] 1/(t1grid[k+1]-t1grid[k]) (hi, lo)
+    float4 cq[4];          // the model's cA..cD as (h, h, l, l) (mixed 2)
     // materialized interpolation (dyn_interpolate)
     double* ip;            // [16][L*L]
     double* rint;          // [L]
@@ -281,18 +282,24 @@ cudaError_t launch_compact(const DevCtx& c, const int* inds, const int* indsD, c
 cudaError_t launch_pack_rows(const double* QK, const double* QR, double2* out, size_t count,
                              cudaStream_t st);
 cudaError_t launch_main_mixed(const DevCtx& c, int s, cudaStream_t st);
-cudaError_t launch_mirror_rows(const double2* in, float2* out, size_t count, cudaStream_t st);
-cudaError_t launch_mirror_lo(const double2* in, float2* out, size_t count, cudaStream_t st);
-// Rows past a history meet the zero taps of the mixed gathers' segment loads
-// (the element after a stencil window that ends a row is the next row's first),
-// so they must hold finite values: zero the FP32 mirror rows [r0, r1) that a
-// shortened or replaced history leaves behind (they may hold a failed step's NaN).
-cudaError_t clear_mirror_rows(const DevCtx& c, size_t r0, size_t r1, cudaStream_t st);
-cudaError_t launch_weights_tapmajor_lo(const double* in, float2* out, size_t targets, int m, cudaStream_t st);
-// [L*L][m] FP64 stencil rows to the tap-major FP32 pair planes of the mixed form
-cudaError_t launch_weights_tapmajor(const double* in, float2* out, size_t targets, int m, cudaStream_t st);
-cudaError_t launch_time_f32(const double* t1, const double* dtr, int n, float* inv_len, float* inv_dtr,
+// FP32 mirrors of history elements [off, off + count) from the FP64 rows (mixed forms)
+cudaError_t launch_mirror(const DevCtx& c, size_t off, size_t count, cudaStream_t st);
+// [L*L][m] FP64 stencil rows to the tap-major planes of the mixed form `mixed` (1: float2, 2: float4)
+cudaError_t launch_weights_tapmajor(const double* in, void* out, int mixed, size_t targets, int m, cudaStream_t st);
+cudaError_t launch_time_f32(const double* t1, const double* dtr, int n, float2* inv_len, float2* inv_dtr,
                             cudaStream_t st);
+// FP32 (hi, lo) pair of an FP64 value
+__host__ __device__ inline float2 hi_lo(double v) {
+    const float h = (float)v;
+    return make_float2(h, (float)(v - (double)h));
+}
+inline void model_quads(const DModel& M, float4 q[4]) {
+    const double v[4] = {M.cA, M.cB, M.cC, M.cD};
+    for (int k = 0; k < 4; ++k) {
+        const float2 p = hi_lo(v[k]);
+        q[k] = make_float4(p.x, p.x, p.y, p.y);
+    }
+}
 cudaError_t launch_fp64_probe(double* out, int blocks, int threads, int iters, cudaStream_t st);
 cudaError_t launch_unpack_rows(const double2* in, double* QK, double* QR, size_t count,
                                cudaStream_t st);

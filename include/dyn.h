@@ -466,7 +466,9 @@ dyn_status dyn_batch_last_row(void* batch, int q, double* qK, double* qR);
  * the FP32-compensated level), not the algorithm. */
 dyn_status dyn_batch_tune(void* batch, int reps, int* threads, int* targets, int* ctas_per_sm, float* ms_best);
 /* Average device time of the gather kernel over `reps` launches for the
- * current stage of every running quench (the kernel is idempotent). */
+ * current stage of every running quench (the kernel is idempotent), with the
+ * B2 sums of that stage in place, as a stage finds them that goes on from
+ * another one of the same call. */
 dyn_status dyn_batch_profile(void* batch, int reps, float* ms_gather);
 
 /* ------------------------------------------------------ discrete adjoint */
