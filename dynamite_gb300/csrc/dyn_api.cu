@@ -61,6 +61,7 @@ struct Ctx {
     dyn_controller ctl{};
     int last_rollback_loop = -1000;  // loop of the last rollback (simulation_runner.cpp:53, :290)
     TailState* tail = nullptr;       // tail fit state across calls (device)
+    CompactBuf compact;              // sparsify workspace
     double specRad = 0.0;
     // pinned staging
     StageDev* stages_h = nullptr;
@@ -112,6 +113,7 @@ struct Ctx {
     void release() {
         drop_graphs();
         release_adjoint();
+        compact.release();
         if (stages_copied) cudaEventDestroy(stages_copied);
         stages_copied = nullptr;
         void* bufs[] = {(void*)d.theta, (void*)d.phi2, (void*)d.integ, (void*)d.iA1, (void*)d.iA2, (void*)d.iB2,
@@ -1601,36 +1603,27 @@ dyn_status dyn_sparsify(void* p, double threshold, int variant, size_t* n_out) {
     const size_t n = c->n;
     if (n_out) *n_out = n;
     if (n < 3) return DYN_OK;
-    unsigned char* fl_d;
-    if (dalloc(&fl_d, n)) return DYN_ERR_NOMEM;
+    CompactBuf& buf = c->compact;
+    cudaError_t e = buf.reserve(n, c->L);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        buf.release();
+        return fail(DYN_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
     std::vector<unsigned char> fl(n);
-    cudaError_t e = launch_sparsify_flags(c->d, (int)n, variant, threshold, fl_d, c->st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(fl.data(), fl_d, n, cudaMemcpyDeviceToHost, c->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
-    cudaFree(fl_d);
-    CK(e);
+    CK(launch_sparsify_flags(c->d, (int)n, variant, threshold, buf.flags, c->st));
+    CK(cudaMemcpyAsync(fl.data(), buf.flags, n, cudaMemcpyDeviceToHost, c->st));
+    CK(cudaStreamSynchronize(c->st));
     std::vector<int> inds, indsD;
     std::vector<double> tfac, t1n, dtrn;
     if (!sparsify_indices(fl.data(), n, variant, c->t1, c->dtr, inds, indsD, tfac, t1n, dtrn)) return DYN_OK;
     const int k = (int)inds.size();
-    // new buffers sized like the old capacity
-    double2 *KRn, *dKRn;
-    double *rn, *drn, *dtmp;
-    int* id;
     dyn_status s;
-    if ((s = dalloc(&KRn, c->cap * c->L)) || (s = dalloc(&dKRn, c->cap * c->L)) || (s = dalloc(&rn, c->cap)) ||
-        (s = dalloc(&drn, c->cap)) || (s = dalloc(&id, 2 * (size_t)k)) || (s = dalloc(&dtmp, (size_t)k)))
-        return s;
-    CK(cudaMemcpyAsync(id, inds.data(), k * sizeof(int), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(id + k, indsD.data(), k * sizeof(int), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(dtmp, tfac.data(), k * sizeof(double), cudaMemcpyHostToDevice, c->st));
-    CK(launch_compact(c->d, id, id + k, variant == 0 ? nullptr : dtmp, k, KRn, dKRn, rn, drn, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    cudaFree(id);
-    cudaFree(dtmp);
-    cudaFree(c->d.KR); cudaFree(c->d.dKR); cudaFree(c->d.rvec); cudaFree(c->d.drvec);
-    c->d.KR = KRn; c->d.dKR = dKRn; c->d.rvec = rn; c->d.drvec = drn;
-    c->drop_graphs();
+    CK(cudaMemcpyAsync(buf.idx, inds.data(), k * sizeof(int), cudaMemcpyHostToDevice, c->st));
+    CK(cudaMemcpyAsync(buf.idx + buf.cap, indsD.data(), k * sizeof(int), cudaMemcpyHostToDevice, c->st));
+    CK(cudaMemcpyAsync(buf.tf, tfac.data(), k * sizeof(double), cudaMemcpyHostToDevice, c->st));
+    CK(launch_compact(c->d, buf.idx, buf.idx + buf.cap, variant == 0 ? nullptr : buf.tf, k, buf, c->st));
+    CK(cudaStreamSynchronize(c->st));  // the host vectors above are sources of the copies
     c->t1 = t1n;
     c->dtr = dtrn;
     c->n = k;

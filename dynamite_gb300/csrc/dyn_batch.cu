@@ -462,8 +462,10 @@ struct Batch {
     cudaGraphExec_t graph = nullptr;
     int graph_ticks = 0;
     std::vector<void*> allocs;
+    CompactBuf compact;  // sparsify workspace
 
     ~Batch() {
+        compact.release();
         if (graph) cudaGraphExecDestroy(graph);
         for (void* p : allocs) cudaFree(p);
         if (plan_pin) cudaFreeHost(plan_pin);
@@ -595,8 +597,7 @@ struct Batch {
     }
 
     // One sparsify pass over quench b's history (the same flag and compaction
-    // kernels and index logic as dyn_sparsify), in place: rows are compacted
-    // into scratch and copied back, times, FP32 mirrors and the plan's row
+    // kernels and index logic as dyn_sparsify), in place: times, FP32 mirrors and the plan's row
     // count follow.  Call at a step boundary (status other than running).
     dyn_status sparsify_pass(int b, double thr, int variant, int* n_out) {
         Quench& q = qh[b];
@@ -604,54 +605,37 @@ struct Batch {
         const size_t n = (size_t)pl.n, L = q.c.L;
         *n_out = pl.n;
         if (n < 3) return DYN_OK;
-        unsigned char* fl_d = nullptr;
-        BCK(cudaMalloc(&fl_d, n));
+        cudaError_t e = compact.reserve(n, L);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            compact.release();
+            return bfail(DYN_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+        }
         std::vector<unsigned char> fl(n);
         std::vector<double> t1(n), dtr(n);
-        cudaError_t e = launch_sparsify_flags(q.c, (int)n, variant, thr, fl_d, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(fl.data(), fl_d, n, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(t1.data(), q.c.t1grid, n * sizeof(double), cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(dtr.data(), q.c.dtr, n * sizeof(double), cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        cudaFree(fl_d);
-        BCK(e);
+        BCK(launch_sparsify_flags(q.c, (int)n, variant, thr, compact.flags, st));
+        BCK(cudaMemcpyAsync(fl.data(), compact.flags, n, cudaMemcpyDeviceToHost, st));
+        BCK(cudaMemcpyAsync(t1.data(), q.c.t1grid, n * sizeof(double), cudaMemcpyDeviceToHost, st));
+        BCK(cudaMemcpyAsync(dtr.data(), q.c.dtr, n * sizeof(double), cudaMemcpyDeviceToHost, st));
+        BCK(cudaStreamSynchronize(st));
         std::vector<int> inds, indsD;
         std::vector<double> tfac, t1n, dtrn;
         if (!sparsify_indices(fl.data(), n, variant, t1, dtr, inds, indsD, tfac, t1n, dtrn)) return DYN_OK;
         const size_t k = inds.size();
-        double2 *KRn = nullptr, *dKRn = nullptr;
-        double *rn = nullptr, *drn = nullptr, *tf = nullptr;
-        int* id = nullptr;
-        auto release = [&]() {
-            cudaFree(KRn); cudaFree(dKRn); cudaFree(rn); cudaFree(drn); cudaFree(tf); cudaFree(id);
-        };
-        if ((e = cudaMalloc(&KRn, k * L * sizeof(double2))) != cudaSuccess ||
-            (e = cudaMalloc(&dKRn, k * L * sizeof(double2))) != cudaSuccess ||
-            (e = cudaMalloc(&rn, k * sizeof(double))) != cudaSuccess ||
-            (e = cudaMalloc(&drn, k * sizeof(double))) != cudaSuccess ||
-            (e = cudaMalloc(&tf, k * sizeof(double))) != cudaSuccess ||
-            (e = cudaMalloc(&id, 2 * k * sizeof(int))) != cudaSuccess) {
-            release();
-            return bfail(DYN_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-        }
         std::vector<double> inv(k);
         for (size_t r = 0; r < k; ++r) inv[r] = dtrn[r] != 0.0 ? 1.0 / dtrn[r] : 0.0;
+        int* id = compact.idx;
         const bool ok =
             cudaMemcpyAsync(id, inds.data(), k * sizeof(int), cudaMemcpyHostToDevice, st) == cudaSuccess &&
-            cudaMemcpyAsync(id + k, indsD.data(), k * sizeof(int), cudaMemcpyHostToDevice, st) == cudaSuccess &&
-            cudaMemcpyAsync(tf, tfac.data(), k * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess &&
-            launch_compact(q.c, id, id + k, variant == 0 ? nullptr : tf, (int)k, KRn, dKRn, rn, drn, st) == cudaSuccess &&
-            cudaMemcpyAsync(q.c.KR, KRn, k * L * sizeof(double2), cudaMemcpyDeviceToDevice, st) == cudaSuccess &&
-            cudaMemcpyAsync(q.c.dKR, dKRn, k * L * sizeof(double2), cudaMemcpyDeviceToDevice, st) == cudaSuccess &&
-            cudaMemcpyAsync(q.c.rvec, rn, k * sizeof(double), cudaMemcpyDeviceToDevice, st) == cudaSuccess &&
-            cudaMemcpyAsync(q.c.drvec, drn, k * sizeof(double), cudaMemcpyDeviceToDevice, st) == cudaSuccess &&
+            cudaMemcpyAsync(id + compact.cap, indsD.data(), k * sizeof(int), cudaMemcpyHostToDevice, st) == cudaSuccess &&
+            cudaMemcpyAsync(compact.tf, tfac.data(), k * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess &&
+            launch_compact(q.c, id, id + compact.cap, variant == 0 ? nullptr : compact.tf, (int)k, compact, st) == cudaSuccess &&
             cudaMemcpyAsync(q.c.t1grid, t1n.data(), k * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess &&
             cudaMemcpyAsync(q.c.dtr, dtrn.data(), k * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess &&
             cudaMemcpyAsync(q.c.inv_dtr, inv.data(), k * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess &&
             launch_mirror(q.c, 0, k * L, st) == cudaSuccess &&
             launch_time_f32(q.c.t1grid, q.c.dtr, (int)k, q.c.inv_len_f, q.c.inv_dtr_f, st) == cudaSuccess;
         e = cudaStreamSynchronize(st);  // the host vectors above are sources of the copies
-        release();
         if (!ok || e != cudaSuccess) return bfail(DYN_ERR_CUDA, "batch sparsify: " + std::string(cudaGetErrorString(cudaGetLastError())));
         pl.n = (int)k;
         pl.T_last = t1n[k - 1];

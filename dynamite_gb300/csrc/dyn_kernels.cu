@@ -18,6 +18,7 @@
 // interpolation arrays and the RHS with the reference CPU build's operation
 // order (no FMA contraction) for the C-ABI calls that mirror
 // interpolateGPU/QKRstepGPU one to one.
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include "dyn_epi.cuh"
@@ -334,31 +335,16 @@ __global__ void __launch_bounds__(EPI_T) k_epi(const DevCtx c, const int s) {
 }
 
 // ------------------------------------------------------------------------
-// Positions of the current state (after init/upload/sparsify/rollback).
+// Positions and B1 rows of the current state (after init/upload/sparsify/rollback).
 __global__ void k_pos_init(const DevCtx c, const int nrows) {
-    const int L = c.L;
-    __shared__ double s_max[32];
     const double T = c.t1grid[nrows - 1];
     const ListView lv{c.t1grid, nrows, T};
-    double mx = 0.0;
-    for (int i = threadIdx.x; i < L; i += blockDim.x) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < c.L; i += gridDim.x * blockDim.x) {
         const double p = search_pos(c.search, lv, __dmul_rn(c.theta[i], T));
         c.posB1x[i] = p;
         c.b1[i] = b1_row(c, p, nrows - 1 < 1 ? 1 : nrows - 1, nrows);
-        mx = fmax(mx, p);
     }
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double m = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, s_max[w]);
-        long long mc = (long long)ceil(m) - 1;
-        c.slots->maxceil = (int)(mc < 1 ? 1 : mc);
-        const double p = search_pos(c.search, lv, __dmul_rn(c.phi2[(size_t)L * L - 1], T));
-        c.slots->maxX = (int)(long long)(p - 0.5);
-        c.slots->counter = 0;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) c.slots->counter = 0;
 }
 
 // ------------------------------------------------------------------------
@@ -564,116 +550,150 @@ __global__ void k_rint_exact(const DevCtx c, const int nrows) {
     }
 }
 
-// ConvA/ConvR of one row, convolution.cpp:5-50 order
-__device__ double conv_row_exact(const DevCtx& c, const double* f, const double* g, int row) {
-    const int L = c.L;
-    double o = 0.0;
-    for (int k = 0; k < L; ++k) o = add(o, mul(mul(c.integ[k], f[(size_t)row * L + k]), g[(size_t)row * L + k]));
-    return o;
+// Sums in the reference's order.  The terms of a sum are formed by all threads, SUM_W columns
+// at a time, in shared memory; one thread per sum adds them in column order.  So only the adds
+// are a serial chain (512 of them ~13 us), not the loads and the products (L = 512: rstep 439
+// -> 26 us, energy 257 -> 23, QKRstep, eight sums a row, 759 -> 36).
+constexpr int SUM_W = 256;  // columns per block of terms, and threads of a CTA
+template <int N>
+using SumTerms = double[N][SUM_W + 1];  // + 1: the adding threads read different banks
+// term(j, put) forms column j's N terms and hands them over with put(k, value); thread k < N
+// returns sum k
+template <int N, typename Term>
+__device__ __forceinline__ double ordered_sums(const int L, SumTerms<N>& s_t, Term term) {
+    double sum = 0.0;
+    for (int j0 = 0; j0 < L; j0 += SUM_W) {
+        const int w = min(SUM_W, L - j0);
+        if (threadIdx.x < w) term(j0 + threadIdx.x, [&](int k, double v) { s_t[k][threadIdx.x] = v; });
+        __syncthreads();
+        if (threadIdx.x < N) {
+            const double* t = s_t[threadIdx.x];
+#pragma unroll 8
+            for (int q = 0; q < w; ++q) sum = add(sum, t[q]);
+        }
+        __syncthreads();
+    }
+    return sum;
 }
 
-// QKstep / QRstep (time_steps.cpp:27-47, 94-100) on the materialized arrays
-__global__ void k_qkr_exact(const DevCtx c, const int nrows, double2* out) {
-    const int L = c.L;
-    const size_t L2 = (size_t)L * L;
+// QKstep / QRstep (time_steps.cpp:27-47, 94-100) on the materialized arrays, a CTA per row
+__global__ void __launch_bounds__(SUM_W) k_qkr_exact(const DevCtx c, const int nrows, double2* out) {
+    const int L = c.L, i = blockIdx.x;
+    const size_t L2 = (size_t)L * L, row = (size_t)i * L;
     const DModel Mo = c.M;
     const double t = c.t1grid[nrows - 1];
     const double* ip = c.ip;
     const double2* q = c.KR + (size_t)(nrows - 1) * L;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < L; i += gridDim.x * blockDim.x) {
-        const double th = c.theta[i];
-        const double tA = mul(t, th), tR = mul(t, sub(1.0, th));
-        const double rE = c.rint[L - 1];
-        const double q0 = q[0].x;
-        const double cR1 = mul(conv_row_exact(c, ip + 11 * L2, ip + 6 * L2, i), tR);   // SigmaRA2, QKB2
-        const double cA1 = mul(conv_row_exact(c, ip + 9 * L2, ip + 4 * L2, i), tA);    // SigmaRA1, QKB1
-        const double cA2 = mul(conv_row_exact(c, ip + 8 * L2, ip + 5 * L2, i), tA);    // SigmaKA1, QRB1
-        const double cR2 = mul(conv_row_exact(c, ip + 3 * L2, ip + 14 * L2, i), tR);   // QRA2, SigmaKB2
-        const double cA3 = mul(conv_row_exact(c, ip + 1 * L2, ip + 12 * L2, i), tA);   // QRA1, SigmaKB1
-        const double cA4 = mul(conv_row_exact(c, ip + 0 * L2, ip + 13 * L2, i), tA);   // QKA1, SigmaRB1
-        const double cR3 = mul(conv_row_exact(c, ip + 11 * L2, ip + 7 * L2, i), tR);   // SigmaRA2, QRB2
-        const double cR4 = mul(conv_row_exact(c, ip + 3 * L2, ip + 15 * L2, i), tR);   // QRA2, SigmaRB2
-        const double qb = ip[4 * L2 + (size_t)i * L];
-        const double fac1 = dvd(Df_x(Mo, q0), Mo.T0);
-        const double d1 = add(add(add(add(mul(qb, fac1), mul(q[i].x, -rE)), cR1), cA1), cA2);
-        const double fac2 = dvd(q0, Mo.T0);
-        const double d2 = sub(add(add(add(add(mul(Df_x(Mo, qb), fac2), mul(q[i].y, mul(2.0, Mo.Gamma))), cR2), cA3), cA4),
-                              mul(q[i].x, c.rint[i]));
-        const double hK = add(d1, mul(d2, th));
-        const double e1 = add(mul(q[i].y, -rE), cR3);
-        const double e2 = sub(mul(q[i].y, c.rint[i]), cR4);
-        out[i] = make_double2(hK, add(e1, mul(e2, th)));
-    }
+    __shared__ SumTerms<8> s_t;
+    __shared__ double s_sum[8];
+    // ConvA/ConvR rows in convolution.cpp:5-50 order
+    const double sum = ordered_sums<8>(L, s_t, [&](int j, auto put) {
+        const double w = c.integ[j];
+        const double* p = ip + row + j;
+        const double wRA2 = mul(w, p[11 * L2]), wQRA2 = mul(w, p[3 * L2]);
+        put(0, mul(wRA2, p[6 * L2]));                // SigmaRA2, QKB2
+        put(1, mul(mul(w, p[9 * L2]), p[4 * L2]));   // SigmaRA1, QKB1
+        put(2, mul(mul(w, p[8 * L2]), p[5 * L2]));   // SigmaKA1, QRB1
+        put(3, mul(wQRA2, p[14 * L2]));              // QRA2, SigmaKB2
+        put(4, mul(mul(w, p[1 * L2]), p[12 * L2]));  // QRA1, SigmaKB1
+        put(5, mul(mul(w, p[0 * L2]), p[13 * L2]));  // QKA1, SigmaRB1
+        put(6, mul(wRA2, p[7 * L2]));                // SigmaRA2, QRB2
+        put(7, mul(wQRA2, p[15 * L2]));              // QRA2, SigmaRB2
+    });
+    if (threadIdx.x < 8) s_sum[threadIdx.x] = sum;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    const double th = c.theta[i];
+    const double tA = mul(t, th), tR = mul(t, sub(1.0, th));
+    const double rE = c.rint[L - 1];
+    const double q0 = q[0].x;
+    const double cR1 = mul(s_sum[0], tR), cA1 = mul(s_sum[1], tA), cA2 = mul(s_sum[2], tA);
+    const double cR2 = mul(s_sum[3], tR), cA3 = mul(s_sum[4], tA), cA4 = mul(s_sum[5], tA);
+    const double cR3 = mul(s_sum[6], tR), cR4 = mul(s_sum[7], tR);
+    const double qb = ip[4 * L2 + row];
+    const double fac1 = dvd(Df_x(Mo, q0), Mo.T0);
+    const double d1 = add(add(add(add(mul(qb, fac1), mul(q[i].x, -rE)), cR1), cA1), cA2);
+    const double fac2 = dvd(q0, Mo.T0);
+    const double d2 = sub(add(add(add(add(mul(Df_x(Mo, qb), fac2), mul(q[i].y, mul(2.0, Mo.Gamma))), cR2), cA3), cA4),
+                          mul(q[i].x, c.rint[i]));
+    const double hK = add(d1, mul(d2, th));
+    const double e1 = add(mul(q[i].y, -rE), cR3);
+    const double e2 = sub(mul(q[i].y, c.rint[i]), cR4);
+    out[i] = make_double2(hK, add(e1, mul(e2, th)));
 }
 
-// rstep (time_steps.cpp:83-92), one thread, reference order
-__global__ void k_rstep_exact(const DevCtx c, const int nrows, double* out) {
-    const int L = c.L;
+// rstep (time_steps.cpp:83-92), one CTA
+__global__ void __launch_bounds__(SUM_W) k_rstep_exact(const DevCtx c, const int nrows, double* out) {
     const DModel Mo = c.M;
     const double t = c.t1grid[nrows - 1];
-    const double2* q = c.KR + (size_t)(nrows - 1) * L;
-    double A = 0.0, B = 0.0;
-    for (int j = 0; j < L; ++j) {
-        const double sk = Df_x(Mo, q[j].x), sr = mul(DDf_x(Mo, q[j].x), q[j].y);
-        A = add(A, mul(mul(mul(t, c.integ[j]), sr), q[j].x));
-        B = add(B, mul(mul(mul(t, c.integ[j]), sk), q[j].y));
-    }
-    const double sk0 = Df_x(Mo, q[0].x);
-    out[0] = add(add(add(Mo.Gamma, A), B), dvd(mul(sk0, q[0].x), Mo.T0));
+    const double2* q = c.KR + (size_t)(nrows - 1) * c.L;
+    __shared__ SumTerms<2> s_t;
+    __shared__ double s_sum[2];
+    const double sum = ordered_sums<2>(c.L, s_t, [&](int j, auto put) {
+        const double2 v = q[j];
+        const double tw = mul(t, c.integ[j]);
+        put(0, mul(mul(tw, mul(DDf_x(Mo, v.x), v.y)), v.x));
+        put(1, mul(mul(tw, Df_x(Mo, v.x)), v.y));
+    });
+    if (threadIdx.x < 2) s_sum[threadIdx.x] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        out[0] = add(add(add(Mo.Gamma, s_sum[0]), s_sum[1]), dvd(mul(Df_x(Mo, q[0].x), q[0].x), Mo.T0));
 }
 
-// drstep2 (time_steps.cpp:117-125), one thread, reference order
-__global__ void k_drstep2_exact(const DevCtx c, const double* qK, const double* qR, const double* dqK,
-                                const double* dqR, const double t, double* out) {
-    const int L = c.L;
+// drstep2 (time_steps.cpp:117-125), one CTA
+__global__ void __launch_bounds__(SUM_W) k_drstep2_exact(const DevCtx c, const double* qK, const double* qR,
+                                                         const double* dqK, const double* dqR, const double t, double* out) {
     const DModel Mo = c.M;
-    double S[6] = {0, 0, 0, 0, 0, 0};
-    double dsk0 = 0.0, sk0 = 0.0;
-    for (int j = 0; j < L; ++j) {
+    __shared__ SumTerms<6> s_t;
+    __shared__ double s_sum[6];
+    const double sum = ordered_sums<6>(c.L, s_t, [&](int j, auto put) {
         const double q = qK[j], r = qR[j], dq = dqK[j], dr = dqR[j];
         const double sk = Df_x(Mo, q), sr = mul(DDf_x(Mo, q), r);
         const double dsk = add(mul(DDf_x(Mo, q), dq), mul(0.0, dr));
         const double dsr = add(mul(mul(DDDf_x(Mo, q), r), dq), mul(DDf_x(Mo, q), dr));
         const double w = c.integ[j], tw = mul(t, w);
-        S[0] = add(S[0], mul(mul(mul(1.0, w), sr), q));
-        S[1] = add(S[1], mul(mul(mul(1.0, w), sk), r));
-        S[2] = add(S[2], mul(mul(tw, dsr), q));
-        S[3] = add(S[3], mul(mul(tw, dsk), r));
-        S[4] = add(S[4], mul(mul(tw, sr), dq));
-        S[5] = add(S[5], mul(mul(tw, sk), dr));
-        if (j == 0) { dsk0 = dsk; sk0 = sk; }
-    }
+        put(0, mul(mul(mul(1.0, w), sr), q));
+        put(1, mul(mul(mul(1.0, w), sk), r));
+        put(2, mul(mul(tw, dsr), q));
+        put(3, mul(mul(tw, dsk), r));
+        put(4, mul(mul(tw, sr), dq));
+        put(5, mul(mul(tw, sk), dr));
+    });
+    if (threadIdx.x < 6) s_sum[threadIdx.x] = sum;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    const double dsk0 = add(mul(DDf_x(Mo, qK[0]), dqK[0]), mul(0.0, dqR[0])), sk0 = Df_x(Mo, qK[0]);
     const double term = dvd(add(mul(dsk0, qK[0]), mul(sk0, dqK[0])), Mo.T0);
-    out[0] = add(add(add(add(add(add(S[0], S[1]), S[2]), S[3]), S[4]), S[5]), term);
+    out[0] = add(add(add(add(add(add(s_sum[0], s_sum[1]), s_sum[2]), s_sum[3]), s_sum[4]), s_sum[5]), term);
 }
 
-// energy at t1grid.back() (time_steps.cu:641-674 with the CPU sum order)
-__global__ void k_energy_exact(const DevCtx c, const int nrows, double* out) {
-    const int L = c.L;
+// energy at t1grid.back() (time_steps.cu:641-674 with the CPU sum order), one CTA
+__global__ void __launch_bounds__(SUM_W) k_energy_exact(const DevCtx c, const int nrows, double* out) {
     const DModel Mo = c.M;
     const double t = c.t1grid[nrows - 1];
-    const double2* q = c.KR + (size_t)(nrows - 1) * L;
-    double A = 0.0;
-    for (int j = 0; j < L; ++j) A = add(A, mul(mul(mul(t, c.integ[j]), Df_x(Mo, q[j].x)), q[j].y));
-    out[0] = -add(A, dvd(Df_x(Mo, q[0].x), Mo.T0));
+    const double2* q = c.KR + (size_t)(nrows - 1) * c.L;
+    __shared__ SumTerms<1> s_t;
+    const double sum = ordered_sums<1>(c.L, s_t, [&](int j, auto put) {
+        const double2 v = q[j];
+        put(0, mul(mul(mul(t, c.integ[j]), Df_x(Mo, v.x)), v.y));
+    });
+    if (threadIdx.x == 0) out[0] = -add(sum, dvd(Df_x(Mo, q[0].x), Mo.T0));
 }
 
 // ConvA / ConvR on device arrays (convolution.cpp:5-50)
-__global__ void k_conv_exact(const DevCtx c, const int kind, const double* f, const double* g,
-                             const int depth, const double t, double* out) {
-    const int L = c.L;
-    if (depth == 1) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-            double temp = 0.0;
-            for (int j = 0; j < L; ++j) temp = add(temp, mul(mul(mul(t, c.integ[j]), f[j]), g[j]));
-            out[0] = temp;
-        }
-        return;
-    }
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < depth; r += gridDim.x * blockDim.x) {
-        const double o = conv_row_exact(c, f, g, r);
-        out[r] = mul(o, kind == 0 ? mul(t, c.theta[r]) : mul(t, sub(1.0, c.theta[r])));
-    }
+__global__ void __launch_bounds__(SUM_W) k_conv_exact(const DevCtx c, const int kind, const double* f, const double* g,
+                                                      const int depth, const double t, double* out) {
+    const int L = c.L, r = blockIdx.x;
+    __shared__ SumTerms<1> s_t;
+    const double sum = ordered_sums<1>(L, s_t, [&](int j, auto put) {
+        const size_t e = (size_t)r * L + j;
+        const double w = depth == 1 ? mul(t, c.integ[j]) : c.integ[j];
+        put(0, mul(mul(w, f[e]), g[e]));
+    });
+    if (threadIdx.x != 0) return;
+    if (depth == 1) out[0] = sum;
+    else out[r] = mul(sum, kind == 0 ? mul(t, c.theta[r]) : mul(t, sub(1.0, c.theta[r])));
 }
 
 __global__ void k_search(const int mode, const double* list, const int nlist, const double* elem,
@@ -684,58 +704,119 @@ __global__ void k_search(const int mode, const double* list, const int nlist, co
         out[k] = search_pos(mode, lv, __dmul_rn(elem[k], last));
 }
 
-// sparsify indicator per node, one thread per node, reference summation order
-__global__ void k_sparsify_flags(const DevCtx c, const int n, const int variant, const double thr,
-                                 unsigned char* flags) {
-    const int L = c.L;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        unsigned char keep;
-        const bool interior = i >= 2 && i + 1 < n;
-        const bool evaluate = interior && (variant != 2 || (i % 2) == 0);
-        if (evaluate) {
-            const double tl = c.t1grid[i - 2], tm = c.t1grid[i];
-            const double td1 = sub(c.t1grid[i - 1], tl), td2 = sub(tm, tl), td3 = sub(c.t1grid[i + 1], tm);
-            const double sc = dvd(td2, 12.0);
-            const double2* X2 = c.KR + (size_t)(i - 2) * L;
-            const double2* X0 = c.KR + (size_t)i * L;
-            const double2* D1 = c.dKR + (size_t)(i - 1) * L;
-            const double2* D3 = c.dKR + (size_t)(i + 1) * L;
-            double val = 0.0;
-            auto term = [&](double f1, double df1, double df2) {
-                return fabs(mul(sc, sub(mul(2.0, f1), mul(td2, add(dvd(df1, td1), dvd(df2, td3))))));
-            };
-            if (variant == 2) {
-                for (int j = 0; j < L; ++j) {
-                    val = add(val, term(sub(X0[j].x, X2[j].x), D1[j].x, D3[j].x));
-                    val = add(val, term(sub(X0[j].y, X2[j].y), D1[j].y, D3[j].y));
-                }
-            } else {
-                for (int j = 0; j < L; ++j) val = add(val, term(sub(X0[j].x, X2[j].x), D1[j].x, D3[j].x));
-                for (int j = 0; j < L; ++j) val = add(val, term(sub(X0[j].y, X2[j].y), D1[j].y, D3[j].y));
-                if (variant == 0)
-                    val = add(val, term(sub(c.rvec[i], c.rvec[i - 2]), c.drvec[i - 1], c.drvec[i + 1]));
-            }
-            keep = (unsigned char)(1 | (val < thr ? 2 : 0) | (val >= thr ? 4 : 0));
-        } else {
-            keep = 0;
-        }
-        flags[i] = keep;  // bit0 evaluated, bit1 val < thr, bit2 val >= thr
+// x / d correctly rounded for many x and one d: y = RN(1/d); q = x y is off by an ulp or two,
+// one Newton correction q + (x - q d) y leaves it within one, and from there the same step
+// rounds correctly (Markstein, IBM J. Res. Dev. 34, 1990).  Five FP64 instructions; the general
+// division where y or the remainders could leave the normal range.
+struct DivBy {
+    double d, y;
+    bool ok;
+    __device__ __forceinline__ void set(double d_) {
+        d = d_;
+        y = dvd(1.0, d_);
+        ok = fabs(d) > 1e-150 && fabs(d) < 1e150;
     }
+    __device__ __forceinline__ double operator()(double x) const {
+        const double m = fabs(x);
+        if (!ok || !(m > 1e-120 && m < 1e120)) return m == 0.0 && ok ? 0.0 : dvd(x, d);
+        double q = mul(x, y);
+        q = fma(fma(-q, d, x), y, q);
+        return fma(fma(-q, d, x), y, q);
+    }
+};
+
+// Sparsify indicator of every node (bit 0 evaluated, bit 1 val < thr, bit 2 val >= thr): val is a
+// sum over the columns in the reference's order.  A CTA takes SP_NODES evaluated nodes; its
+// warps form the terms of 32 columns of a node side by side (coalesced rows), the node's own
+// thread adds them in order.  Bound by the FP64 pipe (16 instructions a term: the two
+// divisions share each row's divisor); n = 8000, L = 512: 847 us with a thread per node, whole
+// divisions and strided reads; the whole sparsify pass 1.56 -> 0.68 ms.
+constexpr int SP_NODES = 16, SP_T = 256;
+__global__ void __launch_bounds__(SP_T) k_sparsify_flags(const DevCtx c, const int n, const int variant, const double thr,
+                                                         unsigned char* flags) {
+    const int L = c.L, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ double s_t[2][2][SP_NODES][33];  // [tile parity][QK, QR]: the adds of one tile run beside the next one's terms
+    __shared__ double s_td2[SP_NODES], s_sc[SP_NODES];
+    __shared__ DivBy s_by1[SP_NODES], s_by3[SP_NODES];
+    // evaluated nodes: 2 <= i < n - 1, of variant 2 the even ones
+    const int step = variant == 2 ? 2 : 1, e0 = blockIdx.x * SP_NODES;
+    auto node = [&](int k) { return 2 + (e0 + k) * step; };
+    if (threadIdx.x < SP_NODES) {
+        const int k = threadIdx.x, i = node(k);
+        if (i + 1 < n) {
+            const double tl = c.t1grid[i - 2], tm = c.t1grid[i];
+            s_td2[k] = sub(tm, tl);
+            s_sc[k] = dvd(s_td2[k], 12.0);
+            s_by1[k].set(sub(c.t1grid[i - 1], tl));
+            s_by3[k].set(sub(c.t1grid[i + 1], tm));
+        }
+    }
+    __syncthreads();
+    double val = 0.0;  // of node(threadIdx.x), threadIdx.x < SP_NODES
+    // variants 0, 1: all QK terms, then all QR terms; variant 2: the two of a column in turn
+    const int passes = variant == 2 ? 1 : 2, tiles = (L + 31) / 32;
+    for (int tile = 0; tile < passes * tiles; ++tile) {
+        const int pass = tile >= tiles, j0 = (tile - pass * tiles) * 32;
+        double(*t)[SP_NODES][33] = s_t[tile & 1];
+        for (int k = warp; k < SP_NODES; k += SP_T / 32) {
+            const int i = node(k), j = j0 + lane;
+            if (i + 1 >= n || j >= L) continue;
+            const double td2 = s_td2[k], sc = s_sc[k];
+            const DivBy by1 = s_by1[k], by3 = s_by3[k];
+            auto term = [&](double f1, double df1, double df2) {
+                return fabs(mul(sc, sub(mul(2.0, f1), mul(td2, add(by1(df1), by3(df2))))));
+            };
+            const size_t at = (size_t)i * L + j;
+            const double2 x0 = c.KR[at], x2 = c.KR[at - 2 * (size_t)L], d1 = c.dKR[at - L], d3 = c.dKR[at + L];
+            if (variant == 2 || pass == 0) t[0][k][lane] = term(sub(x0.x, x2.x), d1.x, d3.x);
+            if (variant == 2 || pass == 1) t[1][k][lane] = term(sub(x0.y, x2.y), d1.y, d3.y);
+        }
+        __syncthreads();
+        if (threadIdx.x < SP_NODES && node(threadIdx.x) + 1 < n) {
+            const int w = min(32, L - j0);
+            for (int q = 0; q < w; ++q) {
+                if (variant == 2) {
+                    val = add(val, t[0][threadIdx.x][q]);
+                    val = add(val, t[1][threadIdx.x][q]);
+                } else {
+                    val = add(val, t[pass][threadIdx.x][q]);
+                }
+            }
+        }
+    }
+    if (threadIdx.x < SP_NODES) {
+        const int i = node(threadIdx.x);
+        if (i + 1 < n) {
+            if (variant == 0) {
+                const double tl = c.t1grid[i - 2], tm = c.t1grid[i];
+                const double td1 = sub(c.t1grid[i - 1], tl), td2 = sub(tm, tl), td3 = sub(c.t1grid[i + 1], tm);
+                const double f1 = sub(c.rvec[i], c.rvec[i - 2]);
+                val = add(val, fabs(mul(dvd(td2, 12.0), sub(mul(2.0, f1), mul(td2, add(dvd(c.drvec[i - 1], td1),
+                                                                                       dvd(c.drvec[i + 1], td3)))))));
+            }
+            flags[i] = (unsigned char)(1 | (val < thr ? 2 : 0) | (val >= thr ? 4 : 0));
+        }
+    }
+    // the nodes nothing is evaluated for
+    const int t = blockIdx.x * SP_T + threadIdx.x;
+    for (int i = t; i < n; i += gridDim.x * SP_T)
+        if (i < 2 || i + 1 >= n || (variant == 2 && (i & 1))) flags[i] = 0;
 }
 
-__global__ void k_compact(const DevCtx c, const int* inds, const int* indsD, const double* tfac, const int k,
-                          double2* KRn, double2* dKRn, double* rn, double* drn) {
+// Rows [r0, r0 + rows) of the compacted history into staging
+__global__ void k_compact(const DevCtx c, const int* inds, const int* indsD, const double* tfac, const int r0,
+                          const int rows, double2* KRn, double2* dKRn, double* rn, double* drn) {
     const int L = c.L;
-    const size_t total = (size_t)k * L;
+    const size_t total = (size_t)rows * L;
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const int r = (int)(e / L), j = (int)(e % L);
+        const int r = r0 + (int)(e / L), j = (int)(e % L);
         KRn[e] = c.KR[(size_t)inds[r] * L + j];
         const double f = tfac ? tfac[r] : 1.0;
         const double2 d = c.dKR[(size_t)indsD[r] * L + j];
         dKRn[e] = make_double2(mul(f, d.x), mul(f, d.y));
         if (j == 0) {
-            rn[r] = c.rvec[inds[r]];
-            drn[r] = mul(f, c.drvec[indsD[r]]);
+            rn[e / L] = c.rvec[inds[r]];
+            drn[e / L] = mul(f, c.drvec[indsD[r]]);
         }
     }
 }
@@ -841,7 +922,7 @@ cudaError_t launch_epi_only(const DevCtx& c, int s, cudaStream_t st) {
 }
 
 cudaError_t launch_pos_init(const DevCtx& c, int nrows, cudaStream_t st) {
-    k_pos_init<<<1, 256, 0, st>>>(c, nrows);
+    k_pos_init<<<(c.L + 63) / 64, 64, 0, st>>>(c, nrows);
     return cudaGetLastError();
 }
 
@@ -863,30 +944,30 @@ cudaError_t launch_b1_exact(const DevCtx& c, int nrows, double* qk, double* qr, 
 }
 
 cudaError_t launch_qkr_exact(const DevCtx& c, int nrows, double2* out, cudaStream_t st) {
-    k_qkr_exact<<<(c.L + 31) / 32, 32, 0, st>>>(c, nrows, out);
+    k_qkr_exact<<<c.L, SUM_W, 0, st>>>(c, nrows, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_rstep_exact(const DevCtx& c, int nrows, double* out, cudaStream_t st) {
-    k_rstep_exact<<<1, 1, 0, st>>>(c, nrows, out);
+    k_rstep_exact<<<1, SUM_W, 0, st>>>(c, nrows, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_drstep2_exact(const DevCtx& c, const double* qK, const double* qR, const double* dqK,
                                  const double* dqR, double t, double* out, cudaStream_t st) {
-    k_drstep2_exact<<<1, 1, 0, st>>>(c, qK, qR, dqK, dqR, t, out);
+    k_drstep2_exact<<<1, SUM_W, 0, st>>>(c, qK, qR, dqK, dqR, t, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_energy_exact(const DevCtx& c, int nrows, double* out, cudaStream_t st) {
-    k_energy_exact<<<1, 1, 0, st>>>(c, nrows, out);
+    k_energy_exact<<<1, SUM_W, 0, st>>>(c, nrows, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_conv_exact(const DevCtx& c, int kind, const double* f, const double* g, size_t n, double t,
                               double* out, cudaStream_t st) {
     const int depth = (int)(n / c.L);
-    k_conv_exact<<<(depth + 31) / 32, 32, 0, st>>>(c, kind, f, g, depth, t, out);
+    k_conv_exact<<<depth, SUM_W, 0, st>>>(c, kind, f, g, depth, t, out);
     return cudaGetLastError();
 }
 
@@ -899,16 +980,67 @@ cudaError_t launch_search(const DevCtx& c, const double* list, size_t nlist, con
 
 cudaError_t launch_sparsify_flags(const DevCtx& c, int n, int variant, double thr, unsigned char* flags,
                                   cudaStream_t st) {
-    k_sparsify_flags<<<(n + 63) / 64, 64, 0, st>>>(c, n, variant, thr, flags);
+    const int nodes = n < 4 ? 0 : variant == 2 ? (n - 2) / 2 : n - 3;
+    k_sparsify_flags<<<std::max(1, (nodes + SP_NODES - 1) / SP_NODES), SP_T, 0, st>>>(c, n, variant, thr, flags);
     return cudaGetLastError();
 }
 
+// The history compacted in place: row r takes inds[r] and, scaled, derivative row indsD[r].
+// Both are at or above r and increase, so chunks of rows go through the staging buffers in
+// order without reaching rows still to be read.
 cudaError_t launch_compact(const DevCtx& c, const int* inds, const int* indsD, const double* tfac, int k,
-                           double2* KRn, double2* dKRn, double* rn, double* drn, cudaStream_t st) {
-    const size_t total = (size_t)k * c.L;
-    const int blocks = (int)((total + 255) / 256 < 8192 ? (total + 255) / 256 : 8192);
-    k_compact<<<blocks > 0 ? blocks : 1, 256, 0, st>>>(c, inds, indsD, tfac, k, KRn, dKRn, rn, drn);
-    return cudaGetLastError();
+                           const CompactBuf& buf, cudaStream_t st) {
+    const size_t L = c.L;
+    for (size_t r0 = 0; r0 < (size_t)k; r0 += buf.rows) {
+        const size_t rows = std::min(buf.rows, (size_t)k - r0), total = rows * L;
+        const int blocks = (int)((total + 255) / 256 < 8192 ? (total + 255) / 256 : 8192);
+        k_compact<<<blocks, 256, 0, st>>>(c, inds, indsD, tfac, (int)r0, (int)rows, buf.KR, buf.dKR, buf.r, buf.dr);
+        cudaError_t e = cudaGetLastError();
+        auto back = [&](void* dst, const void* src, size_t bytes) {
+            if (e == cudaSuccess) e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, st);
+        };
+        back(c.KR + r0 * L, buf.KR, total * sizeof(double2));
+        back(c.dKR + r0 * L, buf.dKR, total * sizeof(double2));
+        back(c.rvec + r0, buf.r, rows * sizeof(double));
+        back(c.drvec + r0, buf.dr, rows * sizeof(double));
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+cudaError_t CompactBuf::reserve(size_t n, size_t L) {
+    // flags and index lists of n rows; staging of at most 64 MB
+    if (n > cap) {
+        cudaFree(flags); cudaFree(idx); cudaFree(tf);
+        flags = nullptr; idx = nullptr; tf = nullptr;
+        cap = 0;
+        cudaError_t e = cudaMalloc((void**)&flags, n);
+        if (e == cudaSuccess) e = cudaMalloc((void**)&idx, 2 * n * sizeof(int));
+        if (e == cudaSuccess) e = cudaMalloc((void**)&tf, n * sizeof(double));
+        if (e != cudaSuccess) return e;
+        cap = n;
+    }
+    const size_t want = std::min(n, std::max<size_t>(1, (64u << 20) / (2 * L * sizeof(double2))));
+    if (want > rows || L > len) {
+        cudaFree(KR); cudaFree(dKR); cudaFree(r); cudaFree(dr);
+        KR = dKR = nullptr;
+        r = dr = nullptr;
+        rows = 0;
+        const size_t l = std::max(L, len), w = std::max(want, rows);
+        cudaError_t e = cudaMalloc((void**)&KR, w * l * sizeof(double2));
+        if (e == cudaSuccess) e = cudaMalloc((void**)&dKR, w * l * sizeof(double2));
+        if (e == cudaSuccess) e = cudaMalloc((void**)&r, w * sizeof(double));
+        if (e == cudaSuccess) e = cudaMalloc((void**)&dr, w * sizeof(double));
+        if (e != cudaSuccess) return e;
+        rows = w;
+        len = l;
+    }
+    return cudaSuccess;
+}
+
+void CompactBuf::release() {
+    for (void* p : {(void*)flags, (void*)idx, (void*)tf, (void*)KR, (void*)dKR, (void*)r, (void*)dr}) cudaFree(p);
+    *this = CompactBuf{};
 }
 
 cudaError_t launch_pack_rows(const double* QK, const double* QR, double2* out, size_t count, cudaStream_t st) {

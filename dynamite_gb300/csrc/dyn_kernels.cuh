@@ -276,9 +276,21 @@ cudaError_t launch_search(const DevCtx& c, const double* list, size_t nlist, con
                           size_t nelem, double* out, cudaStream_t st);
 cudaError_t launch_sparsify_flags(const DevCtx& c, int nrows, int variant, double threshold,
                                   unsigned char* flags, cudaStream_t st);
-cudaError_t launch_compact(const DevCtx& c, const int* inds, const int* indsD, const double* tfac,
-                           int k, double2* KRn, double2* dKRn, double* rn, double* drn,
-                           cudaStream_t st);
+// Workspace of sparsify passes, kept by its context or batch from the first one on: node flags
+// and index lists for `cap` rows, staging for `rows` rows of length `len` (at most 64 MB)
+struct CompactBuf {
+    unsigned char* flags = nullptr;
+    int* idx = nullptr;  // [2 cap]
+    double* tf = nullptr;
+    size_t cap = 0;
+    double2 *KR = nullptr, *dKR = nullptr;
+    double *r = nullptr, *dr = nullptr;
+    size_t rows = 0, len = 0;
+    cudaError_t reserve(size_t n, size_t L);
+    void release();
+};
+cudaError_t launch_compact(const DevCtx& c, const int* inds, const int* indsD, const double* tfac, int k,
+                           const CompactBuf& buf, cudaStream_t st);
 cudaError_t launch_pack_rows(const double* QK, const double* QR, double2* out, size_t count,
                              cudaStream_t st);
 cudaError_t launch_main_mixed(const DevCtx& c, int s, cudaStream_t st);
