@@ -365,10 +365,9 @@ __global__ void __launch_bounds__(EPI_T) k_batch_epi(const Quench* __restrict__ 
     const StageDev& sp = q.stg[pl.sidx * SMAX + s];
     const DevCtx& c = q.c;
     const unsigned G = (unsigned)((c.L + EPI_ROWS - 1) / EPI_ROWS);
-    double ep[EP_N];
-    epi::rows<P, P2, true>(c, sp, s, (int)blk, is_fsal(pl, sp, call), ep);
-    if (!epi::elect_last(c, ep, blk, G)) return;
-    epi::fold<P, P2, true>(c, sp, s, G);
+    const double inv = epi::rows<P, P2, true>(c, sp, s, blk, is_fsal(pl, sp, call));
+    if (!epi::elect_last(c, G)) return;
+    epi::fold<true>(c, sp, s, G, inv);
     if (threadIdx.x != 0) return;
     c.slots->counter = 0;
     // a stage at t = 0 gathers nothing, so the one after it starts the sums

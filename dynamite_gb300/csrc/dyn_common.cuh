@@ -172,6 +172,42 @@ __device__ __forceinline__ int floor_index_near(const ListView& L, double El, in
     return floor_index(L, El, max(hi - step, 0), hi - 1);
 }
 
+// search_pos out of line: for calls that hardly ever need it
+__device__ __noinline__ inline double search_pos_cold(int mode, const double* p, int n, double vlast, double El) {
+    const ListView L{p, n, vlast};
+    return search_pos(mode, L, El);
+}
+
+// search_pos for an element whose interval is near a guess (0-based lower end; two loads
+// instead of a search where it holds).  Same bits as search_pos: which end of the interval its
+// position starts from depends on the last probe of the search, so the probes are replayed on
+// the known interval, without loads.
+__device__ __forceinline__ double search_pos_near(int mode, const ListView& L, double El, int guess) {
+    const int f = floor_index_near(L, El, min(max(guess, 0), L.n - 1));
+    const double a = L.at(f);
+    const bool eq = okey(a) == okey(El);
+    // an element equal to the first entry, or to several, or before the list
+    if (okey(a) > okey(El) || (eq && (f == 0 || okey(L.at(f - 1)) == okey(a))))
+        return search_pos_cold(mode, L.p, L.n, L.vlast, El);
+    if (f >= L.n - 1) return (double)L.n;
+    double x0 = a, x1 = L.at(f + 1);
+    int m = f + 1;
+    if (mode == 1) {  // pos_lower_bound: first entry >= El
+        if (eq) { m = f; x1 = a; x0 = L.at(f - 1); }
+    } else {
+        int n0 = 1, n1 = L.n;
+        while (n0 <= n1) {
+            m = (n0 + n1) >> 1;
+            if (eq && m - 1 == f) break;
+            if (m - 1 <= f) n0 = m + 1; else n1 = m - 1;
+        }
+    }
+    const bool up = m - 1 > f;  // the last probe was the interval's upper end
+    if (up) { const double x = x0; x0 = x1; x1 = x; }
+    const double v = __ddiv_rn(__dsub_rn(El, x0), __dsub_rn(x1, x0));
+    return up ? __dsub_rn((double)m, v) : __dadd_rn((double)m, v);
+}
+
 // Which of a target's four B2 sums a stage has to form: bits 0..3 for S0, S1
 // (rows X-1, X), D1, D2 (derivative rows X, X+1; D2 only on the cubic branch).
 // key: the row whose sums are held; dirty: the first row rewritten since.

@@ -132,245 +132,337 @@ __device__ __forceinline__ double2 row_value(const DevCtx& c, const StageDev& sp
     }
     return make_double2(qb, ri);
 }
-__device__ __forceinline__ double next_position(const DevCtx& c, const StageDev& sp, int i) {
+__device__ __forceinline__ double next_position(const DevCtx& c, const StageDev& sp, int F, int i) {
     const ListView lv{c.t1grid, sp.nrows_next, sp.T_next};
-    return search_pos(c.search, lv, __dmul_rn(c.theta[i], sp.T_next));
+    return search_pos_near(c.search, lv, __dmul_rn(c.theta[i], sp.T_next), F - 1);
 }
 __device__ __forceinline__ void side_value(const DevCtx& c, const StageDev& sp, const B1Row& r, int i) {
     c.rowval[i] = row_value(c, sp, r);
     if (i == 0) c.slots->q0 = c.KR[(size_t)(sp.nrows - 1) * c.L].x;
 }
-__device__ __forceinline__ void side_position(const DevCtx& c, const StageDev& sp, int i) {
-    if (sp.kind != KIND_RHS && sp.pos_reuse < 0) c.posB1x_next[i] = next_position(c, sp, i);
+__device__ __forceinline__ void side_position(const DevCtx& c, const StageDev& sp, int F, int i) {
+    if (sp.kind != KIND_RHS && sp.pos_reuse < 0) c.posB1x_next[i] = next_position(c, sp, F, i);
 }
 __device__ __forceinline__ void side_row(const DevCtx& c, const StageDev& sp, int i) {
     B1Row r = {};
     if (sp.T > 0.0) r = c.b1[i];
     side_value(c, sp, r, i);
-    side_position(c, sp, i);
+    side_position(c, sp, r.F, i);
 }
 
 namespace epi {
 
-// Rows blk*EPI_ROWS .. +EPI_ROWS of stage s (one row per lane of a one-warp
-// CTA).  Leaves in ep[] the warp sums of the scalars this stage needs:
-// [0..2] r(t) terms, [3..9] dr/dt terms (stage 0), [10] error norm,
-// [12] C(t,0), [13] f'(C(t,0)) (last stage).  fsal: stage 0 of an RK54 step whose right-hand
-// side is the previous step's last one (StageDev::fsal); no gather ran for it.
-template <int P, int P2, bool MIXED>
-__device__ __forceinline__ void rows(const DevCtx& c, const StageDev& sp, const int s, const int blk,
-                                     const bool fsal, double ep[EP_N]) {
-    const int L = c.L, tid = threadIdx.x, i = blk * EPI_ROWS + tid;
-    const DModel Mo = c.M;
-#pragma unroll
-    for (int k = 0; k < EP_N; ++k) ep[k] = 0.0;
+// A warp's FP64 instruction costs 64 cycles here however few lanes or dependences it has (a
+// quarter of the SM's rate: its four schedulers each feed their own unit), and the ~190 of a
+// row were the time of a one-warp CTA (k_epi at L = 64 12.2 us, now 8.4; L = 512 (hi, lo)
+// 14.3, now 10.4).  So EPI_ROWS rows, one per
+// lane, are taken by four warps, each with its share of a row's chain:
+//   warp 0: QK: right-hand side, new value, r(t) terms; warp 1: the part of QK's right-hand
+//   side with theta, dr/dt terms at stage 0; warp 2: QR: right-hand side, new value;
+//   warp 3: the next stage's B1 row.
+constexpr int TAB_STAGES = 10;  // most stages of a tableau method
+enum { EP_R0, EP_R1, EP_R2, EP_DR, EP_ERRX, EP_ERRY, EP_QK0, EP_SK0 };  // per-CTA partials
+struct RowParts { double d1[EPI_ROWS], d2[EPI_ROWS], hy[EPI_ROWS], gy[EPI_ROWS]; };
 
-    if (tid < EPI_ROWS && i < L) {
-        double2 hs;
-        if (fsal) {
-            hs = c.h[(size_t)(RK54_STAGES - 1) * L + i];
-        } else {
-            double a[6];
+// Sum over the chunks of the gather's partial k of row i, in chunk order
+__device__ __forceinline__ double part_sum(const DevCtx& c, int k, int i) {
+    const double* p = c.part + (size_t)k * c.L + i;
+    const size_t st = (size_t)6 * c.L;
+    double a = p[0];
+    for (int ch = 1; ch < c.nch; ch += 4) {
+        double v[4];
 #pragma unroll
-            for (int k = 0; k < 6; ++k) a[k] = 0.0;
-            for (int ch = 0; ch < c.nch; ++ch) {
+        for (int q = 0; q < 4; ++q) v[q] = ch + q < c.nch ? p[(ch + q) * st] : 0.0;
 #pragma unroll
-                for (int k = 0; k < 6; ++k) a[k] += c.part[((size_t)ch * 6 + k) * L + i];
+        for (int q = 0; q < 4; ++q) if (ch + q < c.nch) a += v[q];
+    }
+    return a;
+}
+
+// One component (0 QK, 1 QR) of a row through the stage: begin() takes what the stages before
+// this one left, value() the new value (err: the step's error term, last stage), store() writes it.
+struct Comp {
+    double g, ge, gf, h0;
+    __device__ __forceinline__ void begin(const DevCtx& c, const StageDev& sp, const int s, const int i, const int comp) {
+        const size_t L2 = (size_t)2 * c.L, e = (size_t)2 * i + comp;
+        const double* h = reinterpret_cast<const double*>(c.h) + e;
+        g = ge = (reinterpret_cast<const double*>(c.KR) + e)[(size_t)(sp.n0 - 1) * L2];
+        gf = 0.0;
+        h0 = s > 0 ? h[0] : 0.0;
+        if (sp.kind == KIND_TABLEAU) {
+            const bool last = sp.last;
+            double hv[TAB_STAGES], cf[TAB_STAGES], ce[TAB_STAGES];
+#pragma unroll
+            for (int j = 0; j < TAB_STAGES - 1; ++j) {
+                hv[j] = j < s ? h[j * L2] : 0.0;
+                cf[j] = j < s ? sp.coef[j] : 0.0;
+                ce[j] = j < s && last ? sp.coef_e[j] : 0.0;
             }
-            const double t = sp.T, th = c.theta[i];
-            const double tA = t * th, tR = t * (1.0 - th);
-            const double2 q = c.KR[(size_t)(sp.nrows - 1) * L + i];
-            const double2 rv = c.rowval[i];
-            const double rE = c.rowval[L - 1].y;
-            const double q0 = c.slots->q0;
-            const double fac1 = Sig<P, P2>::d1(Mo, q0) * Mo.iT0, fac2 = q0 * Mo.iT0;
-            // fused as written: every kernel that instantiates this rounds alike
-            const double d1 = fma(a[1], tA, fma(a[0], tR, fma(q.x, -rE, __dmul_rn(rv.x, fac1))));
-            const double d2 = fma(-q.x, rv.y, fma(a[3], tA, fma(a[2], tR,
-                              fma(q.y, 2.0 * Mo.Gamma, __dmul_rn(Sig<P, P2>::d1(Mo, rv.x), fac2)))));
-            hs = make_double2(fma(d2, th, d1), fma(fma(-a[5], tR, __dmul_rn(q.y, rv.y)), th,
-                                                   fma(a[4], tR, __dmul_rn(q.y, -rE))));
+#pragma unroll
+            for (int j = 0; j < TAB_STAGES - 1; ++j) {
+                if (j < s) g = fma(hv[j], cf[j], g);
+                if (j < s && last) ge = fma(hv[j], ce[j], ge);
+            }
+        } else if (sp.serk_mode != 0) {
+            g = (reinterpret_cast<const double*>(c.gS))[e];
+            ge = (reinterpret_cast<const double*>(c.geS))[e];
+            gf = (reinterpret_cast<const double*>(c.gfS))[e];
         }
-        c.h[(size_t)s * L + i] = hs;
-        if (sp.kind == KIND_RHS) {
-            c.rhs_out[i] = hs;
+    }
+    __device__ __forceinline__ double value(const DevCtx& c, const StageDev& sp, const int s, const int i, const int comp,
+                                            const double hs) {
+        if (s == 0) h0 = hs;
+        if (sp.kind == KIND_TABLEAU) {
+            g = fma(hs, sp.coef[s], g);
+            if (!sp.last) return 0.0;
+            ge = fma(hs, sp.coef_e[s], ge);
+            return fabs(g - ge);
+        }
+        if (sp.serk_mode == 0) {
+            gf = ge * sp.serk_b0;
+            g = fma(hs, sp.serk_c, g);
+        } else if (sp.serk_mode == 1) {
+            g = fma(hs, sp.serk_c, g);
         } else {
-            const double2 g0 = c.KR[(size_t)(sp.n0 - 1) * L + i];
-            const double2 h0 = s == 0 ? hs : c.h[i];
-            double2 g;
-            if (sp.kind == KIND_TABLEAU) {
-                g = g0;
-                for (int j = 0; j < sp.ncoef; ++j) {
-                    const double2 hj = j == s ? hs : c.h[(size_t)j * L + i];
-                    g.x = fma(hj.x, sp.coef[j], g.x);
-                    g.y = fma(hj.y, sp.coef[j], g.y);
-                }
-                if (sp.last) {
-                    double2 ge = g0;
-                    for (int j = 0; j < sp.ncoef; ++j) {
-                        const double2 hj = j == s ? hs : c.h[(size_t)j * L + i];
-                        ge.x = fma(hj.x, sp.coef_e[j], ge.x);
-                        ge.y = fma(hj.y, sp.coef_e[j], ge.y);
-                    }
-                    ep[10] = fabs(g.x - ge.x) + fabs(g.y - ge.y);
-                }
+            g = fma(hs, sp.serk_c2, fma(2.0, g, -ge));
+            ge = g;
+        }
+        if (sp.serk_bnext != 0.0) gf = fma(g, sp.serk_bnext, gf);
+        const size_t e = (size_t)2 * i + comp;
+        (reinterpret_cast<double*>(c.gS))[e] = g;
+        (reinterpret_cast<double*>(c.geS))[e] = ge;
+        (reinterpret_cast<double*>(c.gfS))[e] = gf;
+        return sp.last ? fabs(gf - g) : 0.0;
+    }
+    template <bool MIXED>
+    __device__ __forceinline__ void store(const DevCtx& c, const StageDev& sp, const int s, const int i, const int comp,
+                                          const double hs) const {
+        const size_t L2 = (size_t)2 * c.L, e = (size_t)2 * i + comp, o = (size_t)sp.n0 * L2 + e;
+        const double dk = sp.tdiff * h0;
+        (reinterpret_cast<double*>(c.h))[(size_t)s * L2 + e] = hs;
+        (reinterpret_cast<double*>(c.KR))[o] = g;
+        (reinterpret_cast<double*>(c.dKR))[o] = dk;
+        if constexpr (MIXED) {
+            if (c.KRq) {
+                const float2 x = hi_lo(g);
+                float* q = reinterpret_cast<float*>(c.KRq + (size_t)sp.n0 * c.L + i) + comp;
+                q[0] = x.x;
+                q[2] = x.y;
             } else {
-                double2 ge, gf;
-                if (sp.serk_mode == 0) {
-                    g = make_double2(fma(hs.x, sp.serk_c, g0.x), fma(hs.y, sp.serk_c, g0.y));
-                    ge = g0;
-                    gf = make_double2(g0.x * sp.serk_b0, g0.y * sp.serk_b0);
-                } else {
-                    g = c.gS[i]; ge = c.geS[i]; gf = c.gfS[i];
-                    if (sp.serk_mode == 1) {
-                        g.x = fma(hs.x, sp.serk_c, g.x);
-                        g.y = fma(hs.y, sp.serk_c, g.y);
-                    } else {
-                        g.x = fma(hs.x, sp.serk_c2, 2.0 * g.x - ge.x);
-                        g.y = fma(hs.y, sp.serk_c2, 2.0 * g.y - ge.y);
-                        ge = g;
-                    }
-                }
-                if (sp.serk_bnext != 0.0) {
-                    gf.x = fma(g.x, sp.serk_bnext, gf.x);
-                    gf.y = fma(g.y, sp.serk_bnext, gf.y);
-                }
-                c.gS[i] = g; c.geS[i] = ge; c.gfS[i] = gf;
-                if (sp.last) ep[10] = fabs(gf.x - g.x) + fabs(gf.y - g.y);
+                (reinterpret_cast<float*>(c.KRf))[o] = (float)g;
             }
-            const double w = c.integ[i];
-            if (s == 0) {
-                // drstep2 (time_steps.cu:564-639) on the step's base row and h0
-                double sk, dd;
-                Sig<P, P2>::d12(Mo, g0.x, sk, dd);
-                const double sr = dd * g0.y;
-                const double dsk = dd * h0.x;
-                const double dsr = fma(dd, h0.y, __dmul_rn(Sig<P, P2>::d3(Mo, g0.x) * g0.y, h0.x));
-                const double tw = sp.T * w;
-                ep[3] = __dmul_rn(w * sr, g0.x);
-                ep[4] = __dmul_rn(w * sk, g0.y);
-                ep[5] = __dmul_rn(tw * dsr, g0.x);
-                ep[6] = __dmul_rn(tw * dsk, g0.y);
-                ep[7] = __dmul_rn(tw * sr, h0.x);
-                ep[8] = __dmul_rn(tw * sk, h0.y);
-                if (i == 0) ep[9] = __dmul_rn(fma(sk, h0.x, __dmul_rn(dsk, g0.x)), Mo.iT0);
-            }
-            const double td = sp.tdiff;
-            c.KR[(size_t)sp.n0 * L + i] = g;
-            c.dKR[(size_t)sp.n0 * L + i] = make_double2(td * h0.x, td * h0.y);
-            if constexpr (MIXED) {
-                const float2 gx = hi_lo(g.x), gy = hi_lo(g.y);
-                if (c.KRq) c.KRq[(size_t)sp.n0 * L + i] = make_float4(gx.x, gy.x, gx.y, gy.y);
-                else c.KRf[(size_t)sp.n0 * L + i] = make_float2(gx.x, gy.x);
-                c.dKRf[(size_t)sp.n0 * L + i] = make_float2((float)(td * h0.x), (float)(td * h0.y));
-            }
-            // rstep (time_steps.cpp:83-92) of the new row at its time
-            const double tn = sp.T_next, tw = tn * w;
-            double sk, dd;
-            Sig<P, P2>::d12(Mo, g.x, sk, dd);
-            ep[0] = __dmul_rn(tw * (dd * g.y), g.x);
-            ep[1] = __dmul_rn(tw * sk, g.y);
-            if (i == 0) {
-                ep[2] = __dmul_rn(sk * g.x, Mo.iT0);
-                ep[12] = g.x;
-                ep[13] = sk;
-            }
-            // positions of the next stage (searched by the gather kernel)
-            const double pos = sp.pos_reuse >= 0 ? c.posB1x_saved[(size_t)sp.pos_reuse * L + i]
-                               : fsal            ? next_position(c, sp, i)  // no gather ran
-                                                 : c.posB1x_next[i];
-            c.posB1x[i] = pos;
-            // the next stage's B1 row; delta_t_ratio of the row being written is not in memory yet
-            c.b1[i] = b1_at(pos, sp.nrows_next - 1 < 1 ? 1 : sp.nrows_next - 1, sp.nrows_next, [&](int k) {
-                return k != sp.n0 ? c.inv_dtr[k] : sp.dtr_new != 0.0 ? 1.0 / sp.dtr_new : 0.0;
-            });
-            if (sp.pos_save >= 0) c.posB1x_saved[(size_t)sp.pos_save * L + i] = pos;
+            (reinterpret_cast<float*>(c.dKRf))[o] = (float)dk;
         }
     }
-    // one warp per CTA: fixed butterfly sums of the quantities this stage uses
-    // (r(t) always; dr/dt at stage 0; error norm and C(t,0), f'(C(t,0)) at the last)
-    if (sp.kind != KIND_RHS) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) ep[k] = warp_sum(ep[k]);
-        if (s == 0) {
-#pragma unroll
-            for (int k = 3; k < 10; ++k) ep[k] = warp_sum(ep[k]);
-        }
-        if (sp.last) {
-            ep[10] = warp_sum(ep[10]);
-            ep[12] = warp_sum(ep[12]);
-            ep[13] = warp_sum(ep[13]);
-        }
-    }
-}
+};
 
-// Publish this CTA's partials (CTA blk of G) and elect the CTA that finishes
-// last (atomic ticket on slots->counter, no waiting); true in every thread
-// of that CTA only.
-__device__ __forceinline__ bool elect_last(const DevCtx& c, const double ep[EP_N], const unsigned blk, const unsigned G) {
-    __shared__ int s_is_last;
-    const int tid = threadIdx.x;
-    if (tid < EP_N) {
-        double v = 0.0;
-#pragma unroll
-        for (int k = 0; k < EP_N; ++k) if (k == tid) v = ep[k];
-        c.epart[(size_t)blk * EP_N + tid] = v;
-    }
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) s_is_last = atomicAdd(&c.slots->counter, 1u) == G - 1;
-    __syncthreads();
-    const bool last = s_is_last;
-    if (last) __threadfence();
-    return last;
-}
-
-// Fold of the G CTAs' partials (in CTA order) and the stage's scalar writes
-// (thread 0): r of the written row, dr/dt, t1grid, delta_t_ratio and, at the
-// last stage, the step result.  Does not reset slots->counter.
+// Rows blk*EPI_ROWS .. +EPI_ROWS of stage s.  Leaves this CTA's partials of the scalars this
+// stage needs in c.epart: r(t) terms, dr/dt (stage 0), error norm, C(t,0), f'(C(t,0)) (last
+// stage).  fsal: stage 0 of an RK54 step whose right-hand side is the previous step's last one
+// (StageDev::fsal); no gather ran for it.  Returns the inverse that the fold of this thread's
+// warp writes: of tdiff (warp 2), of delta_t_ratio (warp 3; 0 where that is 0).
 template <int P, int P2, bool MIXED>
-__device__ __forceinline__ void fold(const DevCtx& c, const StageDev& sp, const int s, const unsigned G) {
-    const int tid = threadIdx.x;
+__device__ __forceinline__ double rows(const DevCtx& c, const StageDev& sp, const int s, const unsigned blk, const bool fsal) {
+    __shared__ RowParts sh;
+    const int L = c.L, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = (int)blk * EPI_ROWS + lane;
+    const bool mine = i < L, step = sp.kind != KIND_RHS;
     const DModel Mo = c.M;
-    double tot = 0.0;
-    if (tid < EP_N) {
-        for (unsigned b = 0; b < G; b += 4) {
-            // four independent loads in flight, summed in block order
-            double v[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) v[q] = b + q < G ? __ldcg(c.epart + (size_t)(b + q) * EP_N + tid) : 0.0;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) tot += v[q];
+    const double t = sp.T;
+    double inv = 0.0, d = 0.0, th = 0.0, w = 0.0, err = 0.0;
+    Comp k = {};
+    // stage 0, warp 1: dr/dt terms of the step's base row (drstep2, time_steps.cu:564-639)
+    double2 g0 = {};
+    double sk0 = 0.0, dd0 = 0.0, sr0 = 0.0, d3g = 0.0, dr = 0.0;
+
+    if (warp == 3) {
+        if (step) {
+            const double dtr_new = sp.dtr_new;
+            const int nrows_next = sp.nrows_next, n0 = sp.n0;
+            inv = dtr_new != 0.0 ? 1.0 / dtr_new : 0.0;
+            if (mine) {
+                const double pos = sp.pos_reuse >= 0 ? c.posB1x_saved[(size_t)sp.pos_reuse * L + i]
+                                   : fsal            ? next_position(c, sp, c.b1[i].F, i)  // no gather ran
+                                                     : c.posB1x_next[i];
+                c.posB1x[i] = pos;
+                if (sp.pos_save >= 0) c.posB1x_saved[(size_t)sp.pos_save * L + i] = pos;
+                // delta_t_ratio of the row being written is not in memory yet
+                c.b1[i] = b1_at(pos, nrows_next - 1 < 1 ? 1 : nrows_next - 1, nrows_next,
+                                [&](int k) { return k != n0 ? c.inv_dtr[k] : inv; });
+            }
+        }
+    } else if (mine) {
+        th = c.theta[i];
+        if (step && warp != 1) k.begin(c, sp, s, i, warp >> 1);
+        if (step && warp != 2) w = c.integ[i];
+        // right-hand side; fused as written: every kernel that instantiates this rounds alike
+        if (fsal) {
+            const double2 hs = c.h[(size_t)(RK54_STAGES - 1) * L + i];
+            d = warp == 2 ? hs.y : hs.x;
+        } else {
+            const double2 q = c.KR[(size_t)(sp.nrows - 1) * L + i], rv = c.rowval[i];
+            const double rE = c.rowval[L - 1].y, q0 = c.slots->q0;
+            const double aA = part_sum(c, 2 * warp + 1, i), aR = part_sum(c, 2 * warp, i);
+            const double tA = t * th, tR = t * (1.0 - th);
+            if (warp == 0) {
+                const double fac1 = Sig<P, P2>::d1(Mo, q0) * Mo.iT0;
+                d = fma(aA, tA, fma(aR, tR, fma(q.x, -rE, __dmul_rn(rv.x, fac1))));
+            } else if (warp == 1) {
+                const double fac2 = q0 * Mo.iT0;
+                d = fma(-q.x, rv.y, fma(aA, tA, fma(aR, tR,
+                    fma(q.y, 2.0 * Mo.Gamma, __dmul_rn(Sig<P, P2>::d1(Mo, rv.x), fac2)))));
+            } else {
+                d = fma(fma(-aA, tR, __dmul_rn(q.y, rv.y)), th, fma(aR, tR, __dmul_rn(q.y, -rE)));
+            }
+        }
+        if (warp == 0) sh.d1[lane] = d;
+        if (warp == 1) {
+            sh.d2[lane] = d;
+            if (step && s == 0) {
+                g0 = c.KR[(size_t)(sp.n0 - 1) * L + i];
+                Sig<P, P2>::d12(Mo, g0.x, sk0, dd0);
+                d3g = Sig<P, P2>::d3(Mo, g0.x) * g0.y;
+                sr0 = dd0 * g0.y;
+                dr = fma(w * sk0, g0.y, __dmul_rn(w * sr0, g0.x));
+            }
+        }
+        if (warp == 2) {
+            sh.hy[lane] = d;
+            if (step) {
+                err = k.value(c, sp, s, i, 1, d);
+                sh.gy[lane] = k.g;
+                inv = 1.0 / sp.tdiff;
+            }
         }
     }
-    __shared__ double s_tot[EP_N];
-    if (tid < EP_N) s_tot[tid] = tot;
+    __syncthreads();  // and every read of the newest row is done
+    double* ep = c.epart + (size_t)blk * EP_N;
+    if (warp == 0) {
+        double r0 = 0.0, r1 = 0.0, r2 = 0.0, sk = 0.0;
+        if (mine) {
+            const double hs = fsal ? d : fma(sh.d2[lane], th, d);
+            if (step) {
+                err = k.value(c, sp, s, i, 0, hs);
+                k.store<MIXED>(c, sp, s, i, 0, hs);
+                // rstep (time_steps.cpp:83-92) of the new row at its time
+                const double tw = sp.T_next * w, gy = sh.gy[lane];
+                double dd;
+                Sig<P, P2>::d12(Mo, k.g, sk, dd);
+                r0 = __dmul_rn(tw * (dd * gy), k.g);
+                r1 = __dmul_rn(tw * sk, gy);
+                if (i == 0) r2 = __dmul_rn(sk * k.g, Mo.iT0);
+            } else {
+                c.h[(size_t)s * L + i].x = hs;
+                c.rhs_out[i].x = hs;
+            }
+        }
+        if (step) {
+            // both sums in five adds a lane: the lower half-warp carries r0, the upper r1
+            const double mv = lane < 16 ? r0 : r1, ot = lane < 16 ? r1 : r0;
+            double v = mv + __shfl_xor_sync(0xffffffffu, ot, 16);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (sp.last) err = warp_sum(err);
+            if (lane == 0) {
+                ep[EP_R0] = v;
+                ep[EP_R2] = r2;
+                if (sp.last) {
+                    ep[EP_ERRX] = err;
+                    ep[EP_QK0] = blk == 0 ? k.g : 0.0;
+                    ep[EP_SK0] = blk == 0 ? sk : 0.0;
+                }
+            }
+            if (lane == 16) ep[EP_R1] = v;
+        }
+    } else if (warp == 1) {
+        if (step && s == 0) {
+            if (mine) {
+                const double hx = fsal ? d : fma(d, th, sh.d1[lane]), hy = sh.hy[lane];
+                const double dsk = dd0 * hx, dsr = fma(dd0, hy, __dmul_rn(d3g, hx)), tw = t * w;
+                dr = fma(tw * dsr, g0.x, dr);
+                dr = fma(tw * dsk, g0.y, dr);
+                dr = fma(tw * sr0, hx, dr);
+                dr = fma(tw * sk0, hy, dr);
+                if (i == 0) dr = fma(fma(sk0, hx, __dmul_rn(dsk, g0.x)), Mo.iT0, dr);
+            }
+            dr = warp_sum(dr);
+            if (lane == 0) ep[EP_DR] = dr;
+        }
+    } else if (warp == 2) {
+        if (mine) {
+            if (step) {
+                k.store<MIXED>(c, sp, s, i, 1, d);
+            } else {
+                c.h[(size_t)s * L + i].y = d;
+                c.rhs_out[i].y = d;
+            }
+        }
+        if (step && sp.last) {
+            err = warp_sum(err);
+            if (lane == 0) ep[EP_ERRY] = err;
+        }
+    }
+    return inv;
+}
+
+// Elect the CTA of G that finishes last (atomic ticket on slots->counter, no waiting);
+// true in every thread of that CTA only.
+__device__ __forceinline__ bool elect_last(const DevCtx& c, const unsigned G) {
+    __shared__ unsigned s_ticket;
+    // releases this CTA's rows and partials, acquires the others': the barriers carry the
+    // order to and from the ticket's thread
     __syncthreads();
-    if (tid != 0) return;
+    if (threadIdx.x == 0)
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(s_ticket) : "l"(&c.slots->counter) : "memory");
+    __syncthreads();
+    return s_ticket == G - 1;
+}
+
+// Fold of the G CTAs' partials (in a fixed order) and the stage's scalar writes: r of the
+// written row, dr/dt, t1grid, delta_t_ratio and, at the last stage, the step result.  Ends
+// with a barrier; does not reset slots->counter.
+template <bool MIXED>
+__device__ __forceinline__ void fold(const DevCtx& c, const StageDev& sp, const int s, const unsigned G, const double inv) {
+    static_assert(EP_N == 8 && EPI_T == 128);
+    __shared__ double s_tot[EPI_T / 32][EP_N];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     Slots* sl = c.slots;
     if (sp.kind != KIND_RHS) {
+        const double dr_old = s == 0 ? 0.0 : sl->dr;
+        double v = 0.0;
+        for (unsigned b = tid / EP_N; b < G; b += EPI_T / EP_N) v += __ldcg(c.epart + (size_t)b * EP_N + tid % EP_N);
+        v += __shfl_xor_sync(0xffffffffu, v, 8);
+        v += __shfl_xor_sync(0xffffffffu, v, 16);
+        if (lane < EP_N) s_tot[warp][lane] = v;
+        __syncthreads();
+        const auto tot = [&](int q) { return (s_tot[0][q] + s_tot[1][q]) + (s_tot[2][q] + s_tot[3][q]); };
         const int n0 = sp.n0;
-        const double r_new = ((Mo.Gamma + s_tot[0]) + s_tot[1]) + s_tot[2];
-        c.rvec[n0] = r_new;
-        if (s == 0)
-            sl->dr = (((((s_tot[3] + s_tot[4]) + s_tot[5]) + s_tot[6]) + s_tot[7]) + s_tot[8]) + s_tot[9];
-        c.drvec[n0] = sp.tdiff * sl->dr;
-        c.t1grid[n0] = sp.T_next;
-        c.dtr[n0] = sp.dtr_new;
-        c.inv_dtr[n0] = sp.dtr_new != 0.0 ? 1.0 / sp.dtr_new : 0.0;
-        if (c.inv_len) c.inv_len[n0 - 1] = 1.0 / sp.tdiff;
-        if constexpr (MIXED) {
-            c.inv_dtr_f[n0] = hi_lo(sp.dtr_new != 0.0 ? 1.0 / sp.dtr_new : 0.0);
-            c.inv_len_f[n0 - 1] = hi_lo(1.0 / sp.tdiff);
-        }
-        if (sp.last) {
-            sl->res_err = s_tot[10];
-            sl->res_energy = -(s_tot[1] + __dmul_rn(s_tot[13], Mo.iT0));
-            sl->res_r = r_new;
-            sl->res_qk0 = s_tot[12];
-            sl->res_dr = sl->dr;
+        if (tid == 0) {
+            const double r1 = tot(EP_R1), r_new = ((c.M.Gamma + tot(EP_R0)) + r1) + tot(EP_R2);
+            c.rvec[n0] = r_new;
+            if (sp.last) {
+                sl->res_energy = -(r1 + __dmul_rn(tot(EP_SK0), c.M.iT0));
+                sl->res_r = r_new;
+            }
+        } else if (tid == 32) {
+            const double dr = s == 0 ? tot(EP_DR) : dr_old;
+            if (s == 0) sl->dr = dr;
+            c.drvec[n0] = sp.tdiff * dr;
+            if (sp.last) sl->res_dr = dr;
+        } else if (tid == 64) {
+            if (c.inv_len) c.inv_len[n0 - 1] = inv;
+            if constexpr (MIXED) c.inv_len_f[n0 - 1] = hi_lo(inv);
+            if (sp.last) {
+                sl->res_err = tot(EP_ERRX) + tot(EP_ERRY);
+                sl->res_qk0 = tot(EP_QK0);
+            }
+        } else if (tid == 96) {
+            c.t1grid[n0] = sp.T_next;
+            c.dtr[n0] = sp.dtr_new;
+            c.inv_dtr[n0] = inv;
+            if constexpr (MIXED) c.inv_dtr_f[n0] = hi_lo(inv);
         }
     }
+    __syncthreads();
 }
 
 }  // namespace epi

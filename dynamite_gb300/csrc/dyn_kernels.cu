@@ -327,10 +327,9 @@ template <int P, int P2, bool MIXED>
 __global__ void __launch_bounds__(EPI_T) k_epi(const DevCtx c, const int s) {
     wait_prior_grid();
     const StageDev& sp = c.stages[s];
-    double ep[EP_N];
-    epi::rows<P, P2, MIXED>(c, sp, s, blockIdx.x, s == 0 && sp.fsal, ep);
-    if (!epi::elect_last(c, ep, blockIdx.x, gridDim.x)) return;
-    epi::fold<P, P2, MIXED>(c, sp, s, gridDim.x);
+    const double inv = epi::rows<P, P2, MIXED>(c, sp, s, blockIdx.x, s == 0 && sp.fsal);
+    if (!epi::elect_last(c, gridDim.x)) return;
+    epi::fold<MIXED>(c, sp, s, gridDim.x, inv);
     if (threadIdx.x == 0) c.slots->counter = 0;
 }
 

@@ -10,10 +10,9 @@ namespace dyn {
 constexpr int SMAX = 32;      // most stages of one step (SERK2 with q <= 16)
 constexpr int RK54_STAGES = 7;
 constexpr int NSAVE = 3;      // SSPRK(10,4) keeps positions of stages 2..4
-constexpr int EPI_T = 32;     // threads per epilogue CTA (one warp)
-constexpr int EPI_ROWS = 32;  // rows per epilogue CTA (one row per lane; spreading rows over
-                              // more SMs did not shorten its FP64 dependency chain)
-constexpr int EP_N = 16;      // per-CTA epilogue partials
+constexpr int EPI_T = 128;    // threads per epilogue CTA: four warps
+constexpr int EPI_ROWS = 32;  // rows per epilogue CTA, one per lane (the warps share a row's work)
+constexpr int EP_N = 8;       // per-CTA epilogue partials
 
 enum StageKind { KIND_TABLEAU = 0, KIND_SERK = 1, KIND_RHS = 2 };
 

@@ -319,7 +319,7 @@ __device__ __forceinline__ void row_setup(const DevCtx& c, const StageDev& sp, c
         sh.bi[0] = r.F; sh.bi[1] = r.cubic;
         sh.c[0] = (float)r.c0; sh.c[1] = (float)r.c1; sh.c[2] = (float)r.c2; sh.c[3] = (float)r.c3;
     }
-    if (BATCH && threadIdx.x == 32) side_position(c, sp, i);
+    if (BATCH && threadIdx.x == 32) side_position(c, sp, sp.fresh ? sp.nrows : c.b1[i].F, i);
     if (brackets) row_brackets(c, sp, i, sh);
 }
 
@@ -814,7 +814,7 @@ __device__ __forceinline__ void row_setup(const DevCtx& c, const StageDev& sp, c
         sh.bi[0] = r.F; sh.bi[1] = r.cubic;
         rc.b1[0] = quad(r.c0); rc.b1[1] = quad(r.c1); rc.b1[2] = quad(-r.c2); rc.b1[3] = quad(-r.c3);
     }
-    if (BATCH && threadIdx.x == 32) side_position(c, sp, i);
+    if (BATCH && threadIdx.x == 32) side_position(c, sp, sp.fresh ? sp.nrows : c.b1[i].F, i);
     if (brackets) row_brackets(c, sp, i, sh);
 }
 
