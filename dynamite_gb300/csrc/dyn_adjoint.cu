@@ -8,12 +8,13 @@
 // row-n0 state and the B1 positions each stage reads), then runs the stages
 // backwards:
 //
-//   k_adj_rowwrite   row n0 after stage s: r = rstep(G_s) (time_steps.cpp:83-92),
+//   k_adj_enter      takes row n0's cotangents over and puts the row back into
+//                    stage s's input state;
+//   k_adj_rows       row n0 after stage s: r = rstep(G_s) (time_steps.cpp:83-92),
 //                    dQK/dQR = tdiff_s h_0, dr = tdiff_s DR and the RK
-//                    combination G_s = g0 + sum_j coef_j h_j, transposed;
-//   k_adj_drstep     DR = drstep2(g0, h_0) (time_steps.cpp:117-125), transposed;
-//   k_adj_restore    puts row n0 back into stage s's input state;
-//   k_adj_epi        the RHS epilogue (QKstep/QRstep, time_steps.cpp:27-47,
+//                    combination G_s = g0 + sum_j coef_j h_j, transposed; at
+//                    stage 0 DR = drstep2(g0, h_0) (time_steps.cpp:117-125);
+//                    then the RHS epilogue (QKstep/QRstep, time_steps.cpp:27-47,
 //                    94-100) transposed: row cotangents of the eight memory
 //                    integrals, the direct last-row terms, QK^{B1}[i,0] and
 //                    rInt (index_vec.cpp:63-156) scattered to the history;
@@ -24,6 +25,7 @@
 //                    a per-row partial, reduced by k_adj_lastreduce).
 //
 // Parameter derivatives (Gamma, lambda) accumulate in device scalars.
+#include <algorithm>
 #include <cmath>
 #include "dyn_epi.cuh"
 
@@ -67,10 +69,10 @@ __device__ __forceinline__ void fder_t(const AdjModel& m, double q, double& v, d
         fder(m, K, q, v, vl);
     } else {
         constexpr double ap = alpha_c<P, K>(), ap2 = alpha_c<P2, K>();
-        const double tp = (P - K >= 0 && ap != 0.0) ? ap * ipow_c<(P - K >= 0 ? P - K : 0)>(q) : 0.0;
-        const double tp2 = (P2 - K >= 0 && ap2 != 0.0) ? ap2 * ipow_c<(P2 - K >= 0 ? P2 - K : 0)>(q) : 0.0;
-        v = m.lam * tp + (1.0 - m.lam) * tp2;
-        vl = tp - tp2;
+        const double tp = (P - K >= 0 && ap != 0.0) ? ipow_c<(P - K >= 0 ? P - K : 0)>(q) : 0.0;
+        const double tp2 = (P2 - K >= 0 && ap2 != 0.0) ? ipow_c<(P2 - K >= 0 ? P2 - K : 0)>(q) : 0.0;
+        v = fma(m.cb[K], tp2, m.ca[K] * tp);
+        vl = fma(ap, tp, -(ap2 * tp2));
     }
 }
 
@@ -128,168 +130,148 @@ __global__ void __launch_bounds__(256) k_adj_seed(const DevCtx c, const AdjDev a
     }
 }
 
-// cotangents of row n0 (state after the last stage) into the stage buffers
-__global__ void k_adj_move(const DevCtx c, const AdjDev a, const int n0) {
-    const int L = c.L;
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < L; j += gridDim.x * blockDim.x) {
-        a.Gbar[j] = a.HKR[(size_t)n0 * L + j];
-        a.Dbar[j] = a.HdKR[(size_t)n0 * L + j];
-        a.HKR[(size_t)n0 * L + j] = make_double2(0.0, 0.0);
-        a.HdKR[(size_t)n0 * L + j] = make_double2(0.0, 0.0);
+// row n0 as stage k left it, and the B1 rows the next stage reads
+__global__ void k_adj_save(const DevCtx c, const AdjDev a, const int k, const int n0) {
+    wait_prior_grid();
+    const int L = c.L, j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < L) {
+        a.Gsave[(size_t)k * L + j] = c.KR[(size_t)n0 * L + j];
+        a.Dsave[(size_t)k * L + j] = c.dKR[(size_t)n0 * L + j];
+        if (k + 1 < SMAX) a.Bsave[(size_t)(k + 1) * L + j] = c.b1[j];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (j < 5) a.tsave[5 * k + j] = (j == 0 ? c.rvec : j == 1 ? c.drvec : j == 2 ? c.t1grid : j == 3 ? c.dtr : c.inv_dtr)[n0];
+}
+
+// Before the reverse of stage s: the cotangents of row n0 (the state after stage s) into the
+// stage buffers, and row n0 back into stage s's input state (the state after stage s-1)
+__global__ void k_adj_enter(const DevCtx c, const AdjDev a, const int s, const int n0) {
+    wait_prior_grid();
+    const int L = c.L, j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < L) {
+        const size_t o = (size_t)n0 * L + j;
+        a.Gbar[j] = a.HKR[o];
+        a.Dbar[j] = a.HdKR[o];
+        a.HKR[o] = make_double2(0.0, 0.0);
+        a.HdKR[o] = make_double2(0.0, 0.0);
+        if (s >= 1) {
+            c.KR[o] = a.Gsave[(size_t)(s - 1) * L + j];
+            c.dKR[o] = a.Dsave[(size_t)(s - 1) * L + j];
+        }
+    }
+    if (j == 0) {
         a.sc[SC_RHO] = a.Hr[n0];
         a.sc[SC_DELTA] = a.Hdr[n0];
         a.Hr[n0] = 0.0;
         a.Hdr[n0] = 0.0;
     }
+    if (s >= 1 && j < 5)
+        (j == 0 ? c.rvec : j == 1 ? c.drvec : j == 2 ? c.t1grid : j == 3 ? c.dtr : c.inv_dtr)[n0] = a.tsave[5 * (s - 1) + j];
 }
+
+// What column j's thread accumulates of the row's scalars
+struct RowBars { double2 g0b, h0b; double lam; };
 
 // ------------------------------------------------- row write of stage s
 template <int P, int P2>
-__global__ void __launch_bounds__(256) k_adj_rowwrite(const DevCtx c, const AdjDev a, const AdjModel am, const int s) {
-    const StageDev& sp = c.stages[s];
+__device__ __forceinline__ RowBars row_write(const DevCtx& c, const AdjDev& a, const AdjModel& am, const StageDev& sp,
+                                             const int s, const int j) {
     const int L = c.L;
-    const double tn = sp.T_next, td = sp.tdiff;
-    const double rb = a.sc[SC_RHO], db = a.sc[SC_DELTA];
-    double lam = 0.0;
-    for (int j = threadIdx.x; j < L; j += blockDim.x) {
-        const double2 G = a.Gsave[(size_t)s * L + j];
-        const double w = c.integ[j];
-        double f1, f1l, f2, f2l, f3, f3l;
-        fder_t<P, P2, 1>(am, G.x, f1, f1l);
-        fder_t<P, P2, 2>(am, G.x, f2, f2l);
-        fder_t<P, P2, 3>(am, G.x, f3, f3l);
-        // r = Gamma + sum_j tn w (f''(K) R K + f'(K) R) + f'(K_0) K_0 / T0
-        double dK = tn * w * (f3 * G.y * G.x + 2.0 * f2 * G.y);
-        const double dR = tn * w * (f2 * G.x + f1);
-        lam += tn * w * (f2l * G.y * G.x + f1l * G.y);
-        if (j == 0) {
-            dK += (f2 * G.x + f1) / am.T0;
-            lam += f1l * G.x / am.T0;
-        }
-        const double2 gb0 = a.Gbar[j];
-        const double2 Gb = make_double2(gb0.x + rb * dK, gb0.y + rb * dR);
-        // G_s = g0 + sum_{j<=s} coef_j h_j
-        double2 g0b = a.g0bar[j];
-        g0b.x += Gb.x;
-        g0b.y += Gb.y;
-        a.g0bar[j] = g0b;
-        for (int q = 0; q < sp.ncoef; ++q) {
-            double2 hb = a.hbar[(size_t)q * L + j];
-            hb.x += sp.coef[q] * Gb.x;
-            hb.y += sp.coef[q] * Gb.y;
-            a.hbar[(size_t)q * L + j] = hb;
-        }
-        // dQK, dQR of row n0 = tdiff_s h_0
-        const double2 Db = a.Dbar[j];
-        double2 h0b = a.hbar[j];
-        h0b.x += td * Db.x;
-        h0b.y += td * Db.y;
-        a.hbar[j] = h0b;
+    const double tn = sp.T_next, rb = a.sc[SC_RHO];
+    const double2 G = a.Gsave[(size_t)s * L + j];
+    const double w = tn * c.integ[j];
+    double f1, f1l, f2, f2l;
+    fder_t<P, P2, 1>(am, G.x, f1, f1l);
+    fder_t<P, P2, 2>(am, G.x, f2, f2l);
+    const double f3 = fd_t<P, P2, 3>(am, G.x);
+    // r = Gamma + sum_j tn w (f''(K) R K + f'(K) R) + f'(K_0) K_0 / T0
+    double dK = w * (f3 * G.y * G.x + 2.0 * f2 * G.y);
+    const double dR = w * (f2 * G.x + f1);
+    RowBars r;
+    r.lam = w * (f2l * G.y * G.x + f1l * G.y);
+    if (j == 0) {
+        dK += (f2 * G.x + f1) / am.T0;
+        r.lam += f1l * G.x / am.T0;
     }
-    lam = block_sum(lam);
-    if (threadIdx.x == 0) {
-        a.sc[SC_LAMBDA] += rb * lam;
-        a.sc[SC_GAMMA] += rb;
-        a.sc[SC_DR] += td * db;  // dr of row n0 = tdiff_s DR
+    r.lam *= rb;
+    const double2 gb0 = a.Gbar[j];
+    const double2 Gb = make_double2(gb0.x + rb * dK, gb0.y + rb * dR);
+    // G_s = g0 + sum_{j<=s} coef_j h_j
+    r.g0b = a.g0bar[j];
+    r.g0b.x += Gb.x;
+    r.g0b.y += Gb.y;
+    for (int q = 1; q < sp.ncoef; ++q) {
+        double2 hb = a.hbar[(size_t)q * L + j];
+        hb.x += sp.coef[q] * Gb.x;
+        hb.y += sp.coef[q] * Gb.y;
+        a.hbar[(size_t)q * L + j] = hb;
     }
+    // dQK, dQR of row n0 = tdiff_s h_0
+    const double2 Db = a.Dbar[j];
+    r.h0b = a.hbar[j];
+    r.h0b.x += sp.coef[0] * Gb.x + sp.tdiff * Db.x;
+    r.h0b.y += sp.coef[0] * Gb.y + sp.tdiff * Db.y;
+    return r;
 }
 
 // DR = drstep2(g0, h_0) at the step start (stage 0 time)
 template <int P, int P2>
-__global__ void __launch_bounds__(256) k_adj_drstep(const DevCtx c, const AdjDev a, const AdjModel am, const int n0) {
-    const int L = c.L;
-    const double T = c.stages[0].T, DRb = a.sc[SC_DR];
-    double lam = 0.0;
-    for (int j = threadIdx.x; j < L; j += blockDim.x) {
-        const double2 g = c.KR[(size_t)(n0 - 1) * L + j];
-        const double2 h = c.h[j];
-        const double w = c.integ[j], tw = T * w;
-        const double K = g.x, R = g.y, hK = h.x, hR = h.y;
-        double f1, f1l, f2, f2l, f3, f3l, f4, f4l;
-        fder_t<P, P2, 1>(am, K, f1, f1l);
-        fder_t<P, P2, 2>(am, K, f2, f2l);
-        fder_t<P, P2, 3>(am, K, f3, f3l);
-        fder_t<P, P2, 4>(am, K, f4, f4l);
-        double dK = w * (f3 * R * K + 2.0 * f2 * R) + tw * (f4 * R * hK * K + 3.0 * f3 * R * hK + f3 * hR * K + 2.0 * f2 * hR);
-        const double dR = w * (f2 * K + f1) + tw * (f3 * hK * K + 2.0 * f2 * hK);
-        double dhK = tw * (f3 * R * K + 2.0 * f2 * R);
-        const double dhR = tw * (f2 * K + f1);
-        double dl = w * (f2l * R * K + f1l * R) + tw * (f3l * R * hK * K + f2l * hR * K + 2.0 * f2l * hK * R + f1l * hR);
-        if (j == 0) {
-            dK += (f3 * K + 2.0 * f2) * hK / am.T0;
-            dhK += (f2 * K + f1) / am.T0;
-            dl += (f2l * K + f1l) * hK / am.T0;
-        }
-        double2 gb = a.g0bar[j];
-        gb.x += DRb * dK;
-        gb.y += DRb * dR;
-        a.g0bar[j] = gb;
-        double2 hb = a.hbar[j];
-        hb.x += DRb * dhK;
-        hb.y += DRb * dhR;
-        a.hbar[j] = hb;
-        lam += dl;
+__device__ __forceinline__ void row_drstep(const DevCtx& c, const AdjModel& am, const int n0, const int j, const double T,
+                                           const double DRb, RowBars& r) {
+    const double2 g = c.KR[(size_t)(n0 - 1) * c.L + j];
+    const double2 h = c.h[j];
+    const double w = c.integ[j], tw = T * w;
+    const double K = g.x, R = g.y, hK = h.x, hR = h.y;
+    double f1, f1l, f2, f2l, f3, f3l;
+    fder_t<P, P2, 1>(am, K, f1, f1l);
+    fder_t<P, P2, 2>(am, K, f2, f2l);
+    fder_t<P, P2, 3>(am, K, f3, f3l);
+    const double f4 = fd_t<P, P2, 4>(am, K);
+    double dK = w * (f3 * R * K + 2.0 * f2 * R) + tw * (f4 * R * hK * K + 3.0 * f3 * R * hK + f3 * hR * K + 2.0 * f2 * hR);
+    const double dR = w * (f2 * K + f1) + tw * (f3 * hK * K + 2.0 * f2 * hK);
+    double dhK = tw * (f3 * R * K + 2.0 * f2 * R);
+    const double dhR = tw * (f2 * K + f1);
+    double dl = w * (f2l * R * K + f1l * R) + tw * (f3l * R * hK * K + f2l * hR * K + 2.0 * f2l * hK * R + f1l * hR);
+    if (j == 0) {
+        dK += (f3 * K + 2.0 * f2) * hK / am.T0;
+        dhK += (f2 * K + f1) / am.T0;
+        dl += (f2l * K + f1l) * hK / am.T0;
     }
-    lam = block_sum(lam);
-    if (threadIdx.x == 0) a.sc[SC_LAMBDA] += DRb * lam;
+    r.g0b.x += DRb * dK;
+    r.g0b.y += DRb * dR;
+    r.h0b.x += DRb * dhK;
+    r.h0b.y += DRb * dhR;
+    r.lam += DRb * dl;
 }
 
-// row n0 back into stage s's input state (the state after stage s-1) and the
-// B1 positions stage s read
-__global__ void k_adj_restore(const DevCtx c, const AdjDev a, const int s, const int n0) {
-    const int L = c.L;
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < L; j += gridDim.x * blockDim.x) {
-        c.posB1x[j] = a.Psave[(size_t)s * L + j];
-        if (s >= 1) {
-            c.KR[(size_t)n0 * L + j] = a.Gsave[(size_t)(s - 1) * L + j];
-            c.dKR[(size_t)n0 * L + j] = a.Dsave[(size_t)(s - 1) * L + j];
-        }
-    }
-    if (s >= 1 && blockIdx.x == 0 && threadIdx.x == 0) {
-        const StageDev& pv = c.stages[s - 1];
-        c.rvec[n0] = a.rsave[s - 1];
-        c.drvec[n0] = a.drsave[s - 1];
-        c.t1grid[n0] = pv.T_next;
-        c.dtr[n0] = pv.dtr_new;
-        c.inv_dtr[n0] = pv.dtr_new != 0.0 ? 1.0 / pv.dtr_new : 0.0;
-    }
-}
-
-// Hermite weights of the B1 interpolation of row i (as k_main's rowval)
-struct B1W {
-    int F, cubic;
-    double c0, c1, c2, c3;
-};
-__device__ __forceinline__ B1W b1w(const DevCtx& c, const StageDev& sp, int i) {
-    const B1Row r = b1_row(c, c.posB1x[i], sp.maxceil, sp.nrows);
-    return {r.F, r.cubic, r.c0, r.c1, r.c2, r.c3};
-}
-__device__ __forceinline__ double rint_of(const DevCtx& c, const B1W& w) {
+__device__ __forceinline__ double rint_of(const DevCtx& c, const B1Row& w) {
     double ri = w.c0 * c.rvec[w.F - 1] + w.c1 * c.rvec[w.F] - w.c2 * c.drvec[w.F];
     if (w.cubic) ri -= w.c3 * c.drvec[w.F + 1];
     return ri;
 }
-__device__ __forceinline__ void scatter_rint(const DevCtx& c, const AdjDev& a, const B1W& w, double rb) {
+__device__ __forceinline__ void scatter_rint(const DevCtx& c, const AdjDev& a, const B1Row& w, double rb) {
     atomicAdd(a.Hr + w.F - 1, w.c0 * rb);
     atomicAdd(a.Hr + w.F, w.c1 * rb);
     atomicAdd(a.Hdr + w.F, -w.c2 * rb);
     if (w.cubic) atomicAdd(a.Hdr + w.F + 1, -w.c3 * rb);
 }
 
-// --------------------------------------------------------- RHS epilogue
+// Row write, dr/dt (stage 0) and RHS epilogue of stage s, transposed: one column per thread,
+// one-warp CTAs.  Bound by a warp's FP64 rate (one instruction in 64 cycles), so the columns
+// spread over as many SMs as they fill; the sums over columns enter the history linearly, so
+// each CTA adds its own share.  L = 512: 41 us as two kernels of one CTA, now 16.5.
+constexpr int ADJ_ROW_T = 32;
 template <int P, int P2>
-__global__ void __launch_bounds__(256) k_adj_epi(const DevCtx c, const AdjDev a, const AdjModel am, const int s) {
+__global__ void __launch_bounds__(ADJ_ROW_T) k_adj_rows(const DevCtx c, const AdjDev a, const AdjModel am, const int s, const int n0) {
+    wait_prior_grid();
     const StageDev& sp = c.stages[s];
-    const int L = c.L, nrows = sp.nrows, lr = nrows - 1;
-    const double t = sp.T;
-    const bool live = t > 0.0;
+    const int L = c.L, nrows = sp.nrows, lr = nrows - 1, i = blockIdx.x * ADJ_ROW_T + threadIdx.x;
+    const double t = sp.T, td = sp.tdiff;
+    const bool live = t > 0.0, first = blockIdx.x == 0 && threadIdx.x == 0;
     const double q0 = c.KR[(size_t)lr * L].x;
     double rE;
-    B1W wE{};
+    B1Row wE{};
     if (live) {
-        wE = b1w(c, sp, L - 1);
+        wE = a.Bsave[(size_t)s * L + L - 1];
         rE = rint_of(c, wE);
     } else {
         rE = c.rvec[0];
@@ -298,12 +280,20 @@ __global__ void __launch_bounds__(256) k_adj_epi(const DevCtx c, const AdjDev a,
     fder_t<P, P2, 1>(am, q0, f1q0, f1lq0);
     const double fac1 = f1q0 / am.T0, fac2 = q0 / am.T0;
     double sE = 0.0, sF1 = 0.0, sF2 = 0.0, lam = 0.0, gam = 0.0;
-    for (int i = threadIdx.x; i < L; i += blockDim.x) {
+    if (i < L) {
+        RowBars rw = row_write<P, P2>(c, a, am, sp, s, i);
+        // dr of row n0 = tdiff_s DR, summed over the stages
+        if (s == 0) row_drstep<P, P2>(c, am, n0, i, t, a.sc[SC_DR] + td * a.sc[SC_DELTA], rw);
+        a.g0bar[i] = rw.g0b;
+        a.hbar[i] = rw.h0b;
+        lam = rw.lam;
+        const double2 hb = s == 0 ? rw.h0b : a.hbar[(size_t)s * L + i];
+
         const double2 q = c.KR[(size_t)lr * L + i];
         double qb, ri;
-        B1W w{};
+        B1Row w{};
         if (live) {
-            w = b1w(c, sp, i);
+            w = a.Bsave[(size_t)s * L + i];
             qb = w.c0 * c.KR[(size_t)(w.F - 1) * L].x + w.c1 * c.KR[(size_t)w.F * L].x - w.c2 * c.dKR[(size_t)w.F * L].x;
             if (w.cubic) qb -= w.c3 * c.dKR[(size_t)(w.F + 1) * L].x;
             ri = rint_of(c, w);
@@ -312,7 +302,6 @@ __global__ void __launch_bounds__(256) k_adj_epi(const DevCtx c, const AdjDev a,
             ri = c.rvec[0];
         }
         const double th = c.theta[i], tA = t * th, tR = t * (1.0 - th);
-        const double2 hb = a.hbar[(size_t)s * L + i];
         // hK = d1 + d2 th;  hR = (R (-rE) + a6 tR) + (R ri - a7 tR) th
         const double d1b = hb.x, d2b = th * hb.x;
         double* ab = a.abar + (size_t)i * 8;
@@ -328,15 +317,15 @@ __global__ void __launch_bounds__(256) k_adj_epi(const DevCtx c, const AdjDev a,
         const double Kb = -rE * d1b - ri * d2b;
         const double Rb = hb.y * (-rE + ri * th) + 2.0 * am.Gamma * d2b;
         add2(a.HKR + (size_t)lr * L + i, Kb, Rb);
-        sE += -q.y * hb.y - q.x * d1b;
+        sE = -q.y * hb.y - q.x * d1b;
         const double rib = q.y * th * hb.y - q.x * d2b;
         double f1qb, f1lqb;
         fder_t<P, P2, 1>(am, qb, f1qb, f1lqb);
         const double qbb = fac1 * d1b + fd_t<P, P2, 2>(am, qb) * fac2 * d2b;
-        sF1 += qb * d1b;
-        sF2 += f1qb * d2b;
+        sF1 = qb * d1b;
+        sF2 = f1qb * d2b;
         lam += f1lqb * fac2 * d2b;
-        gam += 2.0 * q.y * d2b;
+        gam = 2.0 * q.y * d2b;
         if (live) {
             atomicAdd(&a.HKR[(size_t)(w.F - 1) * L].x, w.c0 * qbb);
             atomicAdd(&a.HKR[(size_t)w.F * L].x, w.c1 * qbb);
@@ -348,11 +337,11 @@ __global__ void __launch_bounds__(256) k_adj_epi(const DevCtx c, const AdjDev a,
             atomicAdd(a.Hr, rib);
         }
     }
-    sE = block_sum(sE);
-    sF1 = block_sum(sF1);
-    sF2 = block_sum(sF2);
-    lam = block_sum(lam);
-    gam = block_sum(gam);
+    sE = warp_sum(sE);
+    sF1 = warp_sum(sF1);
+    sF2 = warp_sum(sF2);
+    lam = warp_sum(lam);
+    gam = warp_sum(gam);
     if (threadIdx.x == 0) {
         // rE = rInt of row L-1; q0 = QK of the last row at theta = 0
         if (live) scatter_rint(c, a, wE, sE);
@@ -360,6 +349,10 @@ __global__ void __launch_bounds__(256) k_adj_epi(const DevCtx c, const AdjDev a,
         const double q0b = sF1 * fd_t<P, P2, 2>(am, q0) / am.T0 + sF2 / am.T0;
         atomicAdd(&a.HKR[(size_t)lr * L].x, q0b);
         atomicAdd(a.sc + SC_LAMBDA, lam + sF1 * f1lq0 / am.T0);
+        if (first) {
+            gam += a.sc[SC_RHO];
+            if (s > 0) a.sc[SC_DR] += td * a.sc[SC_DELTA];
+        }
         atomicAdd(a.sc + SC_GAMMA, gam);
     }
 }
@@ -369,29 +362,24 @@ __global__ void __launch_bounds__(256) k_adj_epi(const DevCtx c, const AdjDev a,
 // gathered values recorded by the recompute, Sigma and the int.dat products
 // differentiated, the B1 gathers transposed into the cotangent history
 // (reductions), the A1/A2 cotangents of the target stored for k_adj_lastrow
-// and its B2 packet for k_adj_b2ser.
+// and its B2 packet for k_adj_b2ser.  Bound by the FP64 pipe (82 % busy): 150 instructions a
+// target with whole derivatives and weights formed per product, 105 now (L = 512: 75 -> 57 us).
 template <int M, int P, int P2>
 __global__ void __launch_bounds__(64) k_adj_targets(const DevCtx c, const AdjDev a, const AdjModel am, const int s) {
+    wait_prior_grid();
     const StageDev& sp = c.stages[s];
     const int L = c.L, i = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nrows = sp.nrows;
     const double t = sp.T;
     if (!(t > 0.0)) return;  // t = 0: the memory integrals carry a factor t, all cotangents vanish
-    __shared__ double s_c[4];
-    __shared__ int s_bi[2];
-    if (threadIdx.x == 0) {
-        const B1Row r = b1_row(c, c.posB1x[i], sp.maxceil, nrows);
-        s_c[0] = r.c0; s_c[1] = r.c1; s_c[2] = r.c2; s_c[3] = r.c3;
-        s_bi[0] = r.F; s_bi[1] = r.cubic;
-    }
-    __syncthreads();
     double lam = 0.0;
     if (j < L) {
-        double ab[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) ab[k] = a.abar[(size_t)i * 8 + k];
-        const double bc0 = s_c[0], bc1 = s_c[1], bc2 = s_c[2], bc3 = s_c[3];
-        const int F = s_bi[0], cubic1 = s_bi[1];
+        // row cotangents times the target's weight; rows 1, 2 and 4, 5 have the same
+        const double W = c.integ[j];
+        const double* ar = a.abar + (size_t)i * 8;
+        const double w0 = W * ar[0], w1 = W * ar[1], w3 = W * ar[3], w4 = W * ar[4], w6 = W * ar[6], w7 = W * ar[7];
+        const B1Row br = a.Bsave[(size_t)s * L + i];
+        const double bc0 = br.c0, bc1 = br.c1, bc2 = br.c2, bc3 = br.c3;
+        const int F = br.F, cubic1 = br.cubic;
         const size_t ij = (size_t)i * L + j;
         // ---- forward values, recorded by k_main in the recompute of this stage
         const GatherRec g = a.rec[(size_t)s * L * L + ij];
@@ -414,20 +402,19 @@ __global__ void __launch_bounds__(64) k_adj_targets(const DevCtx c, const AdjDev
         fder_t<P, P2, 3>(am, b2.x, fB2[3], lB2[2]);
         const double sKA1 = fA1[1], sRA1 = fA1[2] * a1.y, sRA2 = fA2[2] * a2.y;
         const double sKB1 = fB1[1], sRB1 = fB1[2] * b1.y, sKB2 = fB2[1], sRB2 = fB2[2] * b2.y;
-        const double W = c.integ[j];
         // ---- cotangents of the eight products P_k (row sums a_k)
-        const double sRA2b = W * (b2.x * ab[0] + b2.y * ab[6]);
-        double b2Kb = W * sRA2 * ab[0], b2Rb = W * sRA2 * ab[6];
-        const double sRA1b = W * b1.x * ab[1];
-        double b1Kb = W * sRA1 * ab[1];
-        const double sKA1b = W * b1.y * ab[2];
-        double b1Rb = W * sKA1 * ab[2];
-        double a2Rb = W * (sKB2 * ab[3] + sRB2 * ab[7]);
-        const double sKB2b = W * a2.y * ab[3], sRB2b = W * a2.y * ab[7];
-        double a1Rb = W * sKB1 * ab[4];
-        const double sKB1b = W * a1.y * ab[4];
-        double a1Kb = W * sRB1 * ab[5];
-        const double sRB1b = W * a1.x * ab[5];
+        const double sRA2b = b2.x * w0 + b2.y * w6;
+        double b2Kb = sRA2 * w0, b2Rb = sRA2 * w6;
+        const double sRA1b = b1.x * w1;
+        double b1Kb = sRA1 * w1;
+        const double sKA1b = b1.y * w1;
+        double b1Rb = sKA1 * w1;
+        double a2Rb = sKB2 * w3 + sRB2 * w7;
+        const double sKB2b = a2.y * w3, sRB2b = a2.y * w7;
+        double a1Rb = sKB1 * w4;
+        const double sKB1b = a1.y * w4;
+        double a1Kb = sRB1 * w4;
+        const double sRB1b = a1.x * w4;
         // ---- Sigma transposed: sK = f'(K), sR = f''(K) R
         a1Kb += fA1[2] * sKA1b + fA1[3] * a1.y * sRA1b;
         a1Rb += fA1[2] * sRA1b;
@@ -460,8 +447,11 @@ __global__ void __launch_bounds__(64) k_adj_targets(const DevCtx c, const AdjDev
 // shared memory when it leaves the column: two FMAs per entry whatever the
 // stencil starts look like (runs of equal starts near theta = 0 or 1 only
 // make long columns, split over several threads).  The row goes to
-// lbar_part[i] for k_adj_lastreduce.
-__global__ void __launch_bounds__(256) k_adj_lastrow(const DevCtx c, const AdjDev a, const int s) {
+// lbar_part[i] for k_adj_lastreduce.  The entries lie as the threads take them, entry q of
+// every thread side by side: read run by run they cost an L1 line per lane (L = 512: 55 us, now
+// 43; the FP64 pipe is 72 % busy).
+__global__ void __launch_bounds__(LR_T) k_adj_lastrow(const DevCtx c, const AdjDev a, const int s) {
+    wait_prior_grid();
     const StageDev& sp = c.stages[s];
     if (!(sp.T > 0.0)) return;
     const int L = c.L, i = blockIdx.x, E = 2 * L * c.m;
@@ -474,24 +464,24 @@ __global__ void __launch_bounds__(256) k_adj_lastrow(const DevCtx c, const AdjDe
     for (int k = threadIdx.x; k < 2 * L; k += blockDim.x) s_cb[k] = a.abarA[2 * row + k];
     for (int k = threadIdx.x; k <= L; k += blockDim.x) s_cs[k] = __ldg(cs + k);
     __syncthreads();
-    const int per = (E + blockDim.x - 1) / blockDim.x;
+    const int per = (E + LR_T - 1) / LR_T;
     const int p0 = threadIdx.x * per, p1 = min(p0 + per, E);
     if (p0 < p1) {
-        const double* w = a.lrW + (size_t)i * E;
-        const int* src = a.lrS + (size_t)i * E;
+        const double* w = a.lrW + (size_t)i * per * LR_T + threadIdx.x;
+        const unsigned short* src = a.lrS + (size_t)i * per * LR_T + threadIdx.x;
         int lo = 0, hi = L;  // column of entry p0: the last k with cs[k] <= p0
         while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (s_cs[mid] <= p0) lo = mid; else hi = mid; }
         int k = lo, kend = s_cs[k + 1];
         double ax = 0.0, ay = 0.0;
         constexpr int B = 8;  // entries loaded ahead
-        for (int pb = p0; pb < p1; pb += B) {
+        for (int pb = p0, k0 = 0; pb < p1; pb += B, k0 += B) {
             double u[B];
             int si[B];
 #pragma unroll
             for (int q = 0; q < B; ++q) {
                 const bool in = pb + q < p1;
-                u[q] = in ? __ldg(w + pb + q) : 0.0;
-                si[q] = in ? __ldg(src + pb + q) : 0;
+                u[q] = in ? __ldg(w + (size_t)(k0 + q) * LR_T) : 0.0;
+                si[q] = in ? __ldg(src + (size_t)(k0 + q) * LR_T) : 0;
             }
 #pragma unroll
             for (int q = 0; q < B; ++q) {
@@ -516,21 +506,25 @@ __global__ void __launch_bounds__(256) k_adj_lastrow(const DevCtx c, const AdjDe
 }
 
 // B2 gathers transposed from the packets in static (iB2, phi2) order.  Each
-// thread runs over B2_RUN consecutive packets; packets with the same key
+// thread runs over `run` consecutive packets; packets with the same key
 // (X, iB2) add into the same 8 m history entries (K rows X-1, X; dK rows X,
 // X+1; two components), so the thread accumulates them in registers (8 m
 // FMAs per packet) and adds the sums to the history when the key changes or
 // the run ends.  A warp whose 32 runs all carry one key (phi2 near 0 or 1)
 // sums the runs across the warp first.  No key order is assumed: a key that
-// recurs non-contiguously only means more additions.
-constexpr int B2_RUN = 8;
-__device__ __forceinline__ void b2_coeffs(const DevCtx& c, int X, double x, int nrows, double e[4]) {
+// recurs non-contiguously only means more additions.  Bound by the FP64 pipe (98 instructions a
+// packet), of which every SM scheduler has its own: the run is what gives each of them two
+// warps (L = 512: 7; runs of 8 leave a sixth of the pipes idle at the end), and at least
+// B2_RUN_MIN, for fewer additions.
+constexpr int B2_RUN_MIN = 2, B2_WARPS_SM = 8;
+// inv: 1 / delta_t_ratio of row X + 1 (unused where X is the last but one)
+__device__ __forceinline__ void b2_coeffs(double inv, int X, double x, int nrows, double e[4]) {
     const double x2 = x * x, x3 = x2 * x;
     if (X < nrows - 1) {
         e[0] = 1.0 - 3.0 * x2 + 2.0 * x3;   // K row X-1
         e[1] = 3.0 * x2 - 2.0 * x3;         // K row X
         e[2] = x - 2.0 * x2 + x3;           // dK row X
-        e[3] = (x3 - x2) * c.inv_dtr[X + 1];  // dK row X+1
+        e[3] = (x3 - x2) * inv;           // dK row X+1
     } else {
         e[0] = 1.0 - x2;
         e[1] = x2;
@@ -538,27 +532,47 @@ __device__ __forceinline__ void b2_coeffs(const DevCtx& c, int X, double x, int 
         e[3] = 0.0;
     }
 }
+// Add the sums of the lanes in `mask` to the history, a lane's 8 M values at a time by the
+// whole warp: its four rows' 2 M consecutive doubles then go out as a few sectors each.  (As
+// 8 M additions of one lane each, all to different lines, they were 9 M requests a stage at
+// L = 512: 84 us, now 68.)
 template <int M>
-__device__ __forceinline__ void b2_flush(const DevCtx& c, const AdjDev& a, int X, int iB2, bool cubic2,
-                                         const double acc[M][8]) {
-    const int L = c.L;
-    const size_t base = (size_t)(X - 1) * L + iB2;
+__device__ __forceinline__ void b2_flush(const DevCtx& c, const AdjDev& a, unsigned mask, int X, int iB2, int nrows,
+                                         const double acc[M][8], double* s_acc) {
+    constexpr int N = 8 * M, STRIDE = N + 2;  // + 2: the lanes' 16-byte stores hit different banks
+    const int lane = threadIdx.x & 31, L2 = 2 * c.L;
+    if ((mask >> lane) & 1u) {
+        double2* o = reinterpret_cast<double2*>(s_acc + lane * STRIDE);
 #pragma unroll
-    for (int d = 0; d < M; ++d) {
-        add2(a.HKR + base + d, acc[d][0], acc[d][1]);
-        add2(a.HKR + base + L + d, acc[d][2], acc[d][3]);
-        add2(a.HdKR + base + L + d, acc[d][4], acc[d][5]);
-        if (cubic2) add2(a.HdKR + base + 2 * L + d, acc[d][6], acc[d][7]);
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int d = 0; d < M; ++d) o[k * M + d] = make_double2(acc[d][2 * k], acc[d][2 * k + 1]);
     }
+    __syncwarp();
+    while (mask) {
+        const int f = __ffs(mask) - 1;
+        mask &= mask - 1;
+        const int fX = __shfl_sync(0xffffffffu, X, f), fB = __shfl_sync(0xffffffffu, iB2, f);
+        const size_t base = ((size_t)(fX - 1) * c.L + fB) * 2;
+#pragma unroll
+        for (int t0 = 0; t0 < N; t0 += 32) {
+            const int t = t0 + lane, k = t / (2 * M), e = t - k * 2 * M;  // row K X-1, K X, dK X, dK X+1
+            if (t < (fX < nrows - 1 ? N : N - 2 * M))
+                atomicAdd(reinterpret_cast<double*>(k < 2 ? a.HKR : a.HdKR) + base + (k == 0 ? 0 : k == 3 ? 2 * L2 : L2) + e,
+                          s_acc[f * STRIDE + t]);
+        }
+    }
+    __syncwarp();
 }
 template <int M>
-__global__ void __launch_bounds__(128) k_adj_b2ser(const DevCtx c, const AdjDev a, const int s) {
+__global__ void __launch_bounds__(32, 8) k_adj_b2ser(const DevCtx c, const AdjDev a, const int s, const int run) {
+    wait_prior_grid();
     const StageDev& sp = c.stages[s];
     if (!(sp.T > 0.0)) return;
+    __shared__ __align__(16) double s_acc[32 * (8 * M + 2)];
     const int L = c.L, nrows = sp.nrows, lane = threadIdx.x & 31;
     const long long NP = (long long)L * L;
-    const long long q0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * B2_RUN;
-    if (__ballot_sync(0xffffffffu, q0 < NP) == 0u) return;  // whole warp past the end
+    const long long q0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * run;
     double acc[M][8];
 #pragma unroll
     for (int d = 0; d < M; ++d)
@@ -566,40 +580,59 @@ __global__ void __launch_bounds__(128) k_adj_b2ser(const DevCtx c, const AdjDev 
         for (int k = 0; k < 8; ++k) acc[d][k] = 0.0;
     long long key = -1;
     int kX = 1, kB = 0, nkeys = 0;
-    for (int r = 0; r < B2_RUN; ++r) {
-        const long long q = q0 + r;
-        if (q >= NP) break;
-        const AdjDev::B2Packet pk = a.b2pk[q];
-        const int iB2 = __ldg(c.iB2 + pk.ij);
+    // the next packet is on its way while this one's FMAs run
+    const int cnt = (int)max(0ll, min((long long)run, NP - q0));
+    AdjDev::B2Packet nx = {};
+    int nB = 0;
+    double ninv = 0.0;
+    if (cnt > 0) {
+        nx = a.b2pk[q0];
+        nB = __ldg(c.iB2 + nx.ij);
+        ninv = c.inv_dtr[min(nx.X + 1, nrows - 1)];
+    }
+    for (int r = 0; r < run; ++r) {
+        const AdjDev::B2Packet pk = nx;
+        const int iB2 = nB;
+        const double inv = ninv;
+        const bool in = r < cnt;
+        double w[M];
+#pragma unroll
+        for (int d = 0; d < M; d += 2) {
+            const double2 v = in ? __ldg(reinterpret_cast<const double2*>(c.wB2 + (size_t)pk.ij * M + d)) : make_double2(0.0, 0.0);
+            w[d] = v.x;
+            w[d + 1] = v.y;
+        }
+        if (r + 1 < cnt) nx = a.b2pk[q0 + r + 1];
         const long long kq = ((long long)pk.X << 32) | (unsigned)iB2;
-        if (kq != key) {
-            if (nkeys > 0) {
-                b2_flush<M>(c, a, kX, kB, kX < nrows - 1, acc);
+        const bool change = in && kq != key;
+        const unsigned mask = __ballot_sync(0xffffffffu, change && nkeys > 0);
+        if (mask) b2_flush<M>(c, a, mask, kX, kB, nrows, acc, s_acc);
+        if (change) {
 #pragma unroll
-                for (int d = 0; d < M; ++d)
+            for (int d = 0; d < M; ++d)
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) acc[d][k] = 0.0;
-            }
+                for (int k = 0; k < 8; ++k) acc[d][k] = 0.0;
             key = kq;
             kX = pk.X;
             kB = iB2;
             ++nkeys;
         }
         double e[4];
-        b2_coeffs(c, pk.X, pk.x, nrows, e);
+        b2_coeffs(inv, pk.X, pk.x, nrows, e);
         double eg[8];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            eg[2 * k] = e[k] * pk.gK;
-            eg[2 * k + 1] = e[k] * pk.gR;
+            eg[2 * k] = in ? e[k] * pk.gK : 0.0;
+            eg[2 * k + 1] = in ? e[k] * pk.gR : 0.0;
         }
-        const double* w = c.wB2 + (size_t)pk.ij * M;
-#pragma unroll
-        for (int d = 0; d < M; ++d) {
-            const double wd = __ldg(w + d);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) acc[d][k] = fma(eg[k], wd, acc[d][k]);
+        if (r + 1 < cnt) {
+            nB = __ldg(c.iB2 + nx.ij);
+            ninv = c.inv_dtr[min(nx.X + 1, nrows - 1)];
         }
+#pragma unroll
+        for (int d = 0; d < M; ++d)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[d][k] = fma(eg[k], w[d], acc[d][k]);
     }
     // one key over the whole warp: reduce across the lanes, 8 lanes add
     const long long k0 = __shfl_sync(0xffffffffu, key, 0);
@@ -618,12 +651,13 @@ __global__ void __launch_bounds__(128) k_adj_b2ser(const DevCtx c, const AdjDev 
         }
         return;
     }
-    if (nkeys > 0) b2_flush<M>(c, a, kX, kB, kX < nrows - 1, acc);
+    b2_flush<M>(c, a, __ballot_sync(0xffffffffu, nkeys > 0), kX, kB, nrows, acc, s_acc);
 }
 
 // B2 transposed for a generic stencil depth: one thread per packet, m taps
 // added directly.
 __global__ void __launch_bounds__(256) k_adj_b2gen(const DevCtx c, const AdjDev a, const int s) {
+    wait_prior_grid();
     const StageDev& sp = c.stages[s];
     if (!(sp.T > 0.0)) return;
     const int L = c.L, m = c.m, nrows = sp.nrows;
@@ -632,7 +666,7 @@ __global__ void __launch_bounds__(256) k_adj_b2gen(const DevCtx c, const AdjDev 
     const AdjDev::B2Packet pk = a.b2pk[q];
     const int iB2 = __ldg(c.iB2 + pk.ij);
     double e[4];
-    b2_coeffs(c, pk.X, pk.x, nrows, e);
+    b2_coeffs(c.inv_dtr[min(pk.X + 1, nrows - 1)], pk.X, pk.x, nrows, e);
     const bool cubic2 = pk.X < nrows - 1;
     const size_t base = (size_t)(pk.X - 1) * L + iB2;
     const double* w = c.wB2 + (size_t)pk.ij * m;
@@ -652,6 +686,7 @@ __global__ void __launch_bounds__(256) k_adj_b2gen(const DevCtx c, const AdjDev 
 constexpr int LR_COLS = 32, LR_LANES = 8, LR_SLICES = 16;
 __global__ void __launch_bounds__(LR_COLS * LR_LANES) k_adj_lastreduce(const DevCtx c, const AdjDev a, const int s,
                                                                       const int lr) {
+    wait_prior_grid();
     const int L = c.L;
     if (!(c.stages[s].T > 0.0)) return;
     __shared__ double2 s_acc[LR_LANES][LR_COLS];
@@ -745,22 +780,26 @@ cudaError_t launch_targets_pp(const DevCtx& c, const AdjDev& a, const AdjModel& 
     const dim3 grid((c.L + 63) / 64, c.L);
     const size_t lsm = lastrow_smem(c.L, c.m);
     const size_t NP = (size_t)c.L * c.L;
-    if (c.m == 10) {
-        k_adj_targets<10, P, P2><<<grid, 64, 0, st>>>(c, a, am, s);
-        k_adj_lastrow<<<c.L, 256, lsm, st>>>(c, a, s);
-        k_adj_b2ser<10><<<(unsigned)((NP + 128 * B2_RUN - 1) / (128 * B2_RUN)), 128, 0, st>>>(c, a, s);
-    } else {
-        k_adj_targets<0, P, P2><<<grid, 64, 0, st>>>(c, a, am, s);
-        k_adj_lastrow<<<c.L, 256, lsm, st>>>(c, a, s);
-        k_adj_b2gen<<<(unsigned)((NP + 255) / 256), 256, 0, st>>>(c, a, s);
-    }
-    return cudaGetLastError();
+    cudaError_t e = launch_pdl(c.m == 10 ? k_adj_targets<10, P, P2> : k_adj_targets<0, P, P2>, grid, dim3(64), 0, st, c, a, am, s);
+    if (e != cudaSuccess) return e;
+    if ((e = launch_pdl(k_adj_lastrow, dim3(c.L), dim3(LR_T), lsm, st, c, a, s)) != cudaSuccess) return e;
+    if (c.m != 10) return launch_pdl(k_adj_b2gen, dim3((unsigned)((NP + 255) / 256)), dim3(256), 0, st, c, a, s);
+    int dev = 0, sms = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    const size_t lanes = (size_t)32 * B2_WARPS_SM * sms;
+    const int run = (int)std::max<size_t>(B2_RUN_MIN, (NP + lanes - 1) / lanes);
+    return launch_pdl(k_adj_b2ser<10>, dim3((unsigned)((NP + 32 * (size_t)run - 1) / (32 * (size_t)run))), dim3(32), 0, st, c, a, s, run);
 }
 cudaError_t launch_targets(const DevCtx& c, const AdjDev& a, const AdjModel& am, int s,
                            cudaStream_t st) {
     if (am.p == 3 && am.p2 == 4) return launch_targets_pp<3, 4>(c, a, am, s, st);
     if (am.p == 3 && am.p2 == 0) return launch_targets_pp<3, 0>(c, a, am, s, st);
     return launch_targets_pp<-1, -1>(c, a, am, s, st);
+}
+
+cudaError_t launch_adj_save(const DevCtx& c, const AdjDev& a, int k, int n0, cudaStream_t st) {
+    return launch_pdl(k_adj_save, dim3((c.L + 63) / 64), dim3(64), 0, st, c, a, k, n0);
 }
 
 cudaError_t launch_adj_step(const DevCtx& c, const AdjDev& a, const AdjModel& am, int S, int n0, cudaStream_t st) {
@@ -770,17 +809,16 @@ cudaError_t launch_adj_step(const DevCtx& c, const AdjDev& a, const AdjModel& am
     if ((e = cudaMemsetAsync(a.hbar, 0, (size_t)SMAX * L * sizeof(double2), st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(a.g0bar, 0, (size_t)L * sizeof(double2), st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(a.sc + SC_DR, 0, sizeof(double), st)) != cudaSuccess) return e;
-    k_adj_move<<<eb, 256, 0, st>>>(c, a, n0);
     for (int s = S - 1; s >= 0; --s) {
-        ADJ_DISPATCH(am, (k_adj_rowwrite<P, P2><<<1, 256, 0, st>>>(c, a, am, s)));
-        if (s == 0) ADJ_DISPATCH(am, (k_adj_drstep<P, P2><<<1, 256, 0, st>>>(c, a, am, n0)));
-        k_adj_restore<<<eb, 256, 0, st>>>(c, a, s, n0);
-        ADJ_DISPATCH(am, (k_adj_epi<P, P2><<<1, 256, 0, st>>>(c, a, am, s)));
+        if ((e = launch_pdl(k_adj_enter, dim3((L + 63) / 64), dim3(64), 0, st, c, a, s, n0)) != cudaSuccess) return e;
+        const dim3 rg((L + ADJ_ROW_T - 1) / ADJ_ROW_T);
+        ADJ_DISPATCH(am, (e = launch_pdl(k_adj_rows<P, P2>, rg, dim3(ADJ_ROW_T), 0, st, c, a, am, s, n0)));
+        if (e != cudaSuccess) return e;
         if ((e = launch_targets(c, a, am, s, st)) != cudaSuccess) return e;
         // the last row of stage s is row n0 (s >= 1) or n0-1 (s = 0)
-        k_adj_lastreduce<<<dim3((L + LR_COLS - 1) / LR_COLS, LR_SLICES), LR_COLS * LR_LANES, 0, st>>>(
-            c, a, s, s >= 1 ? n0 : n0 - 1);
-        if (s >= 1) k_adj_move<<<eb, 256, 0, st>>>(c, a, n0);
+        if ((e = launch_pdl(k_adj_lastreduce, dim3((L + LR_COLS - 1) / LR_COLS, LR_SLICES), dim3(LR_COLS * LR_LANES), 0, st, c, a,
+                            s, s >= 1 ? n0 : n0 - 1)) != cudaSuccess)
+            return e;
     }
     k_adj_finish<<<eb, 256, 0, st>>>(c, a, n0);
     return cudaGetLastError();

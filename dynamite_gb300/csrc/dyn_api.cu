@@ -100,7 +100,7 @@ struct Ctx {
     }
 
     void release_adjoint() {
-        void* ab[] = {ad.HKR, ad.HdKR, ad.Hr, ad.Hdr, ad.Gsave, ad.Dsave, ad.rsave, ad.drsave, ad.Psave, ad.hbar,
+        void* ab[] = {ad.HKR, ad.HdKR, ad.Hr, ad.Hdr, ad.Gsave, ad.Dsave, ad.tsave, ad.Bsave, ad.hbar,
                       ad.g0bar, ad.Gbar, ad.Dbar, ad.abar, ad.lbar_part, ad.abarA, ad.sc, ad.b2pk, ad.b2rank, ad.rec, ad.lrW, ad.lrS, ad.lrC, ad_ck, snap_KR, snap_dKR, snap_time};
         for (void* b : ab) if (b) cudaFree(b);
         std::memset(&ad, 0, sizeof ad);
@@ -401,13 +401,13 @@ struct Ctx {
         dyn_status s;
         if ((s = dalloc(&ad.HKR, cap * Lz)) || (s = dalloc(&ad.HdKR, cap * Lz)) || (s = dalloc(&ad.Hr, cap)) ||
             (s = dalloc(&ad.Hdr, cap)) || (s = dalloc(&ad.Gsave, (size_t)SMAX * Lz)) ||
-            (s = dalloc(&ad.Dsave, (size_t)SMAX * Lz)) || (s = dalloc(&ad.rsave, SMAX)) || (s = dalloc(&ad.drsave, SMAX)) ||
-            (s = dalloc(&ad.Psave, (size_t)SMAX * Lz)) || (s = dalloc(&ad.hbar, (size_t)SMAX * Lz)) ||
+            (s = dalloc(&ad.Dsave, (size_t)SMAX * Lz)) || (s = dalloc(&ad.tsave, 5 * SMAX)) ||
+            (s = dalloc(&ad.Bsave, (size_t)SMAX * Lz)) || (s = dalloc(&ad.hbar, (size_t)SMAX * Lz)) ||
             (s = dalloc(&ad.g0bar, Lz)) || (s = dalloc(&ad.Gbar, Lz)) || (s = dalloc(&ad.Dbar, Lz)) ||
             (s = dalloc(&ad.abar, 8 * Lz)) || (s = dalloc(&ad.lbar_part, Lz * Lz)) || (s = dalloc(&ad.abarA, 2 * Lz * Lz)) || (s = dalloc(&ad.sc, 16)) ||
             (s = dalloc(&ad.b2pk, Lz * Lz)) || (s = dalloc(&ad.b2rank, Lz * Lz)) ||
-            (s = dalloc(&ad.rec, (size_t)SMAX * Lz * Lz)) || (s = dalloc(&ad.lrW, 2 * Lz * Lz * (size_t)d.m)) ||
-            (s = dalloc(&ad.lrS, 2 * Lz * Lz * (size_t)d.m)) || (s = dalloc(&ad.lrC, Lz * (Lz + 1))) ||
+            (s = dalloc(&ad.rec, (size_t)SMAX * Lz * Lz)) || (s = dalloc(&ad.lrW, Lz * lr_per(Lz, d.m) * LR_T)) ||
+            (s = dalloc(&ad.lrS, Lz * lr_per(Lz, d.m) * LR_T)) || (s = dalloc(&ad.lrC, Lz * (Lz + 1))) ||
             (s = dalloc(&ad_ck, 4 * Lz)) || (s = dalloc(&snap_KR, cap * Lz)) || (s = dalloc(&snap_dKR, cap * Lz)) ||
             (s = dalloc(&snap_time, 5 * cap))) {
             release_adjoint();
@@ -435,11 +435,12 @@ struct Ctx {
             for (size_t q = 0; q < L2; ++q) rank[ord[q]] = (int)q;
             CK(cudaMemcpy(ad.b2rank, rank.data(), L2 * sizeof(int), cudaMemcpyHostToDevice));
             // A1/A2 of each row as a column-sorted sparse matrix (counting sort by column)
-            const size_t mz = d.m, E = 2 * Lz * mz;
+            const size_t mz = d.m, per = lr_per(Lz, mz), E = per * LR_T;
             std::vector<double> wA(2 * L2 * mz), lw(Lz * E);
             CK(cudaMemcpy(wA.data(), d.wA1, L2 * mz * sizeof(double), cudaMemcpyDeviceToHost));
             CK(cudaMemcpy(wA.data() + L2 * mz, d.wA2, L2 * mz * sizeof(double), cudaMemcpyDeviceToHost));
-            std::vector<int> ls(Lz * E), lc(Lz * (Lz + 1));
+            std::vector<unsigned short> ls(Lz * E);
+            std::vector<int> lc(Lz * (Lz + 1));
             for (size_t i = 0; i < Lz; ++i) {
                 int* cs = lc.data() + i * (Lz + 1);
                 std::fill(cs, cs + Lz + 1, 0);
@@ -451,13 +452,13 @@ struct Ctx {
                 for (int t = 0; t < 2; ++t)
                     for (size_t j = 0; j < Lz; ++j)
                         for (size_t dd = 0; dd < mz; ++dd) {
-                            const size_t col = iA[t * L2 + i * Lz + j] + dd, p = i * E + fill[col]++;
+                            const size_t col = iA[t * L2 + i * Lz + j] + dd, e = fill[col]++, p = i * E + (e % per) * LR_T + e / per;
                             lw[p] = wA[t * L2 * mz + (i * Lz + j) * mz + dd];
-                            ls[p] = (int)(2 * j + t);
+                            ls[p] = (unsigned short)(2 * j + t);
                         }
             }
             CK(cudaMemcpy(ad.lrW, lw.data(), Lz * E * sizeof(double), cudaMemcpyHostToDevice));
-            CK(cudaMemcpy(ad.lrS, ls.data(), Lz * E * sizeof(int), cudaMemcpyHostToDevice));
+            CK(cudaMemcpy(ad.lrS, ls.data(), Lz * E * sizeof(unsigned short), cudaMemcpyHostToDevice));
             CK(cudaMemcpy(ad.lrC, lc.data(), Lz * (Lz + 1) * sizeof(int), cudaMemcpyHostToDevice));
         }
         ad_cap = cap;
@@ -467,15 +468,15 @@ struct Ctx {
     size_t adjoint_bytes() const {
         const size_t Lz = L;
         return (cap * Lz * 2 * sizeof(double2)) * 2 + cap * 2 * sizeof(double) + 5 * cap * sizeof(double) +
-               (size_t)SMAX * Lz * (3 * sizeof(double2) + sizeof(double)) + 3 * Lz * Lz * sizeof(double2) +
+               (size_t)SMAX * Lz * (3 * sizeof(double2) + sizeof(B1Row)) + 3 * Lz * Lz * sizeof(double2) +
                Lz * Lz * (sizeof(AdjDev::B2Packet) + sizeof(int) + SMAX * sizeof(GatherRec)) +
-               2 * Lz * Lz * (size_t)d.m * (sizeof(double) + sizeof(int)) + Lz * (Lz + 1) * sizeof(int) +
-               Lz * (3 * sizeof(double2) + 9 * sizeof(double)) + 2 * SMAX * sizeof(double) + 16 * sizeof(double);
+               Lz * lr_per(Lz, d.m) * LR_T * (sizeof(double) + sizeof(unsigned short)) + Lz * (Lz + 1) * sizeof(int) +
+               Lz * (3 * sizeof(double2) + 9 * sizeof(double)) + 5 * SMAX * sizeof(double) + 16 * sizeof(double);
     }
 
     // Step n0 -> n0 + 1 again from the history prefix (same kernels, same
     // stage descriptors as the forward), keeping what the reverse sweep needs
-    // of each stage: the B1 positions it read and row n0 after it.
+    // of each stage: the B1 rows it read and row n0 after it.
     dyn_status recompute_step(int method, double dt, int* S_out) {
         // stages_h is the source of an asynchronous copy: the previous step's
         // copy must have run before the records are rewritten
@@ -489,15 +490,12 @@ struct Ctx {
         CK(launch_pos_init(d, (int)n0, st));
         CK(cudaMemcpyAsync(d.stages, stages_h, sizeof(StageDev) * S, cudaMemcpyHostToDevice, st));
         CK(cudaEventRecord(stages_copied, st));
+        CK(cudaMemcpyAsync(ad.Bsave, d.b1, Lz * sizeof(B1Row), cudaMemcpyDeviceToDevice, st));
         for (int k = 0; k < S; ++k) {
-            CK(cudaMemcpyAsync(ad.Psave + k * Lz, d.posB1x, Lz * sizeof(double), cudaMemcpyDeviceToDevice, st));
             DevCtx dr = d;
             dr.rec = ad.rec + (size_t)k * Lz * Lz;  // k_main records its gathers for the reverse stage
             CK(launch_stage(dr, k, st));
-            CK(cudaMemcpyAsync(ad.Gsave + k * Lz, d.KR + n0 * Lz, Lz * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-            CK(cudaMemcpyAsync(ad.Dsave + k * Lz, d.dKR + n0 * Lz, Lz * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-            CK(cudaMemcpyAsync(ad.rsave + k, d.rvec + n0, sizeof(double), cudaMemcpyDeviceToDevice, st));
-            CK(cudaMemcpyAsync(ad.drsave + k, d.drvec + n0, sizeof(double), cudaMemcpyDeviceToDevice, st));
+            CK(launch_adj_save(d, ad, k, (int)n0, st));
         }
         t1.push_back(Tf);
         dtr.push_back(dtrf);

@@ -152,9 +152,8 @@ struct AdjDev {
     double* Hdr;       // [cap]
     double2* Gsave;    // [SMAX][L] row n0 (QK, QR) after stage s
     double2* Dsave;    // [SMAX][L] row n0 (dQK, dQR) after stage s
-    double* rsave;     // [SMAX] r of row n0 after stage s
-    double* drsave;    // [SMAX]
-    double* Psave;     // [SMAX][L] B1 positions stage s read
+    double* tsave;     // [SMAX][5] r, dr, t, delta_t_ratio and its inverse of row n0 after stage s
+    B1Row* Bsave;      // [SMAX][L] B1 rows stage s read
     double2* hbar;     // [SMAX][L] cotangents of the stage right-hand sides
     double2* g0bar;    // [L] cotangent of the step's base row
     double2* Gbar;     // [L] cotangent of row n0's (QK, QR) after the current stage
@@ -175,15 +174,29 @@ struct AdjDev {
     GatherRec* rec;      // [SMAX][L*L] gathered values of each stage of the recomputed step
     // A1 and A2 gathers of each target row as one column-sorted sparse
     // matrix onto the last row (static): entry p of row i adds
-    // lrW[p] * (cotangent 2j+t of the row) to column k for lrC[k] <= p < lrC[k+1]
-    double* lrW;         // [L][2*L*m]
-    int* lrS;            // [L][2*L*m] source 2j+t
+    // lrW(p) * (cotangent 2j+t of the row) to column k for lrC[k] <= p < lrC[k+1].
+    // Thread p / per of the LR_T that share a row takes per = lr_per entries in a run; entry
+    // p lies at (p % per) * LR_T + p / per of its row's per * LR_T
+    double* lrW;             // [L][per * LR_T]
+    unsigned short* lrS;     // [L][per * LR_T] source 2j+t (L <= 4096)
     int* lrC;            // [L][L+1] column starts
 };
 struct AdjModel {
     int p, p2;
     double lam, T0, Gamma;
+    double ca[5], cb[5];  // k-th derivative of f: ca[k] q^(p-k) + cb[k] q^(p2-k)
+    AdjModel(int p_, int p2_, double lam_, double T0_, double Gamma_) : p(p_), p2(p2_), lam(lam_), T0(T0_), Gamma(Gamma_) {
+        double f = 1.0, f2 = 1.0;
+        for (int k = 0; k < 5; ++k) {
+            ca[k] = lam * f;
+            cb[k] = (1.0 - lam) * f2;
+            f *= (double)(p - k);
+            f2 *= (double)(p2 - k);
+        }
+    }
 };
+constexpr int LR_T = 256;  // threads of k_adj_lastrow
+inline size_t lr_per(size_t L, size_t m) { return (2 * L * m + LR_T - 1) / LR_T; }
 
 // Model coefficients in the reference's host evaluation order
 // (math_ops.cpp:27-37: (lambda*p)*(p-1)... with p as the integer exponent)
@@ -318,6 +331,7 @@ cudaError_t launch_unpack_rows(const double2* in, double* QK, double* QR, size_t
 cudaError_t launch_adj_seed(const DevCtx& c, const AdjDev& a, const AdjModel& am, int nl, double wE, double wR,
                             double wDr, const double* cK, const double* cR, const double* cdK, const double* cdR,
                             cudaStream_t st);
+cudaError_t launch_adj_save(const DevCtx& c, const AdjDev& a, int k, int n0, cudaStream_t st);
 cudaError_t launch_adj_step(const DevCtx& c, const AdjDev& a, const AdjModel& am, int S, int n0, cudaStream_t st);
 cudaError_t launch_adj_initial(const AdjDev& a, const AdjModel& am, cudaStream_t st);
 cudaError_t launch_adj_verify(const DevCtx& c, const AdjDev& a, const double2* snapKR, const double2* snapdKR,
