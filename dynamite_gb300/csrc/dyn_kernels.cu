@@ -103,13 +103,21 @@ __device__ __forceinline__ double2 b2_sum(const DevCtx& c, const size_t ij, cons
 // list off with full warps whatever targets it came from, and every target then
 // reads its four sums back.  Without planes (KEEP false: the allocation-free
 // right-hand side, or no memory for them) every target forms its own.
-template <int M, int K, int P, int P2, bool LOGR, bool KEEP>
-__global__ void __launch_bounds__(64) k_main(const DevCtx c, const int s) {
+//
+// SPLIT: two threads a target, two warps each for the halves that meet only in the row sums:
+// the first half of the CTA its position and B2, the second A1, B1 and A2 meanwhile.  For
+// lengths whose rows leave most schedulers without a warp, where a warp's own FP64 rate (one
+// instruction in 64 cycles) bounds the stage; the same bits.
+template <int M, int K, int P, int P2, bool LOGR, bool KEEP, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 128 : 64) k_main(const DevCtx c, const int s) {
+    static_assert(!SPLIT || (KEEP && K == 1));
     wait_prior_grid();
     const StageDev& sp = c.stages[s];
-    const int L = c.L, tpb = blockDim.x, nside = (L + tpb - 1) / tpb;
-    if (blockIdx.y < nside) {  // the rows' own work, tpb rows a CTA
-        const int r = blockIdx.y * tpb + threadIdx.x;
+    const int L = c.L, nthr = blockDim.x, nside = (L + nthr - 1) / nthr;
+    const int tpb = SPLIT ? 64 : nthr, tid = SPLIT ? threadIdx.x & 63 : threadIdx.x;  // target of the CTA
+    const bool half0 = !SPLIT || threadIdx.x < 64, half1 = !SPLIT || threadIdx.x >= 64;
+    if (blockIdx.y < nside) {  // the rows' own work, a row a thread
+        const int r = blockIdx.y * nthr + threadIdx.x;
         if (blockIdx.x == 0 && r < L) side_row(c, sp, r);
         return;
     }
@@ -120,7 +128,8 @@ __global__ void __launch_bounds__(64) k_main(const DevCtx c, const int s) {
     const double t = sp.T;
     const bool live = t > 0.0;
     extern __shared__ double2 s_last[];
-    __shared__ double s_red[2][6];
+    __shared__ double s_red[SPLIT ? 4 : 2][6];
+    __shared__ double2 s_a2[SPLIT ? 64 : 1];
     __shared__ int s_X[KEEP ? 64 * K : 1];
     __shared__ unsigned short s_job[KEEP ? 4 * 64 * K : 1];  // (local target << 2) | sum
     __shared__ int s_njob;
@@ -128,7 +137,7 @@ __global__ void __launch_bounds__(64) k_main(const DevCtx c, const int s) {
     double* s_logR = reinterpret_cast<double*>(s_last + L);  // LOGR only: [L]
 
     const double2* KRl = c.KR + (size_t)(nrows - 1) * L;
-    for (int k = threadIdx.x; k < L; k += tpb) {
+    for (int k = threadIdx.x; k < L; k += nthr) {
         const double2 v = KRl[k];
         s_last[k] = v;
         if constexpr (LOGR) s_logR[k] = v.y > 0.0 ? log(v.y) : v.y;
@@ -153,9 +162,10 @@ __global__ void __launch_bounds__(64) k_main(const DevCtx c, const int s) {
     // ---- positions of the targets in the history: row X, offset x in its interval
     int X[K];
     double x[K];
+    if (half0) {
 #pragma unroll
     for (int kk = 0; kk < K; ++kk) {
-        const int j = blockIdx.x * tpb * K + kk * tpb + threadIdx.x;
+        const int j = blockIdx.x * tpb * K + kk * tpb + tid;
         const size_t ij = (size_t)i * L + j;
         X[kk] = 1;
         x[kk] = 0.0;
@@ -185,7 +195,7 @@ __global__ void __launch_bounds__(64) k_main(const DevCtx c, const int s) {
             }
             if constexpr (KEEP) {
                 need = b2_need(X[kk], key, dirty, X[kk] < nrows - 1);
-                s_X[kk * tpb + threadIdx.x] = X[kk];
+                s_X[kk * tpb + tid] = X[kk];
                 if (X[kk] != key) c.b2key[ij] = X[kk];
             }
         }
@@ -205,16 +215,47 @@ __global__ void __launch_bounds__(64) k_main(const DevCtx c, const int s) {
                 base = __shfl_sync(0xffffffffu, base, 0);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    if (need >> q & 1) s_job[base + __popc(b[q] & lt)] = (unsigned short)((kk * tpb + threadIdx.x) << 2 | q);
+                    if (need >> q & 1) s_job[base + __popc(b[q] & lt)] = (unsigned short)((kk * tpb + tid) << 2 | q);
                     base += __popc(b[q]);
                 }
             }
         }
     }
+    }
+    // the stencils of the last row and B1 of a target
+    const double bc0 = r1.c0, bc1 = r1.c1, bc2 = r1.c2, bc3 = r1.c3;
+    const int F = r1.F, cubic1 = r1.cubic;
+    const auto gather_a = [&](const size_t ij, const int j, double2& a1, double2& a2, double2& b1) {
+        if constexpr (LOGR) {
+            const int ia1 = __ldg(c.iA1 + ij), ia2 = __ldg(c.iA2 + ij);
+            a1 = dot2s_log<M>(c.wA1 + ij * m, s_last + ia1, s_logR + ia1, m);
+            a2 = dot2s_log<M>(c.wA2 + ij * m, s_last + ia2, s_logR + ia2, m);
+        } else {
+            a1 = dot2s<M>(c.wA1 + ij * m, s_last + __ldg(c.iA1 + ij), m);
+            a2 = dot2s<M>(c.wA2 + ij * m, s_last + __ldg(c.iA2 + ij), m);
+        }
+        const double2 x0 = __ldg(c.KR + (size_t)(F - 1) * L + j);
+        const double2 x1 = __ldg(c.KR + (size_t)F * L + j);
+        const double2 d1 = __ldg(c.dKR + (size_t)F * L + j);
+        b1.x = bc0 * x0.x + bc1 * x1.x - bc2 * d1.x;
+        b1.y = bc0 * x0.y + bc1 * x1.y - bc2 * d1.y;
+        double2 d2 = make_double2(0.0, 0.0);
+        if (cubic1) {
+            d2 = __ldg(c.dKR + (size_t)(F + 1) * L + j);
+            b1.x -= bc3 * d2.x;
+            b1.y -= bc3 * d2.y;
+        }
+        if constexpr (LOGR) b1.y = b1_log(bc0, bc1, bc2, cubic1 ? bc3 : 0.0, x0.y, x1.y, d1.y, d2.y, b1.y);
+    };
+    [[maybe_unused]] double2 sa1, sb1;
+    if constexpr (SPLIT) {
+        const int j = blockIdx.x * tpb + tid;
+        if (half1 && live && j < L) gather_a((size_t)i * L + j, j, sa1, s_a2[tid], sb1);
+    }
     if constexpr (KEEP) {
         __syncthreads();
         const int nj = s_njob;
-        for (int q = threadIdx.x; q < nj; q += tpb) {
+        for (int q = threadIdx.x; q < nj; q += nthr) {
             const int job = s_job[q], tl = job >> 2, which = job & 3;
             const size_t ij = (size_t)i * L + blockIdx.x * tpb * K + tl;
             c.b2s[which * L2 + ij] = b2_sum<M>(c, ij, s_X[tl], which, m);
@@ -222,42 +263,25 @@ __global__ void __launch_bounds__(64) k_main(const DevCtx c, const int s) {
         __syncthreads();
     }
 
-    const double bc0 = r1.c0, bc1 = r1.c1, bc2 = r1.c2, bc3 = r1.c3;
-    const int F = r1.F, cubic1 = r1.cubic;
     double acc[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) acc[k] = 0.0;
 
 #pragma unroll
     for (int kk = 0; kk < K; ++kk) {
-        const int j = blockIdx.x * tpb * K + kk * tpb + threadIdx.x;
+        const int j = blockIdx.x * tpb * K + kk * tpb + tid;
         if (j < L) {
             const size_t ij = (size_t)i * L + j;
             double2 a1, a2, b1, b2;
             if (live) {
-                if constexpr (LOGR) {
-                    const int ia1 = __ldg(c.iA1 + ij), ia2 = __ldg(c.iA2 + ij);
-                    a1 = dot2s_log<M>(c.wA1 + ij * m, s_last + ia1, s_logR + ia1, m);
-                    a2 = dot2s_log<M>(c.wA2 + ij * m, s_last + ia2, s_logR + ia2, m);
+                if constexpr (!SPLIT) {
+                    gather_a(ij, j, a1, a2, b1);
                 } else {
-                    a1 = dot2s<M>(c.wA1 + ij * m, s_last + __ldg(c.iA1 + ij), m);
-                    a2 = dot2s<M>(c.wA2 + ij * m, s_last + __ldg(c.iA2 + ij), m);
+                    a1 = sa1;
+                    b1 = sb1;
+                    a2 = s_a2[tid];
                 }
-                {
-                    const double2 x0 = __ldg(c.KR + (size_t)(F - 1) * L + j);
-                    const double2 x1 = __ldg(c.KR + (size_t)F * L + j);
-                    const double2 d1 = __ldg(c.dKR + (size_t)F * L + j);
-                    b1.x = bc0 * x0.x + bc1 * x1.x - bc2 * d1.x;
-                    b1.y = bc0 * x0.y + bc1 * x1.y - bc2 * d1.y;
-                    double2 d2 = make_double2(0.0, 0.0);
-                    if (cubic1) {
-                        d2 = __ldg(c.dKR + (size_t)(F + 1) * L + j);
-                        b1.x -= bc3 * d2.x;
-                        b1.y -= bc3 * d2.y;
-                    }
-                    if constexpr (LOGR) b1.y = b1_log(bc0, bc1, bc2, cubic1 ? bc3 : 0.0, x0.y, x1.y, d1.y, d2.y, b1.y);
-                }
-                {
+                if (half0) {
                     const bool cubic2 = X[kk] < nrows - 1;
                     const double x1 = x[kk], x2 = x1 * x1;
                     double2 S0, S1, D1, D2 = make_double2(0.0, 0.0);
@@ -288,25 +312,35 @@ __global__ void __launch_bounds__(64) k_main(const DevCtx c, const int s) {
                         if (LOGR && S0.y > 0.0 && S1.y > 0.0)  // index_mat.cu:216-222
                             b2.y = exp(e0 * log(S0.y) + x2 * log(S1.y) + e2 * (D1.y / S0.y));
                     }
-                    if (c.rec) c.rec[ij] = GatherRec{a1, a2, b1, b2, x1, X[kk], 0};
+                    if (c.rec) {
+                        GatherRec* g = c.rec + ij;
+                        if (!SPLIT) *g = GatherRec{a1, a2, b1, b2, x1, X[kk], 0};
+                        else { g->a2 = a2; g->b2 = b2; g->x = x1; g->X = X[kk]; }
+                    }
                 }
+                if (SPLIT && half1 && c.rec) { c.rec[ij].a1 = a1; c.rec[ij].b1 = b1; }
             } else {
                 a1 = a2 = b1 = b2 = fill;
             }
-            double sKA1, dA1, sKB1, dB1, sKB2, dB2;
-            SigT<P, P2>::d12(Mo, a1.x, sKA1, dA1);
-            SigT<P, P2>::d12(Mo, b1.x, sKB1, dB1);
-            SigT<P, P2>::d12(Mo, b2.x, sKB2, dB2);
             const double wj = __ldg(c.integ + j);
-            const double wQRA2 = wj * a2.y, wRA2 = wQRA2 * SigT<P, P2>::d2(Mo, a2.x);
-            acc[0] = fma(wRA2, b2.x, acc[0]);            // ConvR(SigmaRA2, QKB2)
-            // ConvA(SigmaRA1, QKB1) + ConvA(SigmaKA1, QRB1)
-            acc[1] = fma(wj, fma(sKA1, b1.y, (dA1 * a1.y) * b1.x), acc[1]);
-            acc[2] = fma(wQRA2, sKB2, acc[2]);           // ConvR(QRA2, SigmaKB2)
-            // ConvA(QRA1, SigmaKB1) + ConvA(QKA1, SigmaRB1)
-            acc[3] = fma(wj, fma(a1.x, dB1 * b1.y, a1.y * sKB1), acc[3]);
-            acc[4] = fma(wRA2, b2.y, acc[4]);            // ConvR(SigmaRA2, QRB2)
-            acc[5] = fma(wQRA2, dB2 * b2.y, acc[5]);     // ConvR(QRA2, SigmaRB2)
+            if (half1) {
+                double sKA1, dA1, sKB1, dB1;
+                SigT<P, P2>::d12(Mo, a1.x, sKA1, dA1);
+                SigT<P, P2>::d12(Mo, b1.x, sKB1, dB1);
+                // ConvA(SigmaRA1, QKB1) + ConvA(SigmaKA1, QRB1)
+                acc[1] = fma(wj, fma(sKA1, b1.y, (dA1 * a1.y) * b1.x), acc[1]);
+                // ConvA(QRA1, SigmaKB1) + ConvA(QKA1, SigmaRB1)
+                acc[3] = fma(wj, fma(a1.x, dB1 * b1.y, a1.y * sKB1), acc[3]);
+            }
+            if (half0) {
+                double sKB2, dB2;
+                SigT<P, P2>::d12(Mo, b2.x, sKB2, dB2);
+                const double wQRA2 = wj * a2.y, wRA2 = wQRA2 * SigT<P, P2>::d2(Mo, a2.x);
+                acc[0] = fma(wRA2, b2.x, acc[0]);            // ConvR(SigmaRA2, QKB2)
+                acc[2] = fma(wQRA2, sKB2, acc[2]);           // ConvR(QRA2, SigmaKB2)
+                acc[4] = fma(wRA2, b2.y, acc[4]);            // ConvR(SigmaRA2, QRB2)
+                acc[5] = fma(wQRA2, dB2 * b2.y, acc[5]);     // ConvR(QRA2, SigmaRB2)
+            }
         }
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -316,7 +350,7 @@ __global__ void __launch_bounds__(64) k_main(const DevCtx c, const int s) {
     __syncthreads();
     if (threadIdx.x < 6) {
         double v = 0.0;
-        for (int w = 0; w < (tpb >> 5); ++w) v += s_red[w][threadIdx.x];
+        for (int w = 0; w < (nthr >> 5); ++w) v += s_red[w][threadIdx.x];
         c.part[((size_t)blockIdx.x * 6 + threadIdx.x) * L + i] = v;
     }
 }
@@ -850,18 +884,25 @@ __global__ void k_fp64_probe(double* out, int iters) {
 
 // ------------------------------------------------------------------------
 // launch wrappers
-template <int M, int K, int P, int P2, bool LOGR, bool KEEP>
+template <int M, int K, int P, int P2, bool LOGR, bool KEEP, bool SPLIT = false>
 static cudaError_t launch_main_t(const DevCtx& c, int s, cudaStream_t st) {
-    dim3 grid(c.nch, c.L + (c.L + c.tpb - 1) / c.tpb), block(c.tpb);
+    const int nthr = SPLIT ? 128 : c.tpb;
+    dim3 grid(c.nch, c.L + (c.L + nthr - 1) / nthr), block(nthr);
     const size_t smem = (size_t)c.L * (LOGR ? sizeof(double2) + sizeof(double) : sizeof(double2));
     static std::atomic<unsigned long long> devs{0};
-    const cudaError_t e = raise_smem_limit(k_main<M, K, P, P2, LOGR, KEEP>, smem, 4096 * (int)(smem / c.L), devs);
+    const cudaError_t e = raise_smem_limit(k_main<M, K, P, P2, LOGR, KEEP, SPLIT>, smem, 4096 * (int)(smem / c.L), devs);
     if (e != cudaSuccess) return e;
-    return launch_pdl(k_main<M, K, P, P2, LOGR, KEEP>, grid, block, smem, st, c, s);
+    return launch_pdl(k_main<M, K, P, P2, LOGR, KEEP, SPLIT>, grid, block, smem, st, c, s);
 }
+
+// Lengths up to which k_main takes two threads a target (RK54 step, one thread a target -> two:
+// L = 64 166 -> 142 us, 128 172 -> 154, 192 198 -> 191, 224 230 -> 231, 320 325 -> 330): beyond
+// 192 a row has four chunks and its warps fill the schedulers by themselves.
+constexpr int SPLIT_L = 192;
 
 template <int M, int P, int P2, bool LOGR>
 static cudaError_t launch_main_kl(const DevCtx& c, int s, cudaStream_t st) {
+    if (c.b2key && c.kpt == 1 && c.tpb == 64 && c.L <= SPLIT_L) return launch_main_t<M, 1, P, P2, LOGR, true, true>(c, s, st);
     if (c.b2key) return c.kpt == 1 ? launch_main_t<M, 1, P, P2, LOGR, true>(c, s, st)
                                    : launch_main_t<M, 2, P, P2, LOGR, true>(c, s, st);
     switch (c.kpt) {

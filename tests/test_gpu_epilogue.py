@@ -34,6 +34,27 @@ def test_rows_at_block_edges(product_built, oracle_built, L, method):
     s.close()
 
 
+@pytest.mark.parametrize("L,Tmax", [(63, 10.0), (65, 100.0), (129, 1e3), (192, 1e5), (193, 1e5)])
+def test_two_threads_a_target(product_built, oracle_built, L, Tmax):
+    """The gathers' two threads a target: chunk edges and both sides of the length where one
+    thread takes a target again."""
+    grid = D.grid.generate(L, Tmax=Tmax)
+    s = D.Simulation(grid, D.Model(p=3, p2=4, lam=0.5, Gamma=0.6))
+    s.init()
+    sched = (1e-4 * 1.3 ** np.arange(5), np.array([1, 1, 2, 1, 4], dtype=np.int32))
+    tr = s.run(5, schedule=sched)
+    og = O.Grid(L, grid.theta, grid.phi1, grid.phi2, grid.integ, grid.indsA1, grid.wA1, grid.indsA2, grid.wA2,
+                grid.indsB2, grid.wB2)
+    p = O.Port(og, O.Model(p=3, p2=4, lam=0.5, Gamma=0.6), search_mode=1, threads=0)
+    p.init_state()
+    tp = p.run(5, schedule=sched)
+    a, b = s.download(), p.get_state()
+    for k in ("QK", "QR", "rvec"):
+        assert rel_err(getattr(a, k), getattr(b, k)) < TRAJ_TOL, k
+    assert rel_err(tr["energy"], tp["energy"]) < TRAJ_TOL
+    s.close()
+
+
 # a short list, one whose intervals a step leaves by several at once, and an even one
 @pytest.mark.parametrize("L,Tmax,n,factor", [(33, 10.0, 2, 1.0), (64, 100.0, 20, 1.5), (257, 1e5, 24, 1.0),
                                              (512, 1e5, 40, 1.2)])
