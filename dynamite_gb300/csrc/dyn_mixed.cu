@@ -87,8 +87,10 @@ cudaError_t launch_t(const DevCtx& c, int s, cudaStream_t st) {
 
 template <int P, int P2>
 cudaError_t launch_pp(const DevCtx& c, int s, cudaStream_t st) {
-    // the depth-10 kernels read the staged row in element pairs: they need an even L
-    const bool ten = c.m == 10 && c.L % 2 == 0;
+    // the depth-10 plain form reads the staged row in element pairs, which pays where whole rows
+    // keep one parity (RK54 step at the odd L = 257: 144 us, the generic depth 141; the (hi, lo)
+    // form 153 against 171 at L = 257, 281 against 321 at 513)
+    const bool ten = c.m == 10 && (c.mixed == 2 || c.L % 2 == 0);
     if (c.b2key) return ten ? launch_t<10, P, P2, true>(c, s, st) : launch_t<0, P, P2, true>(c, s, st);
     return ten ? launch_t<10, P, P2, false>(c, s, st) : launch_t<0, P, P2, false>(c, s, st);
 }

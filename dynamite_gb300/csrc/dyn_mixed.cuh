@@ -191,10 +191,9 @@ __device__ __forceinline__ void shift_offset(float& h, float& l, float s) {
     l = __fsub_rn(e, __fsub_rn(h, t));
 }
 
-// The same for the four segments of one target's B2 sums in turn (rows of an even length L, so
-// every start has the same parity): each read as six 16-byte loads from the even element at or
-// below the start, every tap selecting its element.  Reads up to two elements past a segment
-// and uses none of them.
+// The same for a segment of the history (start b in the whole array): read as six 16-byte loads
+// from the even element at or below the start, every tap selecting its element.  Reads up to
+// two elements past a segment and uses none of them.
 __device__ __forceinline__ float2 seg10(const float w[10], const float2* __restrict__ arr, size_t b) {
     const float4* p = reinterpret_cast<const float4*>(arr + (b & ~(size_t)1));
     const bool sh = b & 1;
