@@ -195,7 +195,7 @@ struct Ctx {
         const bool df = d.mixed == 2;
         if (cudaMalloc((void**)&d.b2key, L2 * sizeof(int)) == cudaSuccess &&
             (d.mixed ? cudaMalloc((void**)&d.b2f, (df ? 2 : 4) * L2 * sizeof(float2))
-                     : cudaMalloc((void**)&d.b2s, 4 * L2 * sizeof(double2))) == cudaSuccess &&
+                     : cudaMalloc((void**)&d.b2s, (d.logr ? 5 : 4) * L2 * sizeof(double2))) == cudaSuccess &&
             (!df || cudaMalloc((void**)&d.b2q, 2 * L2 * sizeof(float4)) == cudaSuccess))
             return;
         cudaGetLastError();

@@ -258,7 +258,9 @@ __global__ void __launch_bounds__(SPLIT ? 128 : 64) k_main(const DevCtx c, const
         for (int q = threadIdx.x; q < nj; q += nthr) {
             const int job = s_job[q], tl = job >> 2, which = job & 3;
             const size_t ij = (size_t)i * L + blockIdx.x * tpb * K + tl;
-            c.b2s[which * L2 + ij] = b2_sum<M>(c, ij, s_X[tl], which, m);
+            const double2 v = b2_sum<M>(c, ij, s_X[tl], which, m);
+            c.b2s[which * L2 + ij] = v;
+            if (LOGR && which < 2 && v.y > 0.0) reinterpret_cast<double*>(c.b2s + 4 * L2)[which * L2 + ij] = log(v.y);
         }
         __syncthreads();
     }
@@ -296,21 +298,27 @@ __global__ void __launch_bounds__(SPLIT ? 128 : 64) k_main(const DevCtx c, const
                         D1 = b2_sum<M>(c, ij, X[kk], 2, m);
                         if (cubic2) D2 = b2_sum<M>(c, ij, X[kk], 3, m);
                     }
+                    // index_mat.cu:203-222: Hermite of log of the row sums; the logs are kept beside
+                    // the sums (L = 519, 3400 rows: RK54 step 2.50 -> 2.39 ms)
+                    const bool logs = LOGR && S0.y > 0.0 && S1.y > 0.0;
+                    double l0 = 0.0, l1 = 0.0;
+                    if (logs) {
+                        const double* b2l = reinterpret_cast<const double*>(c.b2s + 4 * L2);
+                        l0 = KEEP ? b2l[ij] : log(S0.y);
+                        l1 = KEEP ? b2l[L2 + ij] : log(S1.y);
+                    }
                     if (cubic2) {
                         // Hermite weights through y = x^3 - x^2: e1 = x - x^2 + y, e2 = x^2 - 2 y, e0 = 1 - e2
                         const double y = fma(x2, x1, -x2), e1 = (x1 - x2) + y, e2 = fma(-2.0, y, x2), e0 = 1.0 - e2;
                         const double e3 = y * c.inv_dtr[X[kk] + 1];
                         b2.x = fma(e3, D2.x, fma(e2, S1.x, fma(e1, D1.x, e0 * S0.x)));
                         b2.y = fma(e3, D2.y, fma(e2, S1.y, fma(e1, D1.y, e0 * S0.y)));
-                        // index_mat.cu:203-212: Hermite of log of the row sums
-                        if (LOGR && S0.y > 0.0 && S1.y > 0.0)
-                            b2.y = exp(e0 * log(S0.y) + e1 * (D1.y / S0.y) + e2 * log(S1.y) + e3 * (D2.y / S1.y));
+                        if (logs) b2.y = exp(e0 * l0 + e1 * (D1.y / S0.y) + e2 * l1 + e3 * (D2.y / S1.y));
                     } else {
                         const double e0 = 1.0 - x2, e2 = x1 - x2;
                         b2.x = fma(e2, D1.x, fma(x2, S1.x, e0 * S0.x));
                         b2.y = fma(e2, D1.y, fma(x2, S1.y, e0 * S0.y));
-                        if (LOGR && S0.y > 0.0 && S1.y > 0.0)  // index_mat.cu:216-222
-                            b2.y = exp(e0 * log(S0.y) + x2 * log(S1.y) + e2 * (D1.y / S0.y));
+                        if (logs) b2.y = exp(e0 * l0 + x2 * l1 + e2 * (D1.y / S0.y));
                     }
                     if (c.rec) {
                         GatherRec* g = c.rec + ij;

@@ -104,7 +104,7 @@ struct DevCtx {
     double* posB2x_saved;  // [NSAVE][L*L]
     double* inv_len;       // [cap] 1/(t1grid[k+1]-t1grid[k]) (FP64 contexts)
     int* b2key;            // [L*L] row X whose B2 sums the planes hold (null: none kept)
-    double2* b2s;          // [4][L*L] S0, S1, D1, D2 (FP64 form)
+    double2* b2s;          // [4][L*L] S0, S1, D1, D2 (FP64 form); log-space response: then log S0, log S1 of R, [2][L*L] double
     float2* b2f;           // [4][L*L] S0, S1, D1, D2 (mixed 1); [2][L*L] D1, D2 (mixed 2)
     float4* b2q;           // [2][L*L] S0, S1 as (QK hi, lo, QR hi, lo) (mixed 2)
     double2* h;            // [SMAX][L]
