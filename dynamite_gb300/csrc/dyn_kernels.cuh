@@ -234,12 +234,15 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-// Dynamic shared memory above the 48 KB default needs the kernel's
-// MaxDynamicSharedMemorySize attribute, which is per device: raise it to
+// Shared memory above the 48 KB default, dynamic and static together, needs the
+// kernel's MaxDynamicSharedMemorySize attribute, which is per device: raise it to
 // `limit` once per (kernel, device); `devs` is the caller's per-kernel record.
+// SMEM_STATIC: more than any stage kernel's static part (4.3 KB), with which the
+// limit is raised a few lengths early; that costs nothing but the call.
+constexpr size_t SMEM_STATIC = 8 * 1024;
 template <typename Kern>
 inline cudaError_t raise_smem_limit(Kern kern, size_t bytes, int limit, std::atomic<unsigned long long>& devs) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
+    if (bytes + SMEM_STATIC <= 48 * 1024) return cudaSuccess;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;

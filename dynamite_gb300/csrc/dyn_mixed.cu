@@ -78,7 +78,7 @@ cudaError_t launch_t(const DevCtx& c, int s, cudaStream_t st) {
     if (c.mixed == 2) {
         const size_t smem = (size_t)c.L * sizeof(float4);  // with the static part > 48 KB from L = 2700 on
         static std::atomic<unsigned long long> devs{0};
-        const cudaError_t e = raise_smem_limit(k_main_df<M, P, P2, KEEP>, smem + 6 * 1024, 4096 * (int)sizeof(float4), devs);
+        const cudaError_t e = raise_smem_limit(k_main_df<M, P, P2, KEEP>, smem, 4096 * (int)sizeof(float4), devs);
         if (e != cudaSuccess) return e;
         return launch_pdl(k_main_df<M, P, P2, KEEP>, grid, dim3(TPB_M), smem, st, c, s);
     }
