@@ -178,6 +178,14 @@ __device__ __noinline__ inline double search_pos_cold(int mode, const double* p,
     return search_pos(mode, L, El);
 }
 
+// Whether El, with floor_index k and list[k] = tk, lies where a search does not simply give the
+// offset in interval k: before a list that starts after 0 or on its first entry, where the
+// position stays bounded, or on a value that the list holds more than once.
+__device__ __forceinline__ bool off_interval(const ListView& L, double El, int k, double tk) {
+    const long long kE = okey(El), kt = okey(tk);
+    return kt >= kE && (kt > kE || (k == 0 ? kE != 0 : okey(L.at(k - 1)) == kE));
+}
+
 // search_pos for an element whose interval is near a guess (0-based lower end; two loads
 // instead of a search where it holds).  Same bits as search_pos: which end of the interval its
 // position starts from depends on the last probe of the search, so the probes are replayed on

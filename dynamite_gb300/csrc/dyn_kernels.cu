@@ -172,26 +172,34 @@ __global__ void __launch_bounds__(SPLIT ? 128 : 64) k_main(const DevCtx c, const
         int need = 0;
         if (live && j < L) {
             const int key = keep ? c.b2key[ij] : 0;
-            if (pos2_src || sp.kind == KIND_RHS) {
-                const double pos2 = pos2_src ? pos2_src[ij] : search_pos(c.search, lv, __dmul_rn(__ldg(c.phi2 + ij), t));
+            // position as the reference gives it, clamped to the rows there are
+            const auto at_position = [&](const double pos2) {
                 long long Xl = (long long)pos2;
                 if (Xl > maxX) Xl = maxX;
                 if (Xl < 1) Xl = 1;
                 X[kk] = (int)Xl;
                 x[kk] = __dsub_rn(pos2, (double)Xl);
                 if (pos2_dst) pos2_dst[ij] = pos2;
+            };
+            if (pos2_src || sp.kind == KIND_RHS) {
+                at_position(pos2_src ? pos2_src[ij] : search_pos(c.search, lv, __dmul_rn(__ldg(c.phi2 + ij), t)));
             } else {
                 const double El = __dmul_rn(__ldg(c.phi2 + ij), t);
                 const int k = key > 0 ? floor_index_near(lv, El, min(key, nrows) - 1) : floor_index(lv, El, 0, nrows - 1);
-                if (k >= nrows - 1) {
-                    X[kk] = nrows;
+                const double tk = lv.at(k);
+                if (off_interval(lv, El, k, tk)) {
+                    at_position(search_pos_cold(c.search, lv.p, lv.n, lv.vlast, El));
                 } else {
-                    x[kk] = __dmul_rn(__dsub_rn(El, lv.at(k)), __ldg(c.inv_len + k));
-                    X[kk] = k + 1;
+                    if (k >= nrows - 1) {
+                        X[kk] = nrows;
+                    } else {
+                        x[kk] = okey(tk) == okey(El) ? 0.0 : __dmul_rn(__dsub_rn(El, tk), __ldg(c.inv_len + k));
+                        X[kk] = k + 1;
+                    }
+                    if (pos2_dst) pos2_dst[ij] = (double)X[kk] + x[kk];
+                    if (X[kk] > maxX) { x[kk] += (double)(X[kk] - maxX); X[kk] = maxX; }
+                    if (X[kk] < 1) { x[kk] -= (double)(1 - X[kk]); X[kk] = 1; }
                 }
-                if (pos2_dst) pos2_dst[ij] = (double)X[kk] + x[kk];
-                if (X[kk] > maxX) { x[kk] += (double)(X[kk] - maxX); X[kk] = maxX; }
-                if (X[kk] < 1) { x[kk] -= (double)(1 - X[kk]); X[kk] = 1; }
             }
             if constexpr (KEEP) {
                 need = b2_need(X[kk], key, dirty, X[kk] < nrows - 1);
