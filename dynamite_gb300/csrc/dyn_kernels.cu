@@ -1046,9 +1046,9 @@ cudaError_t launch_sparsify_flags(const DevCtx& c, int n, int variant, double th
 // order without reaching rows still to be read.
 cudaError_t launch_compact(const DevCtx& c, const int* inds, const int* indsD, const double* tfac, int k,
                            const CompactBuf& buf, cudaStream_t st) {
-    const size_t L = c.L;
-    for (size_t r0 = 0; r0 < (size_t)k; r0 += buf.rows) {
-        const size_t rows = std::min(buf.rows, (size_t)k - r0), total = rows * L;
+    const size_t L = c.L, per = buf.elems / L;  // rows staged at a time
+    for (size_t r0 = 0; r0 < (size_t)k; r0 += per) {
+        const size_t rows = std::min(per, (size_t)k - r0), total = rows * L;
         const int blocks = (int)((total + 255) / 256 < 8192 ? (total + 255) / 256 : 8192);
         k_compact<<<blocks, 256, 0, st>>>(c, inds, indsD, tfac, (int)r0, (int)rows, buf.KR, buf.dKR, buf.r, buf.dr);
         cudaError_t e = cudaGetLastError();
@@ -1065,31 +1065,29 @@ cudaError_t launch_compact(const DevCtx& c, const int* inds, const int* indsD, c
 }
 
 cudaError_t CompactBuf::reserve(size_t n, size_t L) {
-    // flags and index lists of n rows; staging of at most 64 MB
     if (n > cap) {
-        cudaFree(flags); cudaFree(idx); cudaFree(tf);
-        flags = nullptr; idx = nullptr; tf = nullptr;
+        for (void* p : {(void*)flags, (void*)idx, (void*)tf, (void*)r, (void*)dr}) cudaFree(p);
+        flags = nullptr;
+        idx = nullptr;
+        tf = r = dr = nullptr;
         cap = 0;
         cudaError_t e = cudaMalloc((void**)&flags, n);
         if (e == cudaSuccess) e = cudaMalloc((void**)&idx, 2 * n * sizeof(int));
-        if (e == cudaSuccess) e = cudaMalloc((void**)&tf, n * sizeof(double));
+        for (double** p : {&tf, &r, &dr})
+            if (e == cudaSuccess) e = cudaMalloc((void**)p, n * sizeof(double));
         if (e != cudaSuccess) return e;
         cap = n;
     }
-    const size_t want = std::min(n, std::max<size_t>(1, (64u << 20) / (2 * L * sizeof(double2))));
-    if (want > rows || L > len) {
-        cudaFree(KR); cudaFree(dKR); cudaFree(r); cudaFree(dr);
+    // counted in elements, so that rows of any length share the bound
+    const size_t want = std::min(n * L, (64u << 20) / (2 * sizeof(double2)));
+    if (want > elems) {
+        cudaFree(KR); cudaFree(dKR);
         KR = dKR = nullptr;
-        r = dr = nullptr;
-        rows = 0;
-        const size_t l = std::max(L, len), w = std::max(want, rows);
-        cudaError_t e = cudaMalloc((void**)&KR, w * l * sizeof(double2));
-        if (e == cudaSuccess) e = cudaMalloc((void**)&dKR, w * l * sizeof(double2));
-        if (e == cudaSuccess) e = cudaMalloc((void**)&r, w * sizeof(double));
-        if (e == cudaSuccess) e = cudaMalloc((void**)&dr, w * sizeof(double));
+        elems = 0;
+        cudaError_t e = cudaMalloc((void**)&KR, want * sizeof(double2));
+        if (e == cudaSuccess) e = cudaMalloc((void**)&dKR, want * sizeof(double2));
         if (e != cudaSuccess) return e;
-        rows = w;
-        len = l;
+        elems = want;
     }
     return cudaSuccess;
 }

@@ -291,16 +291,16 @@ cudaError_t launch_search(const DevCtx& c, const double* list, size_t nlist, con
                           size_t nelem, double* out, cudaStream_t st);
 cudaError_t launch_sparsify_flags(const DevCtx& c, int nrows, int variant, double threshold,
                                   unsigned char* flags, cudaStream_t st);
-// Workspace of sparsify passes, kept by its context or batch from the first one on: node flags
-// and index lists for `cap` rows, staging for `rows` rows of length `len` (at most 64 MB)
+// Workspace of sparsify passes, kept by its context or batch from the first one on: node flags,
+// index lists and staged scalars for `cap` rows, staging for `elems` history elements of rows of
+// any length (at most 64 MB; at least one row, of at most 4096)
 struct CompactBuf {
     unsigned char* flags = nullptr;
     int* idx = nullptr;  // [2 cap]
-    double* tf = nullptr;
+    double *tf = nullptr, *r = nullptr, *dr = nullptr;
     size_t cap = 0;
     double2 *KR = nullptr, *dKR = nullptr;
-    double *r = nullptr, *dr = nullptr;
-    size_t rows = 0, len = 0;
+    size_t elems = 0;
     cudaError_t reserve(size_t n, size_t L);
     void release();
 };
