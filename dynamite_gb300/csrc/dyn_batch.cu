@@ -524,9 +524,11 @@ struct Batch {
         int nb = 0;
         const void* f = with_kernel(threads, targets, [](auto* kern) { return (const void*)kern; });
         // the (hi, lo) form stages Lmax float4: with its static part above 48 KB from Lmax = 2700
-        // on; the attribute is set here, before the tile's first launch and any graph capture
-        if (smem > 40 * 1024 &&
-            cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        // on.  The limit belongs to the kernel, not to this batch, so it goes to what the longest
+        // rows there are need: another live batch launches this kernel under it.  Set here,
+        // before the tile's first launch and any graph capture.
+        if (smem + SMEM_STATIC > 48 * 1024 &&
+            cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 4096 * (int)sizeof(float4)) != cudaSuccess)
             return 1;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, f, threads, smem) != cudaSuccess) return 1;
         nb = nb > 0 ? nb : 1;
