@@ -772,13 +772,13 @@ cudaError_t launch_adj_seed(const DevCtx& c, const AdjDev& a, const AdjModel& am
 
 // k_adj_lastrow's shared memory: row sums, the row's A1/A2 cotangents and
 // the column starts
-size_t lastrow_smem(int L, int) { return 3 * (size_t)L * sizeof(double2) + (size_t)(L + 1) * sizeof(int); }
+size_t lastrow_smem(int L) { return 3 * (size_t)L * sizeof(double2) + (size_t)(L + 1) * sizeof(int); }
 
 template <int P, int P2>
 cudaError_t launch_targets_pp(const DevCtx& c, const AdjDev& a, const AdjModel& am, int s,
                               cudaStream_t st) {
     const dim3 grid((c.L + 63) / 64, c.L);
-    const size_t lsm = lastrow_smem(c.L, c.m);
+    const size_t lsm = lastrow_smem(c.L);
     const size_t NP = (size_t)c.L * c.L;
     cudaError_t e = launch_pdl(c.m == 10 ? k_adj_targets<10, P, P2> : k_adj_targets<0, P, P2>, grid, dim3(64), 0, st, c, a, am, s);
     if (e != cudaSuccess) return e;
@@ -829,8 +829,9 @@ cudaError_t launch_adj_initial(const AdjDev& a, const AdjModel& am, cudaStream_t
     return cudaGetLastError();
 }
 
-cudaError_t adj_targets_smem_attr(int L, int m) {
-    return cudaFuncSetAttribute(k_adj_lastrow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lastrow_smem(L, m));
+// The limit belongs to the kernel, which other contexts launch too: what the longest rows need
+cudaError_t adj_lastrow_smem_attr() {
+    return cudaFuncSetAttribute(k_adj_lastrow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lastrow_smem(4096));
 }
 
 }  // namespace dyn

@@ -413,7 +413,7 @@ struct Ctx {
             release_adjoint();
             return s;
         }
-        CK(adj_targets_smem_attr(L, d.m));
+        CK(adj_lastrow_smem_attr());
         {
             // static orders of the transposed gathers (the tables never change)
             const size_t L2 = Lz * Lz;

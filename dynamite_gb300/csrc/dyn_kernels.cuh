@@ -339,6 +339,6 @@ cudaError_t launch_adj_step(const DevCtx& c, const AdjDev& a, const AdjModel& am
 cudaError_t launch_adj_initial(const AdjDev& a, const AdjModel& am, cudaStream_t st);
 cudaError_t launch_adj_verify(const DevCtx& c, const AdjDev& a, const double2* snapKR, const double2* snapdKR,
                               const double* snapr, const double* snapdr, int n0, cudaStream_t st);
-cudaError_t adj_targets_smem_attr(int L, int m);
+cudaError_t adj_lastrow_smem_attr();
 
 }  // namespace dyn

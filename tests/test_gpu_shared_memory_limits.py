@@ -1,5 +1,5 @@
-"""The shared-memory limit of a kernel belongs to the process: a second, shorter batch must
-leave the first one's launches as they were."""
+"""The shared-memory limit of a kernel belongs to the process: a second, shorter batch or adjoint
+context must leave the first one's launches as they were."""
 import numpy as np
 import pytest
 
@@ -28,3 +28,19 @@ def test_two_live_batches(product_built):
         np.testing.assert_array_equal(getattr(a, f)[: v.size], v, err_msg=f)
     for x in (first, second, s):
         x.close()
+
+
+def test_two_adjoint_contexts(product_built):
+    sims = []
+    for L, order in ((960, 1), (64, 9)):
+        s = D.Simulation(D.grid.generate(L, Tmax=1e5 if L > 64 else 100.0, interp_order=order), D.Model(**M))
+        s.init()
+        s.adjoint_forward(2, schedule=(np.full(2, 1e-3), np.ones(2, dtype=np.int32)))
+        sims.append(s)
+    first = sims[0].adjoint_backward(w_energy=1.0)[0]
+    sims[1].adjoint_backward(w_energy=1.0)
+    again, stats = sims[0].adjoint_backward(w_energy=1.0)
+    assert stats["recompute_mismatch"] == 0
+    np.testing.assert_allclose(again, first, rtol=1e-12)  # the additions' order is free
+    for s in sims:
+        s.close()
