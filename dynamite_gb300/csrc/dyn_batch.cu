@@ -255,10 +255,14 @@ __device__ void adapt_step(const Quench& q, Plan& pl, const TabDev& tb) {
 }
 
 // ------------------------------------------------------------------ kernels
-// TPB threads per CTA; the register cap keeps DYN_BATCH_TPSM (K = 1) or 512
-// (K = 2) threads resident per SM: the gathers are latency-bound.
+// TPB threads per CTA; the register cap keeps DYN_BATCH_TPSM (plain, depth 10),
+// DYN_BATCH_GEN_TPSM (plain, other depths), DYN_BATCH_DF_TPSM ((hi, lo)) or, with two targets
+// a thread, 512 threads resident per SM: the gathers are latency-bound.
 #ifndef DYN_BATCH_TPSM
-#define DYN_BATCH_TPSM 1152
+#define DYN_BATCH_TPSM 1280
+#endif
+#ifndef DYN_BATCH_GEN_TPSM
+#define DYN_BATCH_GEN_TPSM 1152
 #endif
 #ifndef DYN_BATCH_SHIFT
 #define DYN_BATCH_SHIFT 0
@@ -266,9 +270,10 @@ __device__ void adapt_step(const Quench& q, Plan& pl, const TabDev& tb) {
 #ifndef DYN_BATCH_DF_TPSM
 #define DYN_BATCH_DF_TPSM 1152
 #endif
-// 56 registers (1152 threads) measure best in both forms.  64 quenches, L = 512, 800 rows:
-// plain 0.71 ms (48 registers 0.81, spilling; 64: 0.70, but slower on short rows, L = 256
-// 63 us against 61), (hi, lo) with its sums kept 1.06 ms (64: 1.09, 72: 1.11).
+// 48 registers (1280 threads) hold the depth-10 plain form without spills, 56 (1152) the
+// generic depth.  Gather of 48 / 56: 64 quenches at L = 256 204 / 216 us, 16 at 512 196 / 199,
+// 64 at 512 703 / 712, 16 at 1024 950 / 992; order 5, 32 at 256 131 / 119, order 11, 32 at 512
+// 637 / 577.  (hi, lo) with its sums kept, 64 at 512: 56 registers 1.06 ms, 64 1.09, 72 1.11.
 //
 // DF: the (hi, lo) form (mdf::chunk_dd).  Bound by issue slots and the latency of its loads:
 // ~1,300 instructions per 32 targets, of which the compensated A1/A2 sums are ~40 %.
@@ -298,7 +303,7 @@ __device__ __forceinline__ void fetch_item(const Quench* Q, const Plan* PL, cons
 // plan says whether its planes go on from the previous stage; 1, 2: measurement, all fill /
 // all keep.
 template <int M, int K, int P, int P2, int TPB, bool DF, bool KEEP>
-__global__ void __launch_bounds__(TPB, DF ? DYN_BATCH_DF_TPSM / TPB : (K == 1 ? DYN_BATCH_TPSM : 512) / TPB)
+__global__ void __launch_bounds__(TPB, (DF ? DYN_BATCH_DF_TPSM : K > 1 ? 512 : M == 10 ? DYN_BATCH_TPSM : DYN_BATCH_GEN_TPSM) / TPB)
     k_batch_gather(const Quench* __restrict__ Q, const Plan* __restrict__ PL, const unsigned* __restrict__ items,
                    const unsigned nitems, Work* work, const int force) {
     wait_prior_grid();

@@ -580,27 +580,40 @@ __device__ __forceinline__ void chunk_sums(const DevCtx& c, const StageDev& sp, 
 }
 
 // After a __syncthreads() that follows the chunks of slots 0..ng-1 (chunks ch0..ch0+ng-1):
-// the block's six sums of each chunk into part[ch][0..6)[i], warps added in order.  The plain
-// form's eight (DF false) are paired here: the two ConvA sums that share their factor.
+// the block's six sums of each chunk into part[ch][0..6)[i], warps added in order, compensated
+// on the high parts, one conversion at the end.  (hi, lo) form: eight lanes a chunk, two idle,
+// in whole warps (a loop bounded by ng measured 1.3 % slower over mixed lengths).  The plain
+// form's eight are paired here, the two ConvA sums that share their factor, by the thread that
+// stores them: pairing across lanes kept so much alive through the batch's loop that it spilled
+// at 48 registers (16 quenches at L = 1024: 1005 us a gather at 56, now 950).
 template <bool DF>
 __device__ __forceinline__ void fold_chunks(const DevCtx& c, const int i, const int ch0, const int ng, const RowShared& sh) {
-    const int nw = blockDim.x >> 5, k = threadIdx.x & 7;
-    for (int g = threadIdx.x >> 3; g < ((ng + 3) & ~3); g += blockDim.x >> 3) {  // whole warps
-        // warps in order, compensated on the high parts; one conversion at the end
-        float h = 0.f, l = 0.f;
-        if (g < ng)
-            for (int w = 0; w < nw; ++w) {
-                const float2 hl = sh.red[(g * nw + w) * 8 + k];
-                pair_add(h, l, hl.x, hl.y);
-            }
-        double v = (double)h + (double)l;
-        int out = k;
-        if constexpr (!DF) {
-            const double next = __shfl_down_sync(0xffffffffu, v, 1);
-            if (k == 1 || k == 4) v += next;
-            out = k < 2 ? k : k == 2 || k == 5 ? 6 : k < 5 ? k - 1 : k - 2;
+    const int nw = blockDim.x >> 5;
+    if constexpr (DF) {
+        const int k = threadIdx.x & 7;
+        for (int g = threadIdx.x >> 3; g < ((ng + 3) & ~3); g += blockDim.x >> 3) {
+            float h = 0.f, l = 0.f;
+            if (g < ng)
+                for (int w = 0; w < nw; ++w) {
+                    const float2 hl = sh.red[(g * nw + w) * 8 + k];
+                    pair_add(h, l, hl.x, hl.y);
+                }
+            const double v = (double)h + (double)l;
+            if (g < ng && k < 6) c.part[((size_t)(ch0 + g) * 6 + k) * c.L + i] = v;
         }
-        if (g < ng && out < 6) c.part[((size_t)(ch0 + g) * 6 + out) * c.L + i] = v;
+    } else {
+        const auto sum = [&](const float2* r) {
+            float h = 0.f, l = 0.f;
+            for (int w = 0; w < nw; ++w) pair_add(h, l, r[8 * w].x, r[8 * w].y);
+            return (double)h + (double)l;
+        };
+        for (int t = threadIdx.x; t < 6 * ng; t += blockDim.x) {
+            const int g = t / 6, out = t - 6 * g, k = out + (out >= 2) + (out >= 4);
+            const float2* r = sh.red + g * nw * 8 + k;
+            double v = sum(r);
+            if (out == 1 || out == 3) v += sum(r + 1);
+            c.part[((size_t)ch0 * 6 + t) * c.L + i] = v;
+        }
     }
 }
 
