@@ -1175,7 +1175,7 @@ dyn_status dyn_rhs(void* p, double* hK, double* hR) {
     dyn_status s = c->pos_init();
     if (s) return s;
     CK(cudaMemcpyAsync(c->d.stages, c->stages_h, sizeof(StageDev), cudaMemcpyHostToDevice, c->st));
-    CK(launch_stage(c->d, 0, c->st));
+    CK(launch_rhs(c->d, c->st));
     CK(cudaMemcpyAsync(c->rhs_h, c->d.rhs_out, c->L * sizeof(double2), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     for (int i = 0; i < c->L; ++i) { hK[i] = c->rhs_h[i].x; hR[i] = c->rhs_h[i].y; }

@@ -951,6 +951,16 @@ cudaError_t launch_stage(const DevCtx& c, int s, cudaStream_t st, bool gather) {
     return launch_stage_pp<-1, -1>(c, s, st, gather);
 }
 
+// Nothing goes on from a lone right-hand side, so its B2 sums go to no planes: with / without
+// them a call measures, at L = 256, 512, 1024, 2048: plain 70 / 60, 82 / 72, 159 / 120, 470 /
+// 345 us; (hi, lo) 70 / 69, 92 / 84, 207 / 170, 819 / 698; FP64 82 / 81, 155 / 150, 430 / 416,
+// 1559 / 1477.  FP64 up to SPLIT_L keeps them: two threads a target 59 us, one 63 (L = 33).
+cudaError_t launch_rhs(const DevCtx& c, cudaStream_t st) {
+    DevCtx one = c;
+    if (c.mixed || c.L > SPLIT_L) one.b2key = nullptr;
+    return launch_stage(one, 0, st);
+}
+
 template <int P, int P2>
 static cudaError_t launch_main_pp(const DevCtx& c, int s, cudaStream_t st) {
     return c.m == 10 ? launch_main_k<10, P, P2>(c, s, st) : launch_main_k<0, P, P2>(c, s, st);

@@ -271,6 +271,8 @@ cudaError_t launch_tail_fit(const DevCtx& c, int nrows, int rollback_loop, doubl
 // launch wrappers (dyn_kernels.cu)
 // gather false: the epilogue alone (StageDev::fsal)
 cudaError_t launch_stage(const DevCtx& c, int s, cudaStream_t st, bool gather = true);
+// the right-hand side alone (KIND_RHS in stages[0])
+cudaError_t launch_rhs(const DevCtx& c, cudaStream_t st);
 cudaError_t launch_main_only(const DevCtx& c, int s, cudaStream_t st);
 cudaError_t launch_epi_only(const DevCtx& c, int s, cudaStream_t st);
 cudaError_t launch_pos_init(const DevCtx& c, int nrows, cudaStream_t st);
