@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(TPB, (DF ? DYN_BATCH_DF_TPSM : K > 1 ? 512 : M
                     else mixed::chunk_sums<M, K, P, P2, DYN_BATCH_SHIFT != 0>(c, sp, ch0 + g, g, s_lastf, sh, i, jb, par, keep);
                 }
                 __syncthreads();
-                mixed::fold_chunks<DF>(c, i, ch0, ng, sh);
+                mixed::fold_chunks<DF, true>(c, i, ch0, ng, sh);
                 if (ch0 + GMAX < nch) __syncthreads();
             }
         }

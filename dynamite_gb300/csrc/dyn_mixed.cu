@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(TPB_M, 10) k_main_mixed(const DevCtx c, const 
     __syncthreads();
     mixed::chunk_sums<M, 1, P, P2, true>(c, sp, blockIdx.x, 0, s_lastf, sh, i, jb, 0, keep);
     __syncthreads();
-    mixed::fold_chunks<false>(c, i, blockIdx.x, 1, sh);
+    mixed::fold_chunks<false, false>(c, i, blockIdx.x, 1, sh);
 }
 
 
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(TPB_M, 8) k_main_df(const DevCtx c, const int 
     __syncthreads();
     mdf::chunk_dd<M, 1, P, P2>(c, sp, blockIdx.x, 0, s_row, rc, sh, i, jb, 0, keep);
     __syncthreads();
-    mixed::fold_chunks<true>(c, i, blockIdx.x, 1, sh);
+    mixed::fold_chunks<true, false>(c, i, blockIdx.x, 1, sh);
 }
 
 namespace {

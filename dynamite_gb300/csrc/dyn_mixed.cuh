@@ -581,15 +581,17 @@ __device__ __forceinline__ void chunk_sums(const DevCtx& c, const StageDev& sp, 
 
 // After a __syncthreads() that follows the chunks of slots 0..ng-1 (chunks ch0..ch0+ng-1):
 // the block's six sums of each chunk into part[ch][0..6)[i], warps added in order, compensated
-// on the high parts, one conversion at the end.  (hi, lo) form: eight lanes a chunk, two idle,
-// in whole warps (a loop bounded by ng measured 1.3 % slower over mixed lengths).  The plain
-// form's eight are paired here, the two ConvA sums that share their factor, by the thread that
-// stores them: pairing across lanes kept so much alive through the batch's loop that it spilled
-// at 48 registers (16 quenches at L = 1024: 1005 us a gather at 56, now 950).
-template <bool DF>
+// on the high parts, one conversion at the end.  Eight lanes a chunk in whole warps ((hi, lo): two
+// of them idle; a loop bounded by ng measured 1.3 % slower over mixed lengths).  The plain form's
+// eight sums (DF false) are paired here, the two ConvA sums that share their factor: across lanes
+// in a kernel of one chunk; in the batch by the thread that stores them, because the exchange kept
+// so much alive through its loop that it spilled at 48 registers (16 quenches at L = 1024: 1005 us
+// a gather at 56, now 950; in the single kernel that form is the slower one, one RK54 step at
+// L = 640 282 us against 270).
+template <bool DF, bool BATCH>
 __device__ __forceinline__ void fold_chunks(const DevCtx& c, const int i, const int ch0, const int ng, const RowShared& sh) {
     const int nw = blockDim.x >> 5;
-    if constexpr (DF) {
+    if constexpr (DF || !BATCH) {
         const int k = threadIdx.x & 7;
         for (int g = threadIdx.x >> 3; g < ((ng + 3) & ~3); g += blockDim.x >> 3) {
             float h = 0.f, l = 0.f;
@@ -598,8 +600,14 @@ __device__ __forceinline__ void fold_chunks(const DevCtx& c, const int i, const 
                     const float2 hl = sh.red[(g * nw + w) * 8 + k];
                     pair_add(h, l, hl.x, hl.y);
                 }
-            const double v = (double)h + (double)l;
-            if (g < ng && k < 6) c.part[((size_t)(ch0 + g) * 6 + k) * c.L + i] = v;
+            double v = (double)h + (double)l;
+            int out = k;
+            if constexpr (!DF) {
+                const double next = __shfl_down_sync(0xffffffffu, v, 1);
+                if (k == 1 || k == 4) v += next;
+                out = k < 2 ? k : k == 2 || k == 5 ? 6 : k < 5 ? k - 1 : k - 2;
+            }
+            if (g < ng && out < 6) c.part[((size_t)(ch0 + g) * 6 + out) * c.L + i] = v;
         }
     } else {
         const auto sum = [&](const float2* r) {
