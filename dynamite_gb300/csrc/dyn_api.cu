@@ -76,7 +76,12 @@ struct Ctx {
     // and after an RK54 step whose row nobody edited the last stage's right-hand side is the next RK54
     // step's first (fsal_ok: Dormand-Prince writes the new row before its last stage evaluates it)
     bool b2_cont = false, fsal_ok = false;
-    void new_call() { b2_cont = fsal_ok = false; }
+    int call_steps = 1;  // steps that the running call may take
+    void forget() { b2_cont = fsal_ok = false; }
+    void new_call(int steps = 1) {
+        forget();
+        call_steps = steps;
+    }
     // discrete adjoint (FP64, fixed schedule): the recorded forward and its buffers
     AdjDev ad{};
     size_t ad_cap = 0;
@@ -339,9 +344,11 @@ struct Ctx {
         return DYN_OK;
     }
 
-    dyn_status enqueue_step(int S, bool fsal) {
+    dyn_status enqueue_step(int S, bool fsal, bool planes) {
+        DevCtx c = d;
+        if (!planes) c.b2key = nullptr;
         CK(cudaMemcpyAsync(d.stages, stages_h, sizeof(StageDev) * S, cudaMemcpyHostToDevice, st));
-        for (int s = 0; s < S; ++s) CK(launch_stage(d, s, st, !(s == 0 && fsal)));
+        for (int s = 0; s < S; ++s) CK(launch_stage(c, s, st, !(s == 0 && fsal)));
         CK(cudaMemcpyAsync(slots_h, d.slots, sizeof(Slots), cudaMemcpyDeviceToHost, st));
         return DYN_OK;
     }
@@ -353,15 +360,17 @@ struct Ctx {
         int S;
         double err_t, Tf, dtrf;
         if ((s = build_step(method, dt, &S, &err_t, &Tf, &dtrf))) return s;
-        const bool fsal = method == DYN_RK54 && fsal_ok;
+        // a step that starts the kept sums needs its first gather
+        const bool planes = b2_planes(d, n, call_steps);
+        const bool fsal = method == DYN_RK54 && fsal_ok && (b2_cont || !planes);
         stages_h[0].fsal = fsal;
-        const int key = fsal ? -method : method;
-        if (cfg.use_graph && warm[method] > 0) {
+        const int form = 2 * method + planes, key = fsal ? -form : form;
+        if (cfg.use_graph && warm[form] > 0) {
             auto it = graphs.find(key);
             if (it == graphs.end()) {
                 cudaGraph_t g;
                 CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-                dyn_status es = enqueue_step(S, fsal);
+                dyn_status es = enqueue_step(S, fsal, planes);
                 cudaError_t ce = cudaStreamEndCapture(st, &g);
                 if (es) return es;
                 CK(ce);
@@ -372,15 +381,15 @@ struct Ctx {
             }
             CK(cudaGraphLaunch(it->second, st));
         } else {
-            if ((s = enqueue_step(S, fsal))) return s;
-            warm[method]++;
+            if ((s = enqueue_step(S, fsal, planes))) return s;
+            warm[form]++;
         }
         CK(cudaStreamSynchronize(st));
         t1.push_back(Tf);
         dtr.push_back(dtrf);
         n += 1;
         gen++;
-        b2_cont = true;
+        b2_cont = planes;
         fsal_ok = method == DYN_RK54 && stages_h[S - 1].T == Tf;
         if (res) {
             res->delta = slots_h->res_err + err_t;
@@ -1287,7 +1296,7 @@ dyn_status dyn_run(void* p, const dyn_run_params* rp, dyn_step_result* last) {
     if (!rp->dt_schedule && (k.method < 1 || !(k.delta_t > 0.0)))
         return fail(DYN_ERR_STATE, "no step size or method: call dyn_controller_set after dyn_state_upload");
     dyn_step_result r{};
-    c->new_call();  // kept from step to step of one call, not between calls
+    c->new_call(rp->nsteps);  // kept from step to step of one call, not between calls
     for (int it = 0; it < rp->nsteps; ++it) {
         if (rp->tmax > 0 && c->t1[c->n - 1] >= rp->tmax) break;
         if (rp->dt_schedule) {
@@ -1374,7 +1383,7 @@ dyn_status dyn_rollback(void* p, int nrows) {
     const size_t target = c->n - nrows;
     c->n = target;
     c->gen++;
-    c->new_call();
+    c->forget();
     c->t1.resize(target);
     c->dtr.resize(target);
     c->ctl.delta_t = c->t1[target - 1] - c->t1[target - 2];
@@ -1626,7 +1635,7 @@ dyn_status dyn_sparsify(void* p, double threshold, int variant, size_t* n_out) {
     c->dtr = dtrn;
     c->n = k;
     c->gen++;
-    c->new_call();
+    c->forget();
     if ((s = c->mirror_all())) return s;
     if ((s = c->upload_times())) return s;
     if ((s = c->pos_init())) return s;

@@ -311,6 +311,8 @@ cudaError_t launch_compact(const DevCtx& c, const int* inds, const int* indsD, c
 cudaError_t launch_pack_rows(const double* QK, const double* QR, double2* out, size_t count,
                              cudaStream_t st);
 cudaError_t launch_main_mixed(const DevCtx& c, int s, cudaStream_t st);
+// whether a step over a history of `rows` rows keeps its B2 sums, in a call of `steps` steps
+bool b2_planes(const DevCtx& c, size_t rows, int steps);
 // FP32 mirrors of history elements [off, off + count) from the FP64 rows (mixed forms)
 cudaError_t launch_mirror(const DevCtx& c, size_t off, size_t count, cudaStream_t st);
 // [L*L][m] FP64 stencil rows to the tap-major planes of the mixed form `mixed` (1: float2, 2: float4)

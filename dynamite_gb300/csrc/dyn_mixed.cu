@@ -85,12 +85,14 @@ cudaError_t launch_t(const DevCtx& c, int s, cudaStream_t st) {
     return launch_pdl(k_main_mixed<M, P, P2, KEEP>, grid, dim3(TPB_M), (size_t)(c.L + 2) * sizeof(float2), st, c, s);
 }
 
+// The depth-10 plain form reads the staged row in element pairs, which pays where whole rows
+// keep one parity (RK54 step at the odd L = 257: 144 us, the generic depth 141; the (hi, lo)
+// form 153 against 171 at L = 257, 281 against 321 at 513)
+bool depth_ten(const DevCtx& c) { return c.m == 10 && (c.mixed == 2 || c.L % 2 == 0); }
+
 template <int P, int P2>
 cudaError_t launch_pp(const DevCtx& c, int s, cudaStream_t st) {
-    // the depth-10 plain form reads the staged row in element pairs, which pays where whole rows
-    // keep one parity (RK54 step at the odd L = 257: 144 us, the generic depth 141; the (hi, lo)
-    // form 153 against 171 at L = 257, 281 against 321 at 513)
-    const bool ten = c.m == 10 && (c.mixed == 2 || c.L % 2 == 0);
+    const bool ten = depth_ten(c);
     if (c.b2key) return ten ? launch_t<10, P, P2, true>(c, s, st) : launch_t<0, P, P2, true>(c, s, st);
     return ten ? launch_t<10, P, P2, false>(c, s, st) : launch_t<0, P, P2, false>(c, s, st);
 }
@@ -127,6 +129,24 @@ __global__ void k_weights_tapmajor(const double* in, void* out, size_t targets, 
 }
 
 }  // namespace
+
+// The planes pay in every form but the plain one at depth 10, whose sums are cheap beside the
+// 36 bytes a target that the planes add to the 144 it reads.  Up to L = 672 all of it stays in
+// L2 and keeping wins.  From there on it does not, while a short history still does, from which
+// the sums are formed anew: a lone step is better off so (its first stage, which fills the planes,
+// costs more than the others save), a call of four steps up to about 8 (L - 640) rows.  From 2048
+// on the weights alone fill L2, and two million elements of history do.  us with planes / without,
+// RK54, one step | a call of four:
+//   L =  704,  300 rows  327 /  300 | 1104 /  1113     L = 1024,  3500 rows  640 /  592 |  2150 /  2142
+//   L =  768,  600 rows  419 /  369 | 1377 /  1340     L = 1536,  4500 rows 1269 / 1161 |  4222 /  4205
+//   L =  768, 1200 rows  419 /  382 | 1382 /  1406     L = 2048,   600 rows 2106 / 2030 |  7005 /  7290
+//   L = 1024,  600 rows  628 /  532 | 2124 /  1945     L = 2048,  1100 rows 2153 / 2294 |  7078 /  8266
+bool b2_planes(const DevCtx& c, size_t rows, int steps) {
+    if (!c.b2key) return false;
+    if (c.mixed != 1 || !depth_ten(c) || c.L <= 672) return true;
+    if (c.L >= 2048) return steps >= 4 || rows * c.L >= (size_t)2 << 20;
+    return steps >= 4 && rows >= 8 * (size_t)(c.L - 640);
+}
 
 cudaError_t launch_main_mixed(const DevCtx& c, int s, cudaStream_t st) {
     if (c.M.p == 3 && c.M.p2 == 4) return launch_pp<3, 4>(c, s, st);
