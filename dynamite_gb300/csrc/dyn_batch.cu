@@ -1156,8 +1156,10 @@ dyn_status dyn_batch_run(void* p, long long max_ticks, long long* ticks_out) {
     TraceRange tr("dyn_batch_run");
     Batch* bt = BT(p);
     long long done = 0;
-    dyn_status s = bt->new_call();
-    if (s || (s = bt->read_plans())) return s;
+    dyn_status s = bt->read_plans();
+    // after the wait for the plans, so that nothing waits for it; not for a batch that is done
+    if (!s && max_ticks > 0 && bt->running() > 0) s = bt->new_call();
+    if (s) return s;
     while (done < max_ticks && bt->running() > 0) {
         if ((s = bt->ensure_graph())) return s;
         if (max_ticks - done >= bt->graph_ticks) {
