@@ -331,8 +331,13 @@ __global__ void __launch_bounds__(TPB, (DF ? DYN_BATCH_DF_TPSM : K > 1 ? 512 : M
             else mixed::row_setup<true>(c, sp, i, s_lastf, sh, !keep);
         }
         __syncthreads();
-        // the next item, by a thread of the last warp while the others work on this one
-        if (threadIdx.x == TPB - 32) fetch_item<KEEP>(Q, PL, items, nitems, work, force, s_item[p ^ 1]);
+        // the next item, by a thread of the last warp: while the others work on this one, or (the
+        // plain form at depth 10) while they fold it.  Taken that early, a batch's last items wait for
+        // whoever took them, not for the first block to be free: RK54 steps of 4 plain quenches at
+        // L = 512 585 us early, 547 late, of 16 at 1024 6.81 / 6.78 ms; order 5, 16 at 512 1.53 /
+        // 1.57; (hi, lo), whose items are longer, 64 at 512 22.9 / 23.0.
+        constexpr bool early = DF || M != 10;
+        if (early && threadIdx.x == TPB - 32) fetch_item<KEEP>(Q, PL, items, nitems, work, force, s_item[p ^ 1]);
         if (it.run) {
             const int nch = c.nch;
             for (int ch0 = 0; ch0 < nch; ch0 += GMAX) {
@@ -346,6 +351,7 @@ __global__ void __launch_bounds__(TPB, (DF ? DYN_BATCH_DF_TPSM : K > 1 ? 512 : M
                 if (ch0 + GMAX < nch) __syncthreads();
             }
         }
+        if (!early && threadIdx.x == TPB - 32) fetch_item<KEEP>(Q, PL, items, nitems, work, force, s_item[p ^ 1]);
         __syncthreads();
         p ^= 1;
     }
