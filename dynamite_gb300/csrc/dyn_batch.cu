@@ -468,6 +468,7 @@ struct Batch {
     int M = 10, pp = 0;  // template selectors: stencil depth, (p, p2) kind
     bool df = false;     // DYN_MIXED_DF: (hi, lo) inputs (mdf::chunk)
     bool keep = false;   // every quench has planes for its B2 sums
+    bool planes = false; // and the running call keeps them there
     size_t smem = 0, Lmax = 0;
     cudaGraphExec_t graph = nullptr;
     int graph_ticks = 0;
@@ -494,29 +495,29 @@ struct Batch {
     }
 
     // Calls f with the gather kernel of a tile shape.  The (hi, lo) form runs one target per
-    // thread.  It keeps its B2 sums, whose compensated products are most of its work; in the
-    // plain form they cost less than the planes' traffic (64 quenches at L = 512: 0.75 ms a
+    // thread.  With `kept` it keeps its B2 sums, whose compensated products are most of its work;
+    // in the plain form they cost less than the planes' traffic (64 quenches at L = 512: 0.75 ms a
     // gather with planes, 0.69 without).
     template <int M_, int P_, int P2_, typename F>
-    auto with_kernel_m(int threads, int targets, F f) {
+    auto with_kernel_m(bool kept, int threads, int targets, F f) {
         const bool wide = threads == 256;
-        if (df && keep) return wide ? f(k_batch_gather<M_, 1, P_, P2_, 256, true, true>) : f(k_batch_gather<M_, 1, P_, P2_, 128, true, true>);
+        if (kept) return wide ? f(k_batch_gather<M_, 1, P_, P2_, 256, true, true>) : f(k_batch_gather<M_, 1, P_, P2_, 128, true, true>);
         if (df) return wide ? f(k_batch_gather<M_, 1, P_, P2_, 256, true, false>) : f(k_batch_gather<M_, 1, P_, P2_, 128, true, false>);
         if (targets == 2) return wide ? f(k_batch_gather<M_, 2, P_, P2_, 256, false, false>) : f(k_batch_gather<M_, 2, P_, P2_, 128, false, false>);
         return wide ? f(k_batch_gather<M_, 1, P_, P2_, 256, false, false>) : f(k_batch_gather<M_, 1, P_, P2_, 128, false, false>);
     }
     template <int P_, int P2_, typename F>
-    auto with_kernel_p(int threads, int targets, F f) {
-        return M == 10 ? with_kernel_m<10, P_, P2_>(threads, targets, f) : with_kernel_m<0, P_, P2_>(threads, targets, f);
+    auto with_kernel_p(bool kept, int threads, int targets, F f) {
+        return M == 10 ? with_kernel_m<10, P_, P2_>(kept, threads, targets, f) : with_kernel_m<0, P_, P2_>(kept, threads, targets, f);
     }
     template <typename F>
-    auto with_kernel(int threads, int targets, F f) {
-        if (pp == 1) return with_kernel_p<3, 4>(threads, targets, f);
-        if (pp == 2) return with_kernel_p<3, 0>(threads, targets, f);
-        return with_kernel_p<-1, -1>(threads, targets, f);
+    auto with_kernel(bool kept, int threads, int targets, F f) {
+        if (pp == 1) return with_kernel_p<3, 4>(kept, threads, targets, f);
+        if (pp == 2) return with_kernel_p<3, 0>(kept, threads, targets, f);
+        return with_kernel_p<-1, -1>(kept, threads, targets, f);
     }
     cudaError_t launch_gather(int force = 0) {
-        return with_kernel(tpb, kpt, [&](auto* kern) {
+        return with_kernel(planes, tpb, kpt, [&](auto* kern) {
             return launch_pdl(kern, dim3(nsm * ctas), dim3(tpb), smem, st, (const Quench*)qd, (const Plan*)pd,
                               (const unsigned*)items, nitems, work, force);
         });
@@ -532,8 +533,12 @@ struct Batch {
     }
 
     int occupancy(int threads, int targets) {
+        if (keep) occupancy(false, threads, targets);  // its limits and hints too
+        return occupancy(keep, threads, targets);
+    }
+    int occupancy(bool kept, int threads, int targets) {
         int nb = 0;
-        const void* f = with_kernel(threads, targets, [](auto* kern) { return (const void*)kern; });
+        const void* f = with_kernel(kept, threads, targets, [](auto* kern) { return (const void*)kern; });
         // the (hi, lo) form stages Lmax float4: with its static part above 48 KB from Lmax = 2700
         // on.  The limit belongs to the kernel, not to this batch, so it goes to what the longest
         // rows there are need: another live batch launches this kernel under it.  Set here,
@@ -695,7 +700,11 @@ struct Batch {
         return any ? read_plans() : DYN_OK;
     }
 
-    dyn_status new_call() {
+    // A call of so many ticks.  One that ends before its later ticks bring in what filling the
+    // planes costs leaves them alone: a call of 1 | 2 | 3 ticks with planes / without, 16 quenches at
+    // L = 512 762 / 574 | 1248 / 1120 | 1327 / 1196 us; 32 at L = 256, order 5, 306 / 292 | 493 / 551.
+    dyn_status new_call(long long ticks) {
+        planes = keep && ticks >= (M == 10 ? 4 : 2);
         k_batch_call<<<1, 32, 0, st>>>(work);
         BCK(cudaGetLastError());
         return DYN_OK;
@@ -733,7 +742,10 @@ struct Batch {
         const int T = cfg.ticks_per_launch > 0 ? cfg.ticks_per_launch : 32;
         cudaGraph_t g;
         BCK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+        const bool p = planes;
+        planes = keep;  // the graph's form (graph_fits)
         dyn_status es = enqueue_ticks(T);
+        planes = p;
         cudaError_t ce = cudaStreamEndCapture(st, &g);
         if (es) return es;
         BCK(ce);
@@ -743,6 +755,8 @@ struct Batch {
         graph_ticks = T;
         return DYN_OK;
     }
+
+    bool graph_fits(long long ticks) const { return planes == keep && ticks >= graph_ticks; }
 
     // t = 0 state of quench b (dyn_state_init: initialization.cpp:204-222)
     dyn_status init_state(int b) {
@@ -1164,11 +1178,11 @@ dyn_status dyn_batch_run(void* p, long long max_ticks, long long* ticks_out) {
     long long done = 0;
     dyn_status s = bt->read_plans();
     // after the wait for the plans, so that nothing waits for it; not for a batch that is done
-    if (!s && max_ticks > 0 && bt->running() > 0) s = bt->new_call();
+    if (!s && max_ticks > 0 && bt->running() > 0) s = bt->new_call(max_ticks);
     if (s) return s;
     while (done < max_ticks && bt->running() > 0) {
         if ((s = bt->ensure_graph())) return s;
-        if (max_ticks - done >= bt->graph_ticks) {
+        if (bt->graph_fits(max_ticks - done)) {
             BCK(cudaGraphLaunch(bt->graph, bt->st));
             done += bt->graph_ticks;
         } else {
@@ -1187,9 +1201,9 @@ dyn_status dyn_batch_enqueue(void* p, long long ticks) {
     TraceRange tr("dyn_batch_enqueue");
     Batch* bt = BT(p);
     dyn_status s = bt->ensure_graph();
-    if (s || (s = bt->new_call())) return s;
+    if (s || (s = bt->new_call(ticks))) return s;
     long long done = 0;
-    for (; done + bt->graph_ticks <= ticks; done += bt->graph_ticks) BCK(cudaGraphLaunch(bt->graph, bt->st));
+    for (; bt->graph_fits(ticks - done); done += bt->graph_ticks) BCK(cudaGraphLaunch(bt->graph, bt->st));
     return bt->enqueue_ticks((int)(ticks - done));
 }
 
@@ -1231,7 +1245,7 @@ dyn_status dyn_batch_profile(void* p, int reps, float* ms) {
     BCK(cudaEventCreate(&b));
     // the pending stage of every quench: all sums once, then as a stage that goes on from
     // there, the form all but a call's first stages have
-    dyn_status s = bt->new_call();
+    dyn_status s = bt->new_call(1 << 20);  // as a long call
     if (s) return s;
     BCK(bt->launch_gather(1));
     BCK(cudaEventRecord(a, bt->st));
