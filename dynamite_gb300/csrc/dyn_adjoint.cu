@@ -18,11 +18,14 @@
 //                    94-100) transposed: row cotangents of the eight memory
 //                    integrals, the direct last-row terms, QK^{B1}[i,0] and
 //                    rInt (index_vec.cpp:63-156) scattered to the history;
-//   k_adj_targets    per target (i,j): the A1/A2/B1/B2 gathers recomputed,
-//                    Sigma and the int.dat products differentiated, and the
-//                    gathers transposed (scatter-adds into the cotangent
-//                    history; the last-row stencils through shared memory and
-//                    a per-row partial, reduced by k_adj_lastreduce).
+//   k_adj_targets    per target (i,j): the A1/A2/B1/B2 values that the recompute
+//                    recorded, Sigma and the int.dat products differentiated, B1
+//                    transposed (scatter-adds into the cotangent history), the
+//                    A1/A2 cotangents stored and B2's as a packet;
+//   k_adj_lastrow    the A1/A2 stencils transposed onto the last row, a partial
+//                    row per target row, summed by k_adj_lastreduce;
+//   k_adj_b2ser      the B2 stencils transposed, from the packets in the order of
+//                    their stencil starts (k_adj_b2gen at other depths than 10).
 //
 // Parameter derivatives (Gamma, lambda) accumulate in device scalars.
 #include <algorithm>
@@ -364,7 +367,7 @@ __global__ void __launch_bounds__(ADJ_ROW_T) k_adj_rows(const DevCtx c, const Ad
 // (reductions), the A1/A2 cotangents of the target stored for k_adj_lastrow
 // and its B2 packet for k_adj_b2ser.  Bound by the FP64 pipe (82 % busy): 150 instructions a
 // target with whole derivatives and weights formed per product, 105 now (L = 512: 75 -> 57 us).
-template <int M, int P, int P2>
+template <int P, int P2>
 __global__ void __launch_bounds__(64) k_adj_targets(const DevCtx c, const AdjDev a, const AdjModel am, const int s) {
     wait_prior_grid();
     const StageDev& sp = c.stages[s];
@@ -780,7 +783,7 @@ cudaError_t launch_targets_pp(const DevCtx& c, const AdjDev& a, const AdjModel& 
     const dim3 grid((c.L + 63) / 64, c.L);
     const size_t lsm = lastrow_smem(c.L);
     const size_t NP = (size_t)c.L * c.L;
-    cudaError_t e = launch_pdl(c.m == 10 ? k_adj_targets<10, P, P2> : k_adj_targets<0, P, P2>, grid, dim3(64), 0, st, c, a, am, s);
+    cudaError_t e = launch_pdl(k_adj_targets<P, P2>, grid, dim3(64), 0, st, c, a, am, s);
     if (e != cudaSuccess) return e;
     if ((e = launch_pdl(k_adj_lastrow, dim3(c.L), dim3(LR_T), lsm, st, c, a, s)) != cudaSuccess) return e;
     if (c.m != 10) return launch_pdl(k_adj_b2gen, dim3((unsigned)((NP + 255) / 256)), dim3(256), 0, st, c, a, s);

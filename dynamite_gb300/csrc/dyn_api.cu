@@ -287,8 +287,6 @@ struct Ctx {
                 const int nx = s + 1;
                 sp.pos_save = (ssp && nx >= 2 && nx <= 4) ? nx - 2 : -1;
                 sp.pos_reuse = (ssp && nx >= 5 && nx <= 7) ? nx - 5 : -1;
-                sp.nb2_save = sp.pos_save;
-                sp.nb2_reuse = sp.pos_reuse;
             }
             double gte = T0;
             for (int j = 0; j < S; ++j) gte += dt * B2[j] * 1.0;
@@ -307,7 +305,7 @@ struct Ctx {
                 sp.serk_c2 = 2 * dt * alpha;
                 sp.serk_b0 = b[0];
                 sp.serk_bnext = b[s + 1];
-                sp.b2_save = sp.b2_reuse = sp.pos_save = sp.pos_reuse = sp.nb2_save = sp.nb2_reuse = -1;
+                sp.b2_save = sp.b2_reuse = sp.pos_save = sp.pos_reuse = -1;
                 if (s == 0) {
                     sp.serk_mode = 0;
                     gt = T0 + dt * alpha * 1.0;
@@ -795,9 +793,9 @@ dyn_status dyn_ctx_create(const dyn_config* cfg, const dyn_tables* tb, void** ou
     d.mixed = cfg->precision == DYN_MIXED ? 1 : cfg->precision == DYN_MIXED_DF ? 2 : 0;
     // tile shape: threads per CTA x targets per thread.  FP64: two targets share a warp
     // reduction from L = 768 on, where enough CTAs are left to balance the SMs; per RK54
-    // step 1 / 2 targets measure 152 / 159 us (L = 64), 228 / 241 (256), 414 / 466 (400),
-    // 555 / 562 (512), 1780 / 1756 (1024).  Mixed: one target per thread keeps more warps
-    // in flight for the latency-bound gathers.
+    // step of a run of 12, 1 / 2 targets measure 152 / 159 us (L = 64), 228 / 241 (256),
+    // 414 / 466 (400), 555 / 562 (512), 1780 / 1756 (1024).  Mixed: one target per thread
+    // keeps more warps in flight for the latency-bound gathers.
     d.tpb = d.mixed ? 128 : 64;
     d.kpt = d.mixed ? 1 : (L >= 768 ? 2 : 1);
     d.nch = (int)((L + (size_t)d.tpb * d.kpt - 1) / ((size_t)d.tpb * d.kpt));
@@ -812,7 +810,7 @@ dyn_status dyn_ctx_create(const dyn_config* cfg, const dyn_tables* tb, void** ou
         (s = dalloc(&w3, L2 * m)) || (s = dalloc(&d.posB1x, L)) || (s = dalloc(&d.posB1x_next, L)) || (s = dalloc(&d.b1, L)) || (s = dalloc(&d.posB1x_saved, NSAVE * L)) ||
         (s = dalloc(&d.posB2x, L2)) || (s = dalloc(&d.posB2x_saved, NSAVE * L2)) ||
         (s = dalloc(&d.h, (size_t)SMAX * L)) || (s = dalloc(&d.gS, L)) || (s = dalloc(&d.geS, L)) ||
-        (s = dalloc(&d.gfS, L)) || (s = dalloc(&d.part, L * (size_t)d.nch * 8)) || (s = dalloc(&d.rowval, L)) ||
+        (s = dalloc(&d.gfS, L)) || (s = dalloc(&d.part, L * (size_t)d.nch * 6)) || (s = dalloc(&d.rowval, L)) ||
         (s = dalloc(&d.epart, (size_t)G * EP_N)) || (s = dalloc(&d.slots, 1)) || (s = dalloc(&d.stages, SMAX)) ||
         (s = dalloc(&d.rhs_out, L)) || (s = dalloc(&d.rint, L)) || (s = dalloc(&c->scratch_dev, 4 * L + 16))) {
         d.theta = th; d.phi2 = p2; d.integ = it; d.iA1 = a1; d.iA2 = a2; d.iB2 = b2; d.wA1 = w1; d.wA2 = w2; d.wB2 = w3;
@@ -1180,7 +1178,7 @@ dyn_status dyn_rhs(void* p, double* hK, double* hR) {
     sp.T = c->t1[c->n - 1];
     Ctx::set_clamps(sp);
     sp.b2_save = NSAVE;  // keep posB2x of the current state readable
-    sp.b2_reuse = sp.pos_save = sp.pos_reuse = sp.nb2_save = sp.nb2_reuse = -1;
+    sp.b2_reuse = sp.pos_save = sp.pos_reuse = -1;
     dyn_status s = c->pos_init();
     if (s) return s;
     CK(cudaMemcpyAsync(c->d.stages, c->stages_h, sizeof(StageDev), cudaMemcpyHostToDevice, c->st));
@@ -1415,7 +1413,7 @@ dyn_status dyn_profile_stage(void* p, int reps, float* ms_main, float* ms_epi) {
     sp.n0 = (int)c->n;
     sp.T = c->t1[c->n - 1];
     Ctx::set_clamps(sp);
-    sp.b2_save = sp.b2_reuse = sp.pos_save = sp.pos_reuse = sp.nb2_save = sp.nb2_reuse = -1;
+    sp.b2_save = sp.b2_reuse = sp.pos_save = sp.pos_reuse = -1;
     dyn_status s = c->pos_init();
     if (s) return s;
     CK(cudaMemcpyAsync(c->d.stages, c->stages_h, sizeof(StageDev), cudaMemcpyHostToDevice, c->st));

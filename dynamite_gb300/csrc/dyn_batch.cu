@@ -9,7 +9,7 @@
 //     mixed-precision row set-up and chunk functions of the single-quench
 //     kernel (dyn_mixed.cuh) on that quench's current stage; the last CTA to
 //     leave resets the counter, so the kernel is idempotent per stage.
-//   k_batch_epi (one one-warp CTA per 32 history rows of every quench): the
+//   k_batch_epi (a CTA of four warps per 32 history rows of every quench): the
 //     epilogue functions of the single-quench kernel (dyn_epi.cuh); the last
 //     CTA of each quench folds its partials and then plans that quench's next
 //     stage: at the end of a step it applies the step-size controller of
@@ -18,9 +18,9 @@
 //     same operation order as the host planner (so times are bit-identical).
 //
 // The host replays a CUDA graph of `ticks_per_launch` ticks and reads the
-// quench plans back between replays; nothing else crosses PCIe.  A quench's
-// one-warp epilogue latency overlaps the other quenches' gathers, which is
-// what a single quench cannot do.
+// quench plans back between replays; nothing else crosses PCIe.  A quench's row
+// set-up latency overlaps the other quenches' targets, which is what a single
+// quench cannot do.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -130,8 +130,6 @@ __device__ void begin_step(const Quench& q, Plan& pl, const TabDev& tb) {
             const int nx = s + 1;
             sp.pos_save = (ssp && nx >= 2 && nx <= 4) ? nx - 2 : -1;
             sp.pos_reuse = (ssp && nx >= 5 && nx <= 7) ? nx - 5 : -1;
-            sp.nb2_save = sp.pos_save;
-            sp.nb2_reuse = sp.pos_reuse;
             sp.serk_mode = 0;
             sp.serk_c = sp.serk_c2 = sp.serk_b0 = sp.serk_bnext = 0.0;
         }
@@ -152,7 +150,7 @@ __device__ void begin_step(const Quench& q, Plan& pl, const TabDev& tb) {
             sp.serk_c2 = c2;
             sp.serk_b0 = tb.serk_b[qq][0];
             sp.serk_bnext = tb.serk_b[qq][s + 1];
-            sp.b2_save = sp.b2_reuse = sp.pos_save = sp.pos_reuse = sp.nb2_save = sp.nb2_reuse = -1;
+            sp.b2_save = sp.b2_reuse = sp.pos_save = sp.pos_reuse = -1;
             if (s == 0) {
                 sp.serk_mode = 0;
                 gt = __dadd_rn(T0, ca);
@@ -967,7 +965,7 @@ dyn_status dyn_batch_create(const dyn_batch_config* cfg, const dyn_batch_grid* g
             (s = bt->alloc(&d.inv_dtr_f, cap)) || (s = bt->alloc(&d.posB1x, L)) || (s = bt->alloc(&d.posB1x_next, L)) || (s = bt->alloc(&d.rowval, L)) || (s = bt->alloc(&d.b1, L)) ||
             (s = bt->alloc(&d.posB1x_saved, NSAVE * L)) || (s = bt->alloc(&d.h, (size_t)SMAX * L)) ||
             (s = bt->alloc(&d.gS, L)) || (s = bt->alloc(&d.geS, L)) || (s = bt->alloc(&d.gfS, L)) ||
-            (s = bt->alloc(&d.part, L * nchm * 8)) ||
+            (s = bt->alloc(&d.part, L * nchm * 6)) ||
             (s = bt->alloc(&d.epart, G * EP_N)) || (s = bt->alloc(&d.slots, 1)) || (s = bt->alloc(&d.rhs_out, L)) ||
             (s = bt->alloc(&q.stg, 2 * SMAX))) {
             delete bt;

@@ -5,14 +5,18 @@
 // drstep2GPU, appendAllGPU_ptr/replaceAllGPU_ptr, rstepGPU, RK54GPU...) runs
 // as two kernels:
 //
-//   k_main (grid L x nch): every target (i, j) gathers its A1/A2/B1/B2
-//     values from the history through the stencil tables, evaluates Sigma,
-//     and accumulates the eight int.dat-weighted products of the memory
-//     integrals; nothing of size L^2 is written.
-//   k_epi (grid L/32): finishes the row reductions, forms the EOM right-hand
-//     side, the RK stage combination, writes the history row, accumulates
-//     r(t) (and dr/dt at stage 0) and computes the next stage's positions;
-//     the last CTA to finish (atomic ticket) folds the per-CTA partials.
+//   k_main (grid L x nch, and a few CTAs for the rows' own work): every
+//     target (i, j) gathers its A1/A2/B1/B2 values from the history through
+//     the stencil tables, evaluates Sigma, and accumulates the eight
+//     int.dat-weighted products of the memory integrals in six sums (two pairs
+//     share their factor).  Of size L^2 it writes what the next stage goes on
+//     from: each target's history row and those of its four B2 sums that
+//     changed.  The rows' own CTAs interpolate QK^{B1}[i,0] and rInt and search
+//     the next stage's B1 positions.
+//   k_epi (grid L/32, four warps a CTA): finishes the row reductions, forms the
+//     EOM right-hand side and the RK stage combination, writes the history row,
+//     accumulates r(t) (and dr/dt at stage 0) and forms the next stage's B1
+//     rows; the last CTA to finish (atomic ticket) folds the per-CTA partials.
 //
 // A second, reference-order family of kernels ("exact") materializes the 16
 // interpolation arrays and the RHS with the reference CPU build's operation
@@ -911,7 +915,7 @@ static cudaError_t launch_main_t(const DevCtx& c, int s, cudaStream_t st) {
     return launch_pdl(k_main<M, K, P, P2, LOGR, KEEP, SPLIT>, grid, block, smem, st, c, s);
 }
 
-// Lengths up to which k_main takes two threads a target (RK54 step, one thread a target -> two:
+// Lengths up to which k_main takes two threads a target (`run` of one RK54 step, one thread a target -> two:
 // L = 64 166 -> 142 us, 128 172 -> 154, 192 198 -> 191, 224 230 -> 231, 320 325 -> 330): beyond
 // 192 a row has four chunks and its warps fill the schedulers by themselves.
 constexpr int SPLIT_L = 192;

@@ -31,7 +31,6 @@ struct StageDev {
     int s, kind, last, nrows, n0, nrows_next;
     int b2_save, b2_reuse;   // main(s): posB2x save/reuse slot, -1 none
     int pos_save, pos_reuse; // epilogue(s): next stage's posB1x save/reuse slot
-    int nb2_reuse, nb2_save; // next stage's posB2x flags (for the B2 clamp)
     int ncoef, serk_mode;    // serk_mode: 0 first stage, 1 even, 2 odd
     int maxceil, maxX;       // B1 Floor clamp and B2 row clamp of this stage (from nrows)
     int fresh;               // 1: the gather searches the B1 positions itself (after a rollback)

@@ -6,8 +6,9 @@
 //   * stencil weights are FP32 copies of the FP64 tables;
 //   * the history is read from an FP32 mirror (float2 (QK,QR), (dQK,dQR))
 //     that the epilogue writes next to the FP64 master rows;
-//   * A1/A2/B1/B2 gathers, Sigma and the eight convolution products are FP32;
-//     each thread accumulates its products with a compensated (TwoSum) sum,
+//   * A1/A2/B1/B2 gathers, Sigma and the eight convolution products are FP32
+//     (in the (hi, lo) form double-float, the two pairs that share their factor
+//     as one sum each); each thread accumulates its products compensated (TwoSum),
 //     and the cross-lane fold and everything of size L (RHS, RK combination,
 //     r(t), dr/dt, C(t,t), the step-error norm, time) stay in FP64.
 // The position search is the exact FP64 binary search (integer compares on

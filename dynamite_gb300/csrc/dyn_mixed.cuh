@@ -183,17 +183,9 @@ __device__ __forceinline__ float2 dot_ldg(const float2* __restrict__ w, size_t L
     }
 }
 
-// (h, l) + s, normalized (the double-float sum of namespace mdf)
-__device__ __forceinline__ void shift_offset(float& h, float& l, float s) {
-    const float t = __fadd_rn(h, s), bp = __fsub_rn(t, h);
-    const float e = __fadd_rn(__fadd_rn(__fsub_rn(h, __fsub_rn(t, bp)), __fsub_rn(s, bp)), __fadd_rn(l, 0.f));
-    h = __fadd_rn(t, e);
-    l = __fsub_rn(e, __fsub_rn(h, t));
-}
-
-// The same for a segment of the history (start b in the whole array): read as six 16-byte loads
-// from the even element at or below the start, every tap selecting its element.  Reads up to
-// two elements past a segment and uses none of them.
+// A ten-tap sum as dot_ldg's over a segment of the history (start b in the whole array), read as
+// six 16-byte loads from the even element at or below the start, every tap selecting its element.
+// Reads up to two elements past a segment and uses none of them.
 __device__ __forceinline__ float2 seg10(const float w[10], const float2* __restrict__ arr, size_t b) {
     const float4* p = reinterpret_cast<const float4*>(arr + (b & ~(size_t)1));
     const bool sh = b & 1;
@@ -208,6 +200,14 @@ __device__ __forceinline__ float2 seg10(const float w[10], const float2* __restr
 #pragma unroll
     for (int d = 0; d < 10; ++d) acc = ffma2s(w[d], sh ? e[d + 1] : e[d], acc);
     return acc;
+}
+
+// (h, l) + s, normalized (the double-float sum of namespace mdf)
+__device__ __forceinline__ void shift_offset(float& h, float& l, float s) {
+    const float t = __fadd_rn(h, s), bp = __fsub_rn(t, h);
+    const float e = __fadd_rn(__fadd_rn(__fsub_rn(h, __fsub_rn(t, bp)), __fsub_rn(s, bp)), __fadd_rn(l, 0.f));
+    h = __fadd_rn(t, e);
+    l = __fsub_rn(e, __fsub_rn(h, t));
 }
 
 // TwoSum accumulation: s + c carries the sum to about twice FP32 precision
@@ -634,7 +634,7 @@ __device__ __forceinline__ void fold_chunks(const DevCtx& c, const int i, const 
 // (hi, lo) pairs; the A1/A2 and B2 stencil sums add every product w x with its
 // rounding error (TwoProd, TwoSum) and the cross terms (w_hi x_lo + w_lo x_hi); the gathered values stay
 // (hi, lo) and everything that changes from stage to stage -- the B2 interval offset,
-// the Hermite weights, B1, Sigma and the eight int.dat products -- runs in double-float
+// the Hermite weights, B1, Sigma and the int.dat products -- runs in double-float
 // (chunk_dd), so the stage derivatives carry no stage-to-stage FP32 rounding noise and
 // the embedded error estimate sees the method's error, as in the FP64 form.  The
 // derivative rows (dQK, dQR), a step's worth of change, stay single FP32.
